@@ -728,7 +728,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
     if ((rc = ws_begin(w))) return rc;
     const size_t n = (size_t)g.n, nc = (size_t)g.ncell;
     PSIM_CUDA(w.posd.ensure(32 * n));
-    PSIM_CUDA(w.posh.ensure(16 * n));
+    PSIM_CUDA(w.posh.ensure(16 * (n + kPoshPad)));
     PSIM_CUDA(w.posl.ensure(16 * n));
     PSIM_CUDA(w.cellid.ensure(4 * n));
     PSIM_CUDA(w.tag_out.ensure(4 * n));
@@ -1999,7 +1999,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
     ok = ok && !s->cellid.ensure(4 * n) && !s->key.ensure(4 * n) && !s->rank.ensure(4 * n) &&
          !s->tmp.ensure(4 * n) && !s->start.ensure(4 * nc) &&
          !s->scratch.ensure(4 * scan_scratch_ints(g.ncell)) &&
-         !s->posh.ensure(16 * (n + 4)) &&   // + 4: the list build reads up to 3 past a run
+         !s->posh.ensure(16 * (n + kPoshPad)) &&
          !s->vel.ensure(24 * n) && !s->err.ensure(4) && !s->state.ensure(sizeof(StepState)) &&
          !s->occ.ensure(4);
     if (ok && cfg->precision == PSIM_PRECISION_FP64) ok = !s->posd.ensure(32 * n);

@@ -27,6 +27,11 @@ struct ForceSetup {
     int lj_pure;       // LennardJones with yukawaStrength 0 in every replica
 };
 
+// Elements a posh array holds past its n particles wherever a pair list is
+// built on it: the build reads its runs four candidates at a time, up to three
+// past the last particle.
+constexpr int kPoshPad = 4;
+
 // Positions and cell ranges in sorted (cell) order, as the force kernels read them.
 struct CellView {
     const double4_32a* posd;  // {x, y, z, R}  (FP64 form)
