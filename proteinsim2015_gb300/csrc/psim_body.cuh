@@ -29,25 +29,53 @@ struct ComboPair {  // AO + LJ(n) summed; each part inside its own cutoff
     }
 };
 
-// Plain form of one pair (i <- j): the reference's own minimum-image rules,
-// pbcDist's |dx| > L/2.0 for r^2 (utilities.cpp:79-104) and unitVectorAdv's
-// |dx| > int(L)/2 for the unit vector (utilities.cpp:114-142), the overlap
-// check (AOPotential.cpp:83-88) and, for AO, the NaN check (:105-109).
-// Each row's partial sum is folded into the total, as the reference folds
-// each cell's partial (AOPotential.cpp:165-167).
+// F(r)/r of a pair at r^2 in FP64: a functor's own fr64(r2, size, size^2) of
+// 1/r or 1/r^2 (rsqrt64 / rcp64) with fused multiply-adds, or fnet64 / r for a
+// functor that has only that (a plugin's, the composite), which may test r or
+// r^2 against distances of its own and so gets them as the reference rounds
+// them: r is the square root by Markstein's correction of r2/sqrt(r2).
+// GB300 issues two FP64 operations a clock and SM, so the FP64 pass takes as
+// long as it has FP64 operations: sqrt, 1/r and fnet64 in the reference's order
+// were ~180 a pair, the LJ(6) form here is 12 and AO's 17.
+template <class P, class = void>
+struct HasFr64 : std::false_type {};
+template <class P>
+struct HasFr64<P, decltype((void)&P::fr64)> : std::true_type {};
+template <class P>
+__device__ __forceinline__ double pair_fr64(const P& p, double r2, double size, double s2) {
+    if constexpr (HasFr64<P>::value) {
+        return p.fr64(r2, size, s2);
+    } else {
+        const double ri = rsqrt64(r2);
+        double r = __dmul_rn(r2, ri);
+        r = __fma_rn(__dmul_rn(0.5, ri), __fma_rn(-r, r, r2), r);
+        return __dmul_rn(p.fnet64(r2, r, ri, size), ri);
+    }
+}
+
+// Plain form of one pair (i <- j), as the reference decides it: pbcDist's
+// minimum image |dx| > L/2.0 (utilities.cpp:79-104) and r^2 < rc^2 on the
+// r^2 it rounds product by product, the overlap check r < 0.8 size
+// (AOPotential.cpp:83-88) and, for AO, the NaN check (:105-109).  Its tests run
+// on the bit patterns as integers, which order like the non-negative values, and
+// the exact ones only next to a threshold; the force itself is pair_fr64 on an
+// r^2 summed with fused multiply-adds.  The image that unitVectorAdv takes by
+// |dx| > int(L)/2 (utilities.cpp:114-142) is the same one for a pair in range:
+// its |dx| is below rc or above L - rc, and rc <= cellSize <= L/3 <= int(L)/2.
 template <class Pair>
 struct F64Body {
     Pair pf;
     using Aux = double4_32a;  // the FP64 neighbour positions {x, y, z, R}
     static constexpr bool kBatchable = !std::is_same<Pair, ComboPair>::value;
-    // the reference's summation order and image rules: always the staged walk
-    static constexpr bool kDirectWalk = false;
+    static constexpr bool kQuadWalk = true;   // force_quad_kernel
     struct Home {
         double4_32a p;
+        double size, s2;      // contact diameter with a neighbour of the same radius, squared
+        int over_hi;          // high word of r^2 at or below which such a pair may overlap
     };
     using Shifted = Home;     // the FP64 form takes raw differences
     struct Acc {
-        double n0, n1, n2, c0, c1, c2;
+        double n0, n1, n2;
         int cnt;
     };
     __device__ __forceinline__ const Aux* aux(const CellView& cv) const { return cv.posd; }
@@ -60,47 +88,85 @@ struct F64Body {
         return b;
     }
     __device__ __forceinline__ void init(Acc& a) const {
-        a.n0 = a.n1 = a.n2 = a.c0 = a.c1 = a.c2 = 0.0;
+        a.n0 = a.n1 = a.n2 = 0.0;
         a.cnt = 0;
     }
     __device__ __forceinline__ void load_home(const CellView& cv, int i, Home& h) const {
         h.p = cv.posd[i];
+        h.size = h.p.w + h.p.w;
+        h.s2 = __dmul_rn(h.size, h.size);
+        h.over_hi = __double2hiint(__dmul_rn(0.64, h.s2)) + 1;
     }
     __device__ __forceinline__ void shift(const Home& h, const float4&, int, int, int,
                                           const DevGeom&, Shifted& o) const {
         o = h;
     }
+    // r^2 as the reference rounds it
+    static __device__ __forceinline__ double r2_exact(double d0, double d1, double d2) {
+        return __dadd_rn(__dadd_rn(__dmul_rn(d0, d0), __dmul_rn(d1, d1)), __dmul_rn(d2, d2));
+    }
     __device__ __forceinline__ void eval(const float4&, const double4_32a& pj, const Home& h,
                                          Acc& a, uint32_t& err) const {
         const DevGeom& g = geom;
         double d0 = pj.x - h.p.x, d1 = pj.y - h.p.y, d2 = pj.z - h.p.z;
-        double a0 = fabs(d0), a1 = fabs(d1), a2 = fabs(d2);
-        if (a0 > g.half) a0 -= g.L;
-        if (a1 > g.half) a1 -= g.L;
-        if (a2 > g.half) a2 -= g.L;
-        const double r2 = (a0 * a0) + (a1 * a1) + (a2 * a2);
+        if (abs_above(d0, g.half) | abs_above(d1, g.half) | abs_above(d2, g.half)) {
+            // keeps the compiler from doing the additions for every pair
+            asm volatile("" : "+d"(d0), "+d"(d1), "+d"(d2));
+            if (abs_above(d0, g.half)) d0 += toward(g.L, d0);
+            if (abs_above(d1, g.half)) d1 += toward(g.L, d1);
+            if (abs_above(d2, g.half)) d2 += toward(g.L, d2);
+        }
+        const double r2 = HasFr64<Pair>::value
+                              ? __fma_rn(d2, d2, __fma_rn(d1, d1, __dmul_rn(d0, d0)))
+                              : r2_exact(d0, d1, d2);
         // updateInteractions' test: r = sqrt(pbcDist) < 1.2 (systemHandling.cpp:112-115)
-        if (cont > 0.0 && sqrt(r2) < cont) ++a.cnt;
-        if (r2 < pf.rc2) {
-            const double r = sqrt(r2);
-            const double size = h.p.w + pj.w;
-            if (r < 0.8 * size) err |= EBIT_OVERLAP;
-            const double rinv = 1.0 / r;
-            const double f = pf.fnet64(r2, r, rinv, size);
-            if (Pair::kCheckNan && isnan(f)) err |= EBIT_NAN;
-            if (fabs(d0) > g.half_uv) d0 = (d0 < 0) ? d0 + g.L : d0 - g.L;
-            if (fabs(d1) > g.half_uv) d1 = (d1 < 0) ? d1 + g.L : d1 - g.L;
-            if (fabs(d2) > g.half_uv) d2 = (d2 < 0) ? d2 + g.L : d2 - g.L;
-            a.c0 += f * (d0 * rinv);
-            a.c1 += f * (d1 * rinv);
-            a.c2 += f * (d2 * rinv);
+        if (count && sqrt(r2_exact(d0, d1, d2)) < cont) ++a.cnt;
+        // r^2 < rc^2 by the high words (a NaN is above); where they are equal, or
+        // r^2's is one less, the reference's r^2 decides
+        const int hr = __double2hiint(r2), hc = __double2hiint(pf.rc2);
+        bool in = hr < hc;
+        if ((unsigned)(hc - hr) <= 1u) {
+            asm volatile("" : "+d"(d0));
+            in = r2_exact(d0, d1, d2) < pf.rc2;
+        }
+        if (in) {
+            double size = h.size, s2 = h.s2;
+            bool close = hr <= h.over_hi;
+            if (__double_as_longlong(pj.w) != __double_as_longlong(h.p.w)) {
+                size = h.p.w + pj.w;
+                s2 = __dmul_rn(size, size);
+                close = true;
+            }
+            if (close && sqrt(r2_exact(d0, d1, d2)) < 0.8 * size) err |= EBIT_OVERLAP;
+            const double f = pair_fr64(pf, r2, size, s2);
+            // a NaN, by its bits (isnan would be an FP64 operation)
+            if (Pair::kCheckNan &&
+                (__double_as_longlong(f) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll)
+                err |= EBIT_NAN;
+            a.n0 = __fma_rn(f, d0, a.n0);
+            a.n1 = __fma_rn(f, d1, a.n1);
+            a.n2 = __fma_rn(f, d2, a.n2);
         }
     }
-    __device__ __forceinline__ void fold(Acc& a) const {
-        a.n0 += a.c0;
-        a.n1 += a.c1;
-        a.n2 += a.c2;
-        a.c0 = a.c1 = a.c2 = 0.0;
+    // L for d < 0, else -L
+    static __device__ __forceinline__ double toward(double L, double d) {
+        return __hiloint2double(__double2hiint(L) | (~__double2hiint(d) & 0x80000000),
+                                __double2loint(L));
+    }
+    // |d| > h for h > 0, to 20 bits: an image's |d| is never near L/2
+    static __device__ __forceinline__ bool abs_above(double d, double h) {
+        return (__double2hiint(d) & 0x7fffffff) > __double2hiint(h);
+    }
+    __device__ __forceinline__ void fold(Acc&) const {}
+    // the sums of the four lanes of a particle, added in lane order
+    __device__ __forceinline__ void add_quad(Acc& a) const {
+#pragma unroll
+        for (int k = 1; k < 4; k <<= 1) {
+            a.n0 += __shfl_xor_sync(0xffffffffu, a.n0, k);
+            a.n1 += __shfl_xor_sync(0xffffffffu, a.n1, k);
+            a.n2 += __shfl_xor_sync(0xffffffffu, a.n2, k);
+            a.cnt += __shfl_xor_sync(0xffffffffu, a.cnt, k);
+        }
     }
     // the FP64 form takes raw differences; only the FP32 test copy is imaged
     __device__ __forceinline__ void image(float4& h, double4_32a&, int sx, int sy, int sz,
@@ -135,7 +201,8 @@ struct F64Body {
         if (out.coor) out.coor[i] = a.cnt;
     }
     DevGeom geom;
-    double cont = 0.0;   // > 0: count the neighbours closer than cont (ForceOut::coor)
+    double cont = 0.0;   // count the neighbours closer than cont (ForceOut::coor)
+    bool count = false;
 };
 
 struct ComboPairF {
@@ -172,8 +239,7 @@ struct MixedBody {
     float cont2f = 0.f;  // > 0: count the neighbours with r^2 < cont2f (ForceOut::coor)
     using Aux = float4;  // the low parts of the neighbour positions
     static constexpr bool kBatchable = !std::is_same<Pair, ComboPairF>::value;
-    // the 27-cell walk that keeps its queues across rows (force_direct_kernel)
-    static constexpr bool kDirectWalk = true;
+    static constexpr bool kQuadWalk = false;   // force_direct_kernel, force_pass_kernel
     struct Home {
         float4 lo;
     };

@@ -39,6 +39,7 @@ struct DevGeom {
     double inv_cs;  // 1 / cellSize (fast path of the cell hash)
     float Lhi, Llo; // L as a float pair (Lhi + Llo == L to ~1e-14)
     float inv_csf;  // 1 / cellSize in FP32 (the FP32 cell hash)
+    float inv_s, inv_s2; // 1 / s and 1 / s^2 (cell_xyz)
     float hash_guard; // distance from a cell face (in cells) below which FP64 decides
     // a system's place in a batch of independent replicas (one system: 0, 0, n):
     // its first global cell and its particle range in every storage order
@@ -62,6 +63,8 @@ inline void fill_geom(int n, int s, double L, double cs, DevGeom* g) {
     g->Lhi = (float)L;
     g->Llo = (float)(L - (double)g->Lhi);
     g->inv_csf = (float)g->inv_cs;
+    g->inv_s = 1.0f / (float)s;
+    g->inv_s2 = 1.0f / (float)g->s2;
     // FP32 hash error: x cut or rounded to FP32 (< ulp(L)) scaled by 1/cs, plus
     // the roundings of 1/cs and of the product (each ~s 2^-24 cells); 4x that
     // is the guard
@@ -139,6 +142,24 @@ __device__ __forceinline__ double widen_f32(float f) {
     const unsigned long long ed = e == 0u ? 0ull : (e == 255u ? 2047ull : (unsigned long long)(e + 896u));
     const unsigned long long m = e == 0u ? 0ull : (unsigned long long)(b & 0x7FFFFFu) << 29;
     return __longlong_as_double((long long)(sign | (ed << 52) | m));
+}
+
+// 1/a and 1/sqrt(a) to about an ulp in 3 and 5 FP64 operations, from the
+// hardware's ~20-bit seeds (rcp.approx / rsqrt.approx, not on the FP64 unit) and
+// one third-order Householder iteration: with h = 1 - a y (1 - a y^2) the seed's
+// relative error e becomes e^3, below the rounding of the last operation.  a
+// positive and normal; 0 gives a NaN.
+__device__ __forceinline__ double rcp64(double a) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double h = __fma_rn(-a, y, 1.0);
+    return __fma_rn(y, __fma_rn(h, h, h), y);
+}
+__device__ __forceinline__ double rsqrt64(double a) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double h = __fma_rn(-__dmul_rn(a, y), y, 1.0);
+    return __fma_rn(__dmul_rn(y, h), __fma_rn(h, 0.375, 0.5), y);
 }
 
 // Knuth's TwoSum: s + e == a + b exactly.
@@ -269,6 +290,40 @@ __device__ __forceinline__ int wrap_cell(int c, int s, int& shift) {
     return w;
 }
 
+// c + d for |d| <= 1 and c in [0, s): the wrapped cell and its image
+__device__ __forceinline__ int wrap_near(int c, int s, int& shift) {
+    shift = 0;
+    if (c < 0) {
+        c += s;
+        shift = -1;
+    } else if (c >= s) {
+        c -= s;
+        shift = 1;
+    }
+    return c;
+}
+
+// c / d and its remainder r for 0 <= c < 2^24, d > 0, inv = 1 / d: the FP32
+// quotient is off by at most one, which the remainder corrects.
+__device__ __forceinline__ int div_small(int c, int d, float inv, int& r) {
+    int q = (int)((float)c * inv);
+    r = c - q * d;
+    if (r < 0) {
+        --q;
+        r += d;
+    } else if (r >= d) {
+        ++q;
+        r -= d;
+    }
+    return q;
+}
+// The cell coordinates of cell c of grid g (at most 256 cells a side).
+__device__ __forceinline__ void cell_xyz(int c, const DevGeom& g, int& x, int& y, int& z) {
+    int r;
+    z = div_small(c, g.s2, g.inv_s2, r);
+    y = div_small(r, g.s, g.inv_s, x);
+}
+
 // ------------------------------------------------------------ pair functors
 // fnet64: the plugin's FP64 per-pair magnitude in the reference's operation
 // order, except that integer powers use binary powering and divisions by r2
@@ -318,6 +373,15 @@ struct AOPair {
         double f = 36.0 * r38 + c1 * rinv + c2 * r;
         return -f;
     }
+    // F(r)/r for the FP64 passes (see pair_fr64)
+    __device__ __forceinline__ double fr64(double r2, double, double) const {
+        const double ri = rsqrt64(r2);
+        const double i2 = __dmul_rn(ri, ri), i4 = __dmul_rn(i2, i2), i8 = __dmul_rn(i4, i4),
+                     i16 = __dmul_rn(i8, i8);
+        const double i39 =
+            __dmul_rn(__dmul_rn(__dmul_rn(i16, i16), __dmul_rn(i4, i2)), ri);
+        return -__fma_rn(36.0, i39, __fma_rn(c1, i2, c2));
+    }
     __device__ __forceinline__ float fnet32(float r2, float r, float rinv, float) const {
         float r36 = pow36(rinv);
         float r38 = r36 * (rinv * rinv);
@@ -338,6 +402,8 @@ struct LJPair {
     double rc2, kTwd, four_n, yuk, lambda, inv_lambda;
     float rc2f, kTwdf, four_nf, yukf, lambdaf, inv_lambdaf;
     int n;
+    int pure;   // no Yukawa term
+    double c64; // -kTwd four_n
     static constexpr bool kCheckNan = false;
     __host__ __device__ __forceinline__ double fnet64(double r2, double r, double rinv, double size) const {
         double lj = powi_binary(size * rinv, n);
@@ -349,6 +415,25 @@ struct LJPair {
             repel = e * (rinv * rinv * (lambda + r) * yuk);
         }
         return -kTwd * (attract + repel);
+    }
+    // F(r)/r with the Yukawa term at 1/r = ri and L = lj (see pair_fr64)
+    __device__ __forceinline__ double fr64_of(double r2, double ri, double i2, double lj) const {
+        double a = __dmul_rn(__dmul_rn(c64, lj), __fma_rn(2.0, lj, -1.0));
+        if (!pure) {
+            const double r = __dmul_rn(r2, ri);
+            const double e = exp(-1.0 * (r * inv_lambda));
+            a = __fma_rn(-__dmul_rn(kTwd, yuk), __dmul_rn(e, __dmul_rn(ri, __dadd_rn(lambda, r))), a);
+        }
+        return __dmul_rn(a, i2);
+    }
+    // an even exponent without a Yukawa term needs 1/r^2 alone
+    __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
+        if ((n & 1) == 0 && pure) {
+            const double i2 = rcp64(r2);
+            return fr64_of(r2, 0.0, i2, powi_binary(__dmul_rn(s2, i2), n / 2));
+        }
+        const double ri = rsqrt64(r2);
+        return fr64_of(r2, ri, __dmul_rn(ri, ri), powi_binary(__dmul_rn(size, ri), n));
     }
     __device__ __forceinline__ float fnet32(float r2, float r, float rinv, float size) const {
         float lj = powi_binary(size * rinv, n);
@@ -376,6 +461,12 @@ struct CalPair {
     static constexpr bool kCheckNan = false;
     __host__ __device__ __forceinline__ double fnet64(double, double, double rinv, double) const {
         return -(36.0 * (pow36(rinv) * rinv));
+    }
+    // F(r)/r = -36 r^-38 for the FP64 passes (see pair_fr64)
+    __device__ __forceinline__ double fr64(double r2, double, double) const {
+        const double i2 = rcp64(r2), i4 = __dmul_rn(i2, i2), i8 = __dmul_rn(i4, i4),
+                     i16 = __dmul_rn(i8, i8);
+        return __dmul_rn(-36.0, __dmul_rn(__dmul_rn(i16, i16), __dmul_rn(i4, i2)));
     }
     __device__ __forceinline__ float fnet32(float, float, float rinv, float) const {
         return -(36.0f * (pow36(rinv) * rinv));
@@ -412,6 +503,8 @@ inline LJPair make_lj_pair(double kT, double wd, int n, double yuk, double lambd
     p.n = n;
     p.four_n = 4.0 * n;
     p.yuk = yuk;
+    p.pure = yuk == 0.0;
+    p.c64 = -p.kTwd * p.four_n;
     p.lambda = lambda;
     p.inv_lambda = 1.0 / lambda;
     p.rc2f = (float)p.rc2;

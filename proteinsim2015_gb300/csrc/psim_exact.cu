@@ -26,7 +26,8 @@ static cudaError_t run_fp64(const Pair& p, const DevGeom& g, const CellView& cv,
                             const ForceOut& out, float pre, cudaStream_t st, int tile,
                             const BatchView* bv) {
     F64Body<Pair> body{p, g};
-    body.cont = out.coor ? out.cont : 0.0;   // updateInteractions fused into the pass
+    body.count = out.coor && out.cont > 0.0;   // updateInteractions fused into the pass
+    body.cont = out.cont;
     if (tile && !bv) return launch_force_cells(body, g, cv, out, pre, st);
     return launch_force_pass(body, g, cv, out, pre, st, bv);
 }

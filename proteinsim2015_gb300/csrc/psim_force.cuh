@@ -26,9 +26,10 @@
 //
 // Body supplies the precision-specific parts (psim_exact.cu: FP64 plain form
 // with the reference's image rules; psim_mixed.cu: FP32 pairs with Kahan
-// sums).  The staged walk serves the FP64 form; the mixed form takes the
-// direct walk (force_direct_kernel, below), which reads the rows through L1
-// and keeps its queues across rows.
+// sums).  The FP64 form takes the four-lane walk (force_quad_kernel) and the
+// mixed form the direct walk (force_direct_kernel), which reads the rows through
+// L1 and keeps its queues across rows; the staged walk is left for the mixed
+// form of systems beyond the direct walk's 2^27 slots.
 #pragma once
 
 #include <climits>
@@ -215,22 +216,15 @@ force_pass_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_rc2
 // direct walk beat the staged walk at every occupancy tried (1 to 21
 // particles per cell: force pass 3-37% shorter).  The image is applied to
 // the neighbour (Body::image).  A single system and each replica of a batch
-// follow the same rule, so that a replica steps alike in both.  The FP64
-// form keeps the staged walk, whose sums follow the reference's cell order:
-// a direct walk with a fold marker at each row's end gave the same bits but
-// measured 6-18% slower (its 32-byte FP64 neighbour loads through L1).
-constexpr int kDirectQueue = kQueue;          // the staged walk's queue rows, reused
+// follow the same rule, so that a replica steps alike in both.
 constexpr int kDirectMaxN = 1 << 27;          // slots the queue entries can hold
 constexpr int kDirectCentre = 13;             // image code of (0, 0, 0)
 
-// walk: 0 the body's own choice, 1 the staged walk, 2 the direct walk (where
-// the body allows it).  A queue entry holds a storage slot in 27 bits: the
-// grid's particles (a replica's, in a batch: global slots up to p1) must end
-// below 2^27.
-template <class Body>
+// walk: 1 the staged walk, else the direct walk.  A queue entry holds a storage
+// slot in 27 bits: the grid's particles (a replica's, in a batch: global slots up
+// to p1) must end below 2^27.
 __host__ __device__ __forceinline__ bool direct_walk(const DevGeom& g, int walk = 0) {
-    if constexpr (Body::kDirectWalk) return g.p1 <= kDirectMaxN && walk != 1;
-    return false;
+    return g.p1 <= kDirectMaxN && walk != 1;
 }
 
 template <class Body>
@@ -319,9 +313,9 @@ __device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeo
                     q[cnt][lane] = (uint32_t)j | code;
                     cnt += in ? 1 : 0;
                 }
-                // at most kDirectQueue - kUnroll entries before a batch of
+                // at most kQueue - kUnroll entries before a batch of
                 // kUnroll: slots stay below kQueueCap
-                if (__any_sync(0xffffffffu, cnt > kDirectQueue - kUnroll)) drain();
+                if (__any_sync(0xffffffffu, cnt > kQueue - kUnroll)) drain();
             }
         }
     }
@@ -340,6 +334,159 @@ force_direct_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_r
                       s_q[w]);
 }
 
+// The FP64 form's 27-cell walk: four lanes a particle, eight particles a warp.
+// GB300 issues an FP64 instruction of a warp in 16 clocks of an SM's one unit
+// (and ~68 for a warp alone), whatever its active lanes, so what counts is how
+// many lanes of each carry a pair and, on few particles, how long a lane's chain
+// is.  The lanes of a particle test four candidates at a time and put those in
+// range into the particle's queue, each at its rank in the lanes' ballot; lane m
+// then evaluates entries m, m + 4, ... .  So a warp's FP64 instructions wait for
+// the fullest of eight neighbourhoods over 4 (83% of their lanes carry a pair on
+// the liquid), where a lane per particle that drained its own queue after every
+// row of cells waited for the fullest of 32 at each row (29%).  A lane's terms
+// are added in order and the lanes' sums as (0 + 1) + (2 + 3): the same for one
+// system and a batch.  Force pass, staged rows and the reference's order of
+// operations before, and after: 2^20 LJ at 13 a cell 17.4 -> 2.46 ms (FP64 unit
+// 83% busy), 4000 AO colloids 56 -> 13 us.
+constexpr int kQuadWarps = 2;                   // warps per block
+constexpr int kQuadCap = 128;                   // queue entries per particle
+constexpr int kQuadStride = kQuadCap + 4;       // distinct banks for eight particles
+constexpr int kQuadBatches = 2;                 // batches of 4 candidates between drain checks
+
+// A row per lane below 8 particles a cell: the nine rows then take three rounds,
+// and short runs leave no lane waiting for a fourth candidate.  Force pass with a
+// row per lane / a row at a time, us: AO at 0.5 particles a cell 4000 13.2 / 17.7,
+// 50001 27.5 / 37.3; LJ at 13 a cell 16384 71.5 / 67.1, 2^20 2501 / 2468.
+__device__ __forceinline__ bool quad_rows(const DevGeom& g) {
+    return g.n < 8ll * g.ncell;
+}
+
+template <class Body>
+__device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom& g,
+                                                const CellView& cv, const ForceOut& out,
+                                                float pre_rc2, int i, int lane,
+                                                uint32_t (*qs)[kQuadStride]) {
+    using Aux = typename Body::Aux;
+    const Aux* g_aux = body.aux(cv);
+    const int m = lane & 3;
+    const bool active = i < g.p1;
+    uint32_t* q = qs[lane >> 2];
+    float4 hi = make_float4(0.f, 0.f, 0.f, 0.f);
+    int cx = 0, cy = 0, cz = 0;
+    typename Body::Home home;
+    typename Body::Acc acc;
+    body.init(acc);
+    if (active) {
+        hi = cv.posh[i];
+        cell_xyz(cv.cellid[i] - g.c0, g, cx, cy, cz);
+        body.load_home(cv, i, home);
+    }
+    uint32_t err = 0;
+    int cnt = 0;    // entries in the particle's queue
+    int done = 0;   // entries evaluated before them
+    auto drain = [&]() {
+        __syncwarp();   // the lanes' entries are written
+        int k = (m - done) & 3;
+        const int last = __reduce_max_sync(0xffffffffu, cnt);
+        // the next neighbour is loaded while this one's terms are formed
+        Aux aj{};
+        if (k < cnt) aj = g_aux[q[k]];
+        for (int it = 0; it < last; it += 4, k += 4) {
+            Aux an{};
+            if (k + 4 < cnt) an = g_aux[q[k + 4]];
+            if (k < cnt) body.eval(hi, aj, home, acc, err);
+            aj = an;
+        }
+        done += cnt;
+        cnt = 0;
+        __syncwarp();   // the entries are read
+    };
+    const bool edge = active && (cx == 0 || cx == g.s - 1);
+    const int parts = __any_sync(0xffffffffu, edge) ? 2 : 1;
+    const uint32_t below = (1u << m) - 1u;
+    // one row of cells at a time, the lanes on neighbouring candidates, or (few
+    // particles per cell) a row per lane
+    const bool rows4 = quad_rows(g);
+    const int step = rows4 ? 1 : 4, first = rows4 ? 0 : m;
+#pragma unroll 1
+    for (int round = 0; round < (rows4 ? 3 : 9); ++round) {
+        const int row = rows4 ? 4 * round + m : round;
+        const int dz = row / 3 - 1, dy = row - 3 * (row / 3) - 1;
+        int sy, sz;
+        const int y = wrap_near(cy + dy, g.s, sy);
+        const int z = wrap_near(cz + dz, g.s, sz);
+        const int base = g.c0 + g.s * y + g.s2 * z;
+        const float hy = hi.y - (float)sy * g.Lhi;
+        const float hz = hi.z - (float)sz * g.Lhi;
+        // part 0: the cells of [cx-1, cx+1] inside the grid, contiguous;
+        // part 1: the one cell that wraps around in x (if any)
+#pragma unroll 1
+        for (int part = 0; part < parts; ++part) {
+            int a = 0, len = 0, sx = 0;
+            if ((part == 0 ? active : edge) && row < 9) {
+                if (part != 0) sx = cx == 0 ? -1 : 1;
+                const int xa = part == 0 ? max(cx - 1, 0) : (cx == 0 ? g.s - 1 : 0);
+                const int xb = part == 0 ? min(cx + 1, g.s - 1) : xa;
+                a = cv.cstart[base + xa];
+                len = cv.cstart[base + xb] + cv.ccount[base + xb] - a;
+            }
+            const int lmax = __reduce_max_sync(0xffffffffu, len);
+            const float hx = hi.x - (float)sx * g.Lhi;
+            const float4* pp = cv.posh + a;
+            const int self = i - a;   // the home particle is this candidate of its run
+            for (int t0 = 0; t0 < lmax; t0 += step * kQuadBatches) {
+                float4 hj[kQuadBatches];
+#pragma unroll
+                for (int u = 0; u < kQuadBatches; ++u) {
+                    const int t = t0 + u * step + first;
+                    if (t < len) hj[u] = __ldg(pp + t);
+                }
+#pragma unroll
+                for (int u = 0; u < kQuadBatches; ++u) {
+                    const int t = t0 + u * step + first;
+                    const float ex = hj[u].x - hx, ey = hj[u].y - hy, ez = hj[u].z - hz;
+                    const float r2 = ex * ex + ey * ey + ez * ez;
+                    const bool in = (t < len) & (r2 < pre_rc2) & (t != self);
+                    const uint32_t bits = __ballot_sync(0xffffffffu, in) >> (lane & 28) & 15u;
+                    if (in) q[cnt + __popc(bits & below)] = (uint32_t)(a + t);
+                    cnt += __popc(bits);
+                }
+                if (__any_sync(0xffffffffu, cnt > kQuadCap - 4 * kQuadBatches)) drain();
+            }
+        }
+    }
+    drain();
+    body.add_quad(acc);
+    if (active && m == 0) body.store(out, i, acc);
+    if (err) atomicOr(out.err, err);
+}
+
+template <class Body>
+__global__ void __launch_bounds__(kQuadWarps * 32)
+force_quad_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_rc2) {
+    __shared__ uint32_t s_q[kQuadWarps][8][kQuadStride];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (pass_failed(out, lane)) return;  // warp-uniform
+    force_quad_warp(body, g, cv, out, pre_rc2, (blockIdx.x * kQuadWarps + w) * 8 + (lane >> 2),
+                    lane, s_q[w]);
+}
+
+// A batch of replicas: four warps a task of 32 particles of one replica.
+template <class Body>
+__global__ void __launch_bounds__(kQuadWarps * 32)
+force_quad_batch_kernel(Body body0, CellView cv, ForceOut out, BatchView bv) {
+    __shared__ uint32_t s_q[kQuadWarps][8][kQuadStride];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (pass_failed(out, lane)) return;
+    const int warp = blockIdx.x * kQuadWarps + w;
+    if (warp / 4 >= bv.n_tasks) return;
+    const int2 t = bv.tasks[warp / 4];
+    const DevGeom g = bv.geoms[t.x];
+    const Body body = body0.for_replica(bv.pairs, t.x, g);
+    force_quad_warp(body, g, cv, out, bv.pre[t.x], t.y + 8 * (warp % 4) + (lane >> 2), lane,
+                    s_q[w]);
+}
+
 // A batch of replicas: each warp takes a task (replica, first particle) and
 // that replica's geometry, pair functor and prefilter bound.
 template <class Body>
@@ -355,7 +502,7 @@ force_batch_kernel(Body body0, CellView cv, ForceOut out, BatchView bv, int walk
     const int2 t = bv.tasks[task];
     const DevGeom g = bv.geoms[t.x];
     const Body body = body0.for_replica(bv.pairs, t.x, g);
-    if (direct_walk<Body>(g, walk))   // the rule a single system of this replica follows
+    if (direct_walk(g, walk))   // the rule a single system of this replica follows
         force_direct_warp(body, g, cv, out, bv.pre[t.x], t.y + lane, lane, s_q[w]);
     else
         force_pass_warp(body, g, cv, out, bv.pre[t.x], t.y + lane, lane, s_hi[w], s_aux[w],
@@ -370,20 +517,30 @@ cudaError_t launch_force_pass(const Body& body, const DevGeom& g, const CellView
     if (bv && bv->tasks) {
         if constexpr (Body::kBatchable) {
             if (bv->n_tasks == 0) return cudaSuccess;
-            const int blocks = (bv->n_tasks + kForceWarps - 1) / kForceWarps;
-            force_batch_kernel<Body><<<blocks, threads, 0, st>>>(body, cv, out, *bv, walk);
+            if constexpr (Body::kQuadWalk) {
+                const int blocks = (4 * bv->n_tasks + kQuadWarps - 1) / kQuadWarps;
+                force_quad_batch_kernel<Body><<<blocks, kQuadWarps * 32, 0, st>>>(body, cv, out,
+                                                                                 *bv);
+            } else {
+                const int blocks = (bv->n_tasks + kForceWarps - 1) / kForceWarps;
+                force_batch_kernel<Body><<<blocks, threads, 0, st>>>(body, cv, out, *bv, walk);
+            }
             return cudaGetLastError();
         }
         return cudaErrorInvalidValue;
     }
     if (g.n == 0) return cudaSuccess;
-    if (direct_walk<Body>(g, walk)) {
+    if constexpr (Body::kQuadWalk) {
+        const int per = 8 * kQuadWarps;
+        force_quad_kernel<Body><<<(g.n + per - 1) / per, kQuadWarps * 32, 0, st>>>(body, g, cv, out,
+                                                                                  pre_rc2);
+    } else if (direct_walk(g, walk)) {
         force_direct_kernel<Body><<<(g.n + threads - 1) / threads, threads, 0, st>>>(
             body, g, cv, out, pre_rc2);
-        return cudaGetLastError();
+    } else {
+        force_pass_kernel<Body><<<(g.n + threads - 1) / threads, threads, 0, st>>>(body, g, cv,
+                                                                                  out, pre_rc2);
     }
-    force_pass_kernel<Body><<<(g.n + threads - 1) / threads, threads, 0, st>>>(body, g, cv, out,
-                                                                              pre_rc2);
     return cudaGetLastError();
 }
 
@@ -401,6 +558,15 @@ struct LJFixed : LJPair {
             repel = e * (rinv * rinv * (lambda + r) * yuk);
         }
         return -kTwd * (attract + repel);
+    }
+    // LJPair::fr64's operations with the exponent unrolled
+    __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
+        if (N % 2 == 0 && pure) {
+            const double i2 = rcp64(r2);
+            return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));
+        }
+        const double ri = rsqrt64(r2);
+        return fr64_of(r2, ri, __dmul_rn(ri, ri), powi_fixed<N>(__dmul_rn(size, ri)));
     }
     __device__ __forceinline__ float fnet32(float r2, float r, float rinv, float size) const {
         float attract = 0.0f;
@@ -420,6 +586,10 @@ struct LJFixed : LJPair {
 template <int N>
 struct LJPure : LJPair {
     static_assert(N > 0 && N % 2 == 0, "an even, positive exponent");
+    __device__ __forceinline__ double fr64(double r2, double, double s2) const {
+        const double i2 = rcp64(r2);
+        return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));
+    }
     __device__ __forceinline__ float fnet32(float, float, float rinv, float size) const {
         const float lj = powi_fixed<N>(size * rinv);
         return -kTwdf * ((2.0f * lj - 1.0f) * (four_nf * rinv * lj));

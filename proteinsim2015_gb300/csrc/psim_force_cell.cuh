@@ -36,19 +36,6 @@ constexpr int kCellQueueCap = kCellQueue + kCellUnroll;
 // kCellUnroll: below chunk + kCellUnroll * kCellThreads
 constexpr int kCellPad = kCellUnroll * kCellThreads;
 
-// c + d for |d| <= 1 and c in [0, s): the wrapped cell and its image
-__device__ __forceinline__ int wrap_near(int c, int s, int& shift) {
-    shift = 0;
-    if (c < 0) {
-        c += s;
-        shift = -1;
-    } else if (c >= s) {
-        c -= s;
-        shift = 1;
-    }
-    return c;
-}
-
 template <class Body>
 __global__ void __launch_bounds__(kCellThreads)
 force_cell_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_rc2) {
