@@ -214,7 +214,11 @@ force_pass_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_rc2
 // share their rows' runs, so the candidate reads broadcast through L1 about
 // as well as they would from a shared-memory stage.  Measured on GB300 the
 // direct walk beat the staged walk at every occupancy tried (1 to 21
-// particles per cell: force pass 3-37% shorter).  The image is applied to
+// particles per cell: force pass 3-37% shorter).  It is bound by instruction
+// issue: a candidate's address is an offset from its run's pointer and its load
+// and test are predicated by the run's length, the home cell is decoded without
+// integer divisions, and the wrapped part of a row is walked only by a warp with a
+// particle at the box edge.  The gel at 2^21: 275 -> 228 us.  The image is applied to
 // the neighbour (Body::image).  A single system and each replica of a batch
 // follow the same rule, so that a replica steps alike in both.
 constexpr int kDirectMaxN = 1 << 27;          // slots the queue entries can hold
@@ -230,11 +234,10 @@ __host__ __device__ __forceinline__ bool direct_walk(const DevGeom& g, int walk 
 template <class Body>
 __device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeom& g,
                                                   const CellView& cv, const ForceOut& out,
-                                                  float pre_rc2, int i, int lane,
+                                                  float pre_rc2, int i, bool active, int lane,
                                                   uint32_t (*q)[32]) {
     using Aux = typename Body::Aux;
     const Aux* g_aux = body.aux(cv);
-    const bool active = i < g.p1;
     float4 hi = make_float4(0.f, 0.f, 0.f, 0.f);
     int cx = 0, cy = 0, cz = 0;
     typename Body::Home home;
@@ -242,80 +245,80 @@ __device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeo
     body.init(acc);
     if (active) {
         hi = cv.posh[i];
-        const int c = cv.cellid[i] - g.c0;
-        cx = c % g.s;
-        cy = (c / g.s) % g.s;
-        cz = c / g.s2;
+        cell_xyz(cv.cellid[i] - g.c0, g, cx, cy, cz);
         body.load_home(cv, i, home);
     }
     typename Body::Shifted hs;
     body.shift(home, hi, 0, 0, 0, g, hs);
     uint32_t err = 0;
-    int cnt = 0;
-    const int jlast = g.p1 - 1;
+    int cnt = 0;   // entries in the lane's queue
     auto drain = [&]() {
         const int kmax = __reduce_max_sync(0xffffffffu, cnt);
         for (int k = 0; k < kmax; ++k) {
             if (k < cnt) {
                 const uint32_t e = q[k][lane];
                 const int j = (int)(e & (uint32_t)(kDirectMaxN - 1));
-                const int img = (int)(e >> 27);
+                const int code = (int)(e >> 27);
                 float4 hj = __ldg(&cv.posh[j]);
                 Aux aj = g_aux[j];
-                if (img != kDirectCentre)
-                    body.image(hj, aj, img % 3 - 1, (img / 3) % 3 - 1, img / 9 - 1, g);
+                if (code != kDirectCentre)
+                    body.image(hj, aj, code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1, g);
                 body.eval(hj, aj, hs, acc, err);
             }
         }
         body.fold(acc);
         cnt = 0;
     };
-    for (int row = 0; row < 9; ++row) {
-        const int dz = row / 3 - 1, dy = row % 3 - 1;
-        int sy, sz;
-        const int y = wrap_cell(cy + dy, g.s, sy);
-        const int z = wrap_cell(cz + dz, g.s, sz);
-        const int base = g.c0 + g.s * y + g.s2 * z;
+    const bool edge = active && (cx == 0 || cx == g.s - 1);
+    const bool any_edge = __any_sync(0xffffffffu, edge);
 #pragma unroll 1
-        for (int part = 0; part < 2; ++part) {
-            // part 0: the cells of [cx-1, cx+1] inside the grid, contiguous;
-            // part 1: the one cell that wraps around in x (if any)
-            int a = 0, len = 0, sx = 0;
-            if (active) {
-                if (part == 0) {
-                    const int xa = cx > 0 ? cx - 1 : 0;
-                    const int xb = cx < g.s - 1 ? cx + 1 : g.s - 1;
-                    a = cv.cstart[base + xa];
-                    len = cv.cstart[base + xb] + cv.ccount[base + xb] - a;
-                } else if (cx == 0 || cx == g.s - 1) {
-                    const int xw = cx == 0 ? g.s - 1 : 0;
-                    sx = cx == 0 ? -1 : 1;
-                    a = cv.cstart[base + xw];
-                    len = cv.ccount[base + xw];
-                }
-            }
-            const int lmax = __reduce_max_sync(0xffffffffu, len);
-            if (lmax == 0) continue;
-            // the neighbour's image is +s L: x_j + s L - x_i
-            const float hx = hi.x - (float)sx * g.Lhi;
+    for (int dz = -1; dz <= 1; ++dz) {
+        int sz;
+        const int z = wrap_near(cz + dz, g.s, sz);
+#pragma unroll 1
+        for (int dy = -1; dy <= 1; ++dy) {
+            int sy;
+            const int y = wrap_near(cy + dy, g.s, sy);
+            const int base = g.c0 + g.s * y + g.s2 * z;
             const float hy = hi.y - (float)sy * g.Lhi;
             const float hz = hi.z - (float)sz * g.Lhi;
-            const uint32_t code = (uint32_t)((sx + 1) + 3 * (sy + 1) + 9 * (sz + 1)) << 27;
-            for (int t0 = 0; t0 < lmax; t0 += kUnroll) {
-#pragma unroll
-                for (int u = 0; u < kUnroll; ++u) {
-                    const int t = t0 + u;
-                    const int j = min(a + t, jlast);
-                    const float4 hj = __ldg(&cv.posh[j]);
-                    const float ex = hj.x - hx, ey = hj.y - hy, ez = hj.z - hz;
-                    const float r2 = ex * ex + ey * ey + ez * ez;
-                    const bool in = (t < len) & (r2 < pre_rc2) & (j != i);
-                    q[cnt][lane] = (uint32_t)j | code;
-                    cnt += in ? 1 : 0;
+            // part 0: the cells of [cx-1, cx+1] inside the grid, contiguous;
+            // part 1: the one cell that wraps around in x (if any)
+#pragma unroll 1
+            for (int part = 0; part < (any_edge ? 2 : 1); ++part) {
+                int a = 0, len = 0, sx = 0;
+                if (part == 0 ? active : edge) {
+                    if (part != 0) sx = cx == 0 ? -1 : 1;
+                    const int xa = part == 0 ? max(cx - 1, 0) : (cx == 0 ? g.s - 1 : 0);
+                    const int xb = part == 0 ? min(cx + 1, g.s - 1) : xa;
+                    a = cv.cstart[base + xa];
+                    len = cv.cstart[base + xb] + cv.ccount[base + xb] - a;
                 }
-                // at most kQueue - kUnroll entries before a batch of
-                // kUnroll: slots stay below kQueueCap
-                if (__any_sync(0xffffffffu, cnt > kQueue - kUnroll)) drain();
+                const int lmax = __reduce_max_sync(0xffffffffu, len);
+                // the neighbour's image is +s L: x_j + s L - x_i
+                const float hx = hi.x - (float)sx * g.Lhi;
+                uint32_t e =
+                    (uint32_t)a | (uint32_t)((sx + 1) + 3 * (sy + 1) + 9 * (sz + 1)) << 27;
+                const int self = i - a;   // the home particle is this candidate of its run
+                const float4* pp = cv.posh + a;
+                for (int t0 = 0; t0 < lmax; t0 += kUnroll, pp += kUnroll, e += kUnroll) {
+                    const int rem = len - t0, me = self - t0;
+                    float4 hj[kUnroll];
+#pragma unroll
+                    for (int u = 0; u < kUnroll; ++u)
+                        if (u < rem) hj[u] = __ldg(pp + u);
+#pragma unroll
+                    for (int u = 0; u < kUnroll; ++u) {
+                        const float ex = hj[u].x - hx, ey = hj[u].y - hy, ez = hj[u].z - hz;
+                        const float r2 = ex * ex + ey * ey + ez * ez;
+                        const bool in = (u < rem) & (r2 < pre_rc2) & (u != me);
+                        q[cnt][lane] = e + u;
+                        cnt += in ? 1 : 0;
+                    }
+                    // at most kQueue - kUnroll entries before a batch of kUnroll:
+                    // slots stay below kQueueCap
+                    if (__any_sync(0xffffffffu, cnt > kQueue - kUnroll)) drain();
+                }
             }
         }
     }
@@ -330,8 +333,8 @@ force_direct_kernel(Body body, DevGeom g, CellView cv, ForceOut out, float pre_r
     __shared__ uint32_t s_q[kForceWarps][kQueueCap][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (pass_failed(out, lane)) return;  // warp-uniform
-    force_direct_warp(body, g, cv, out, pre_rc2, blockIdx.x * blockDim.x + threadIdx.x, lane,
-                      s_q[w]);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    force_direct_warp(body, g, cv, out, pre_rc2, i, i < g.p1, lane, s_q[w]);
 }
 
 // The FP64 form's 27-cell walk: four lanes a particle, eight particles a warp.
@@ -503,7 +506,8 @@ force_batch_kernel(Body body0, CellView cv, ForceOut out, BatchView bv, int walk
     const DevGeom g = bv.geoms[t.x];
     const Body body = body0.for_replica(bv.pairs, t.x, g);
     if (direct_walk(g, walk))   // the rule a single system of this replica follows
-        force_direct_warp(body, g, cv, out, bv.pre[t.x], t.y + lane, lane, s_q[w]);
+        force_direct_warp(body, g, cv, out, bv.pre[t.x], t.y + lane, t.y + lane < g.p1, lane,
+                          s_q[w]);
     else
         force_pass_warp(body, g, cv, out, bv.pre[t.x], t.y + lane, lane, s_hi[w], s_aux[w],
                         s_q[w]);
