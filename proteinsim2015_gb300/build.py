@@ -4,6 +4,8 @@ Translation units are compiled in parallel with one -gencode each:
   psim_exact.cu  --fmad=false (FP64 update and plain force form keep the
                  reference's two-rounding a*b+c)
   psim_mixed.cu  FP32 pair math (contraction allowed)
+  psim_step.cu   the mixed form's list step as one kernel (as psim_mixed.cu)
+  psim_list_build.cu  the pair list's build
   psim_cells.cu  integer counting sort and layout conversions
   psim_api.cu    host side of the C ABI
   psim_noalloc.cu  the cell-list build on a static device scratch array
@@ -26,6 +28,8 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = {
     "psim_exact.cu": ["--fmad=false"],
     "psim_mixed.cu": [],
+    "psim_step.cu": [],
+    "psim_list_build.cu": [],
     "psim_cells.cu": [],
     "psim_api.cu": [],
     "psim_noalloc.cu": [],

@@ -1164,7 +1164,8 @@ struct psim_system {
     bool snap_pending = false;
     // one graph per buffer phase (one step), and one of kGraphSteps steps
     // starting at phase 0 (fewer graph launches for small systems)
-    cudaGraphExec_t graph[6] = {};
+    // (fused: normal steps in the one kernel of psim_step.cu)
+    cudaGraphExec_t graph[6] = {}, fused[6] = {};
     cudaGraphExec_t graph_multi = nullptr;
     uint32_t latched = 0;
     // Verlet pair list of the mixed form (list_on): list slot of each storage
@@ -1175,7 +1176,9 @@ struct psim_system {
     double skin = 0.0;
     int lcap = 0, hcap = 0;
     float lpre = 0.f, ldisp2 = 0.f, hr = 0.f;
-    DevBuf lslot[2], lbuild, lpos, list, lcount, lflag, lhalo, lhcount;
+    // the records (lpos) ping-pong with the step's parity: a step reads one buffer and
+    // writes the next step's
+    DevBuf lslot[2], lbuild, lpos[2], list, lcount, lflag, lhalo, lhcount;
     // With a pair list the cell list is rebuilt only with the list (the
     // storage order then stays the list order between builds): the state is
     // carried into the new order through pscratch (15 n doubles), and the
@@ -1228,10 +1231,11 @@ double* d3(DevBuf& b, int n, int k) { return b.as<double>() + (size_t)k * n; }
 
 // The list-order records the canonicalisation writes when the list is
 // rebuilt: positions, build positions and halo images.
-void set_halo_args(psim_system* s, CanonArgs& ca) {
+// t: the step that reads the records.
+void set_halo_args(psim_system* s, CanonArgs& ca, long long t) {
     ca.xorder = 1;   // each row of cells sorted by x: the list build trims its runs
     ca.lbuild = s->lbuild.as<float4>();
-    ca.lpos = s->lpos.as<float4>();
+    ca.lpos = s->lpos[t & 1].as<float4>();
     ca.linv_unit = s->lcompact ? 1.0f / s->lunit : 0.f;
     ca.lhalo = s->lhalo.as<int>();
     ca.lhcount = s->lhcount.as<int>();
@@ -1263,6 +1267,19 @@ cudaError_t enqueue_list_build(psim_system* s, int cb, const int* gate) {
     return launch_list_build(s->g, cv, lb, s->err.as<uint32_t>(), s->st);
 }
 
+// The pair list of the state at phase ph (the storage order is the list order: no
+// slot table); in a batch, with each particle's replica and its pair functor.
+PairList pair_list(psim_system* s, const Phase& ph) {
+    PairList pl{nullptr, s->lpos[ph.sb].as<float4>(), s->lcount.as<int>(), s->list.as<uint32_t>(),
+                s->n, s->lcompact, s->lradius, s->lunit};
+    if (s->n_reps) {
+        pl.rep = s->b_rep.as<int>();
+        pl.pairs = s->b_pairs.p;
+    }
+    pl.lanes = s->list_lanes;
+    return pl;
+}
+
 // The force pass on the state after `total` steps (phase ph): the cell walk,
 // or the pair list in the mixed form with a skin; forces in storage order.
 cudaError_t enqueue_force(psim_system* s, const Phase& ph, const ForceOut& fo) {
@@ -1273,18 +1290,12 @@ cudaError_t enqueue_force(psim_system* s, const Phase& ph, const ForceOut& fo) {
         if (s->cfg.precision == PSIM_PRECISION_FP64)
             return fr.run(PSIM_PASS_FP64, s->g, &cv, nullptr, fo, s->st);
         if (s->list_on) {
-            PairList pl{nullptr, s->lpos.as<float4>(), s->lcount.as<int>(),
-                        s->list.as<uint32_t>(), s->n, s->lcompact, s->lradius, s->lunit};
+            const PairList pl = pair_list(s, ph);
             return fr.run(PSIM_PASS_LIST, s->g, nullptr, &pl, fo, s->st);
         }
         return fr.run(PSIM_PASS_MIXED, s->g, &cv, nullptr, fo, s->st);
     }
-    if (s->n_reps && s->list_on) {   // each particle with its replica's pair functor
-        PairList pl{nullptr, s->lpos.as<float4>(), s->lcount.as<int>(), s->list.as<uint32_t>(),
-                    s->n, s->lcompact, s->lradius, s->lunit, s->b_rep.as<int>(), s->b_pairs.p};
-        pl.lanes = s->list_lanes;
-        return launch_forces_list(s->fs, s->g, pl, fo, s->st);
-    }
+    if (s->list_on) return launch_forces_list(s->fs, s->g, pair_list(s, ph), fo, s->st);
     if (s->n_reps) {
         BatchView bv{s->b_tasks.as<int2>(), s->n_tasks, s->b_geoms.as<DevGeom>(),
                      s->b_pairs.p, s->b_pre.as<float>()};
@@ -1293,13 +1304,6 @@ cudaError_t enqueue_force(psim_system* s, const Phase& ph, const ForceOut& fo) {
         return launch_forces_mixed(s->fs, s->g, cv, fo, s->st, &bv);
     }
     if (s->cfg.precision == PSIM_PRECISION_FP64) return launch_forces_fp64(s->fs, s->g, cv, fo, s->st);
-    if (s->list_on) {
-        // the storage order is the list order: no slot table
-        PairList pl{nullptr, s->lpos.as<float4>(), s->lcount.as<int>(),
-                    s->list.as<uint32_t>(), s->n, s->lcompact, s->lradius, s->lunit};
-        pl.lanes = s->list_lanes;
-        return launch_forces_list(s->fs, s->g, pl, fo, s->st);
-    }
     return launch_forces_mixed(s->fs, s->g, cv, fo, s->st);
 }
 
@@ -1349,7 +1353,7 @@ int enqueue_rebuild_lazy(psim_system* s, long long t) {
     ca.posh = s->posh.as<float4>();
     ca.vel_freq = s->vp.vel_freq;
     ca.err = err;
-    set_halo_args(s, ca);   // list records, build positions and halo images on the new order
+    set_halo_args(s, ca, t + 1);   // list records, build positions and halo images on the new order
     PSIM_CUDA(launch_canonicalize(ca, st));
     // the state into the new order: positions, previous positions, noise
     // memory, and the forces of this step and the one before
@@ -1379,9 +1383,10 @@ int enqueue_rebuild_lazy(psim_system* s, long long t) {
 }
 
 // Step t with a pair list.  In a graph (evs null) this enqueues the force
-// pass, the integrator and the step end; the caller adds the conditional
-// rebuild.  Timed directly (evs: 4 events), the rebuild decision is read back.
-int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs) {
+// pass and the integrator (or, fused, the one kernel of both) and the step end;
+// the caller adds the conditional rebuild.  Timed directly (evs: 4 events), the
+// rebuild decision is read back.
+int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs, bool fused = false) {
     const Phase ph = phase_of(t);
     const int n = s->n, sb = ph.sb, nsb = 1 - ph.sb;
     cudaStream_t st = s->st;
@@ -1389,7 +1394,7 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs) {
     if (evs) PSIM_CUDA(cudaEventRecord(evs[0], st));
     ForceOut fo{d3(s->frc[ph.fcur], n, 0), d3(s->frc[ph.fcur], n, 1), d3(s->frc[ph.fcur], n, 2),
                 s->err.as<uint32_t>(), nullptr};
-    PSIM_CUDA(enqueue_force(s, ph, fo));
+    if (!fused) PSIM_CUDA(enqueue_force(s, ph, fo));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[1], st));
     VgbSystemArgs a{};
     a.n = n;
@@ -1400,6 +1405,7 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs) {
     a.x0 = d3(s->pos0[sb], n, 0); a.y0 = d3(s->pos0[sb], n, 1); a.z0 = d3(s->pos0[sb], n, 2);
     a.mx = d3(s->mem[sb], n, 0); a.my = d3(s->mem[sb], n, 1); a.mz = d3(s->mem[sb], n, 2);
     a.fx = fo.fx; a.fy = fo.fy; a.fz = fo.fz;
+    a.ofx = fo.fx; a.ofy = fo.fy; a.ofz = fo.fz;
     a.gx = d3(s->frc[ph.fprev], n, 0); a.gy = d3(s->frc[ph.fprev], n, 1);
     a.gz = d3(s->frc[ph.fprev], n, 2);
     a.vel = s->vel.as<double>();
@@ -1411,7 +1417,7 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs) {
     a.state = s->state.as<StepState>();
     a.lslot = nullptr;  // list slot = storage slot
     a.lbuild = s->lbuild.as<float4>();
-    a.lpos = s->lpos.as<float4>();
+    a.lpos = s->lpos[nsb].as<float4>();
     a.linv_unit = s->lcompact ? 1.0f / s->lunit : 0.f;
     a.lflag_set = lflag;
     a.lflag_clear = s->lflag.as<int>() + (1 - (t & 1));
@@ -1425,7 +1431,10 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs) {
         a.seeds = s->b_seeds.as<uint32_t>();
     }
     NoiseView nz{s->cfg.noise_mode, s->noise.as<double>(), s->noise_first, s->noise_steps};
-    PSIM_CUDA(launch_vgb_system_fast(a, s->vp, s->g, nz, st));
+    if (fused)
+        PSIM_CUDA(launch_step_list(s->fs, s->g, pair_list(s, ph), a, s->vp, nz, st));
+    else
+        PSIM_CUDA(launch_vgb_system_fast(a, s->vp, s->g, nz, st));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[2], st));
     PSIM_CUDA(launch_step_end(s->state.as<StepState>(), lflag, s->err.as<uint32_t>(),
                               s->vp.vel_freq, s->cond, evs ? 0 : 1, st));
@@ -1451,8 +1460,6 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     cudaStream_t st = s->st;
     const int sb = ph.sb, nsb = 1 - ph.sb, ob = ph.ob, nob = 1 - ph.ob, cb = ph.cb, ncb = 1 - ph.cb;
     const int pb = ph.pb, npb = 1 - ph.pb;
-    // the rebuild flag of this step's parity (pair list only)
-    int* lflag = s->list_on ? s->lflag.as<int>() + (t & 1) : nullptr;
     if (evs) PSIM_CUDA(cudaEventRecord(evs[0], st));
     ForceOut fo{d3(s->frc[ph.fcur], n, 0), d3(s->frc[ph.fcur], n, 1), d3(s->frc[ph.fcur], n, 2),
                 s->err.as<uint32_t>(), nullptr};
@@ -1480,17 +1487,6 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     a.count = s->count[ncb].as<int>();
     a.err = s->err.as<uint32_t>();
     a.state = s->state.as<StepState>();
-    if (s->list_on) {
-        a.lslot = s->lslot[ob].as<int>();
-        a.lbuild = s->lbuild.as<float4>();
-        a.lpos = s->lpos.as<float4>();
-        a.linv_unit = s->lcompact ? 1.0f / s->lunit : 0.f;
-        a.lflag_set = lflag;
-        a.lflag_clear = s->lflag.as<int>() + (1 - (t & 1));
-        a.ldisp2 = s->ldisp2;
-        a.lhalo = s->lhalo.as<int>();
-        a.lhcount = s->lhcount.as<int>();
-    }
     if (s->n_reps) {
         a.rep = s->b_rep.as<int>();
         a.geoms = s->b_geoms.as<DevGeom>();
@@ -1530,14 +1526,7 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     ca.advance = 1;
     ca.vel_freq = s->vp.vel_freq;
     ca.err = s->err.as<uint32_t>();
-    if (s->list_on) {
-        ca.rebuild = lflag;
-        ca.lslot_in = s->lslot[ob].as<int>();
-        ca.lslot_out = s->lslot[nob].as<int>();
-        set_halo_args(s, ca);
-    }
     PSIM_CUDA(launch_canonicalize(ca, st));
-    if (s->list_on) PSIM_CUDA(enqueue_list_build(s, ncb, lflag));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[3], st));
     return PSIM_OK;
 }
@@ -1547,7 +1536,7 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
 // Steps phase .. phase + steps - 1 with a pair list, captured into one graph:
 // each step's kernels followed by a conditional node whose body is that
 // step's rebuild (the step end sets the node's condition).
-int graph_lazy_steps(psim_system* s, int phase, int steps, cudaGraphExec_t* out) {
+int graph_lazy_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_t* out) {
     cudaGraph_t g = nullptr;
     PSIM_CUDA(cudaGraphCreate(&g, 0));
     auto done = [&](int rc) {
@@ -1569,7 +1558,7 @@ int graph_lazy_steps(psim_system* s, int phase, int steps, cudaGraphExec_t* out)
     int rc = PSIM_OK;
     for (int k = 0; k < steps && !rc; ++k) {
         s->cond = conds[k];
-        rc = enqueue_step_lazy(s, phase + k, nullptr);
+        rc = enqueue_step_lazy(s, phase + k, nullptr, fused);
         if (rc) break;
         cudaStreamCaptureStatus cs;
         const cudaGraphNode_t* deps = nullptr;
@@ -1618,8 +1607,8 @@ int graph_lazy_steps(psim_system* s, int phase, int steps, cudaGraphExec_t* out)
 }
 
 // Steps phase .. phase + steps - 1, captured into one graph.
-int graph_steps(psim_system* s, int phase, int steps, cudaGraphExec_t* out) {
-    if (s->list_on) return graph_lazy_steps(s, phase, steps, out);
+int graph_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_t* out) {
+    if (s->list_on) return graph_lazy_steps(s, phase, steps, fused, out);
     cudaGraph_t g = nullptr;
     PSIM_CUDA(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSIM_OK;
@@ -1633,19 +1622,53 @@ int graph_steps(psim_system* s, int phase, int steps, cudaGraphExec_t* out) {
     return PSIM_OK;
 }
 
-int graph_for(psim_system* s, int phase, cudaGraphExec_t* out) {
-    if (!s->graph[phase]) {
-        int rc = graph_steps(s, phase, 1, &s->graph[phase]);
-        if (rc) return rc;
-    }
-    *out = s->graph[phase];
-    return PSIM_OK;
+// Whether the normal steps of s run in the one kernel of psim_step.cu.
+bool fused_steps(const psim_system* s) {
+    return s->list_on && s->lcompact && s->list_lanes == 1 && !s->cfg.force_launch && !s->img.p;
 }
+// The velocity counter's period: step t > 0 writes the velocities when it
+// divides t; step 0 is the first step.
+bool normal_step(const psim_system* s, long long t) { return t % (s->vp.vel_freq + 1LL) != 0; }
 
 void drop_graphs(psim_system* s) {
-    for (auto& g : s->graph)
-        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-    if (s->graph_multi) { cudaGraphExecDestroy(s->graph_multi); s->graph_multi = nullptr; }
+    auto drop = [](cudaGraphExec_t& g) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    };
+    for (auto& g : s->graph) drop(g);
+    for (auto& g : s->fused) drop(g);
+    drop(s->graph_multi);
+}
+
+// The graphs of n_steps steps from the system's step on, in order: visit(graph,
+// phase, steps, fused).  kGraphSteps steps at a time where a buffer period begins
+// and all of them are of one kind, else single steps.  (A system whose velocity
+// steps come at least every kGraphSteps steps has no run of fused ones that long:
+// its multi-step graph is unfused.)
+template <class Visit>
+int each_graph(psim_system* s, int n_steps, Visit&& visit) {
+    const bool fuse = fused_steps(s), one_kind = !fuse || s->vp.vel_freq < kGraphSteps - 1;
+    const bool multi = s->graph_multi || n_steps >= kGraphSteps + 5;
+    int rc = PSIM_OK;
+    for (long long t = s->total, end = t + n_steps; t < end && !rc;) {
+        bool run = multi && t % 6 == 0 && end - t >= kGraphSteps;
+        for (int k = 0; run && !one_kind && k < kGraphSteps; ++k) run = normal_step(s, t + k);
+        const bool fused = fuse && (run ? !one_kind : normal_step(s, t));
+        const int phase = (int)(t % 6), steps = run ? kGraphSteps : 1;
+        rc = visit(run ? s->graph_multi : (fused ? s->fused[phase] : s->graph[phase]), phase, steps,
+                   fused);
+        t += steps;
+    }
+    return rc;
+}
+
+// The graphs of the next n_steps steps that are not captured yet.
+int capture_graphs(psim_system* s, int n_steps) {
+    return each_graph(s, n_steps, [&](cudaGraphExec_t& g, int phase, int steps, bool fused) {
+        if (g) return (int)PSIM_OK;
+        PSIM_CUDA(cudaStreamSynchronize(s->st));
+        return graph_steps(s, phase, steps, fused, &g);
+    });
 }
 
 struct DeviceGuard {
@@ -1908,7 +1931,8 @@ psim_system* psim_batch_create_list(const psim_replica* reps, int32_t n_reps,
                          put(s->b_lpre, lpre.data(), lpre.size() * sizeof(float)) &&
                          put(s->b_hr, hr.data(), hr.size() * sizeof(float)) &&
                          !s->list.ensure(4 * n * (size_t)(cap + kListFold)) &&
-                         !s->lpos.ensure(32 * (n + 1 + (size_t)s->hcap));
+                         !s->lpos[0].ensure(32 * (n + 1 + (size_t)s->hcap)) &&
+                         !s->lpos[1].ensure(32 * (n + 1 + (size_t)s->hcap));
         if (!ok2) {
             fail(PSIM_ERR_INPUT, "the batch's pair list does not fit (%lld particles, %d entries "
                  "each)", (long long)P, cap);
@@ -2007,7 +2031,8 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
         ok = !s->posl.ensure(16 * n);
     if (ok && list_on) {
         ok = !s->lslot[0].ensure(4 * n) && !s->lslot[1].ensure(4 * n) && !s->lbuild.ensure(16 * n) &&
-             !s->lpos.ensure(32 * (n + 1 + (size_t)s->hcap)) &&
+             !s->lpos[0].ensure(32 * (n + 1 + (size_t)s->hcap)) &&
+             !s->lpos[1].ensure(32 * (n + 1 + (size_t)s->hcap)) &&
              !s->list.ensure(4 * n * (size_t)(s->lcap + kListFold)) && !s->lcount.ensure(4 * n) &&
              !s->lflag.ensure(8) && !s->lhalo.ensure(4 * n) && !s->lhcount.ensure(4) &&
              !s->pscratch.ensure(15 * 8 * (size_t)n) &&
@@ -2037,7 +2062,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
             const ForceRunner fr{&s->fs, cfg->force_launch, &s->cfg.force};
             CellView cv{s->posd.as<double4_32a>(), s->posh.as<float4>(), s->posl.as<float4>(),
                         s->cellid.as<int>(), s->start.as<int>(), s->count[0].as<int>()};
-            PairList pl{nullptr, s->lpos.as<float4>(), s->lcount.as<int>(),
+            PairList pl{nullptr, s->lpos[0].as<float4>(), s->lcount.as<int>(),
                         s->list.as<uint32_t>(), s->n, 0, 0.f, 0.f};
             const int pass = cfg->precision == PSIM_PRECISION_FP64
                                  ? PSIM_PASS_FP64
@@ -2067,7 +2092,7 @@ void psim_system_destroy(psim_system* s) {
     drop_graphs(s);
     DevBuf* arrs[] = {&s->cellid, &s->key, &s->rank, &s->tmp, &s->start, &s->scratch, &s->posd,
                       &s->posh, &s->posl, &s->vel, &s->err, &s->state, &s->occ, &s->noise,
-                      &s->snap, &s->lslot[0], &s->lslot[1], &s->lbuild, &s->lpos, &s->list,
+                      &s->snap, &s->lslot[0], &s->lslot[1], &s->lbuild, &s->lpos[0], &s->lpos[1], &s->list,
                       &s->lcount, &s->lflag, &s->lhalo, &s->lhcount, &s->pscratch, &s->b_tasks,
                       &s->b_geoms, &s->b_pairs, &s->b_pre, &s->b_rep, &s->b_seeds,
                       &s->img, &s->track_start, &s->b_lpre, &s->b_hr};
@@ -2173,14 +2198,15 @@ int psim_system_upload(psim_system* s, const double* pos, const double* pos0, co
         const float4 ghost[2] = {compact ? make_float4(0.f, 0.f, 0.f, kGhostBias)
                                          : make_float4(1e18f, 1e18f, 1e18f, R),
                                  make_float4(0.f, 0.f, 0.f, 0.f)};
-        float4* grec = s->lpos.as<float4>() + (compact ? 1 : 2) * (size_t)n;
-        PSIM_CUDA(cudaMemcpyAsync(grec, ghost, compact ? 16 : 32, cudaMemcpyHostToDevice, st));
+        for (DevBuf& b : s->lpos)
+            PSIM_CUDA(cudaMemcpyAsync(b.as<float4>() + (compact ? 1 : 2) * (size_t)n, ghost,
+                                      compact ? 16 : 32, cudaMemcpyHostToDevice, st));
     }
     if (s->list_on) {
         // the first list, on the first cell order (the list slots are the
         // storage slots: the state is carried into that order below)
         PSIM_CUDA(cudaMemsetAsync(s->lflag.p, 0, 8, st));
-        set_halo_args(s, ca);
+        set_halo_args(s, ca, 0);
         PSIM_CUDA(cudaMemsetAsync(s->lhcount.p, 0, 4, st));
     }
     PSIM_CUDA(launch_canonicalize(ca, st));
@@ -2241,35 +2267,12 @@ int psim_system_step_async(psim_system* s, int32_t n_steps) {
     if (s->latched) return fail(code_from_bits(s->latched), "%s", bits_text(s->latched));
     if (n_steps < 0) return fail(PSIM_ERR_INPUT, "negative step count");
     DeviceGuard dg(s->device);
-    for (int ph = 0; ph < 6 && n_steps > 0; ++ph) {  // capture before anything is in flight
-        cudaGraphExec_t ge;
-        if (!s->graph[ph]) {
-            PSIM_CUDA(cudaStreamSynchronize(s->st));
-            int rc = graph_for(s, ph, &ge);
-            if (rc) return rc;
-        }
-    }
-    if (n_steps >= kGraphSteps + 5 && !s->graph_multi) {
-        PSIM_CUDA(cudaStreamSynchronize(s->st));
-        int rc = graph_steps(s, 0, kGraphSteps, &s->graph_multi);
-        if (rc) return rc;
-    }
-    // single steps up to a multiple of 6, then kGraphSteps steps per launch
-    while (n_steps > 0) {
-        if (s->graph_multi && s->total % 6 == 0 && n_steps >= kGraphSteps) {
-            PSIM_CUDA(cudaGraphLaunch(s->graph_multi, s->st));
-            s->total += kGraphSteps;
-            n_steps -= kGraphSteps;
-            continue;
-        }
-        cudaGraphExec_t ge;
-        int rc = graph_for(s, (int)(s->total % 6), &ge);
-        if (rc) return rc;
-        PSIM_CUDA(cudaGraphLaunch(ge, s->st));
-        s->total++;
-        --n_steps;
-    }
-    return PSIM_OK;
+    if (int rc = capture_graphs(s, n_steps)) return rc;   // before anything is in flight
+    return each_graph(s, n_steps, [&](cudaGraphExec_t& g, int, int steps, bool) {
+        PSIM_CUDA(cudaGraphLaunch(g, s->st));
+        s->total += steps;
+        return (int)PSIM_OK;
+    });
 }
 
 int psim_system_sync(psim_system* s) {
@@ -2765,9 +2768,10 @@ int psim_system_profile(psim_system* s, int32_t n_steps, double* out_ms) {
 
 int psim_system_launches_per_step(psim_system* s) {
     // force, vGB, scan x3, scatter, canonicalise (+1 memset node); with a
-    // pair list: force, vGB, step end (the rebuild's kernels run on the
-    // steps that rebuild: psim_system_launches_per_rebuild)
-    return (s && s->list_on) ? 3 : 7;
+    // pair list: force, vGB (one kernel on normal steps where fused_steps
+    // allows), step end (the rebuild's kernels run on the steps that rebuild:
+    // psim_system_launches_per_rebuild)
+    return (s && s->list_on) ? (fused_steps(s) ? 2 : 3) : 7;
 }
 
 int psim_system_launches_per_rebuild(psim_system* s) {
@@ -2800,17 +2804,7 @@ int psim_system_time_steps(psim_system* s, int32_t n_steps, double* ms) {
     // capture the graphs first so the timed region holds only launches
     int rc = psim_system_step_async(s, 0);
     if (rc) return rc;
-    for (int ph = 0; ph < 6; ++ph) {
-        cudaGraphExec_t ge;
-        if (!s->graph[ph]) {
-            PSIM_CUDA(cudaStreamSynchronize(s->st));
-            if ((rc = graph_for(s, ph, &ge))) return rc;
-        }
-    }
-    if (n_steps >= kGraphSteps + 5 && !s->graph_multi) {
-        PSIM_CUDA(cudaStreamSynchronize(s->st));
-        if ((rc = graph_steps(s, 0, kGraphSteps, &s->graph_multi))) return rc;
-    }
+    if (n_steps > 0 && (rc = capture_graphs(s, n_steps))) return rc;
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     PSIM_CUDA(cudaEventRecord(s->ev[0], s->st));
     if ((rc = psim_system_step_async(s, n_steps))) return rc;

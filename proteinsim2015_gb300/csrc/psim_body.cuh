@@ -387,12 +387,52 @@ struct MixedBody {
     // the compensated sum s - k formed in FP64 (exact: both parts fit 48
     // bits); the floats are widened with integer operations, as the FP64
     // unit that would convert them runs at 1/64 of the FP32 rate on GB300
+    __device__ __forceinline__ void sum(const Acc& a, double F[3]) const {
+        F[0] = widen_f32(a.s0) - widen_f32(a.k0);
+        F[1] = widen_f32(a.s1) - widen_f32(a.k1);
+        F[2] = widen_f32(a.s2) - widen_f32(a.k2);
+    }
     __device__ __forceinline__ void store(const ForceOut& out, int i, const Acc& a) const {
-        out.fx[i] = widen_f32(a.s0) - widen_f32(a.k0);
-        out.fy[i] = widen_f32(a.s1) - widen_f32(a.k1);
-        out.fz[i] = widen_f32(a.s2) - widen_f32(a.k2);
+        double F[3];
+        sum(a, F);
+        out.fx[i] = F[0];
+        out.fy[i] = F[1];
+        out.fz[i] = F[2];
         if (out.coor) out.coor[i] = a.cnt;
     }
 };
+
+// The plugin's pair functor handed to run(pair, rc2f): LennardJones without
+// a Yukawa term gets its exponent fixed at compile time for the common ljNum
+// values 6, 12 and 18, the pure Yukawa form (ljNum 0) likewise; other
+// LennardJones settings run the general functor.
+template <class Run>
+cudaError_t with_pair(const ForceSetup& fs, Run&& run) {
+    switch (fs.kind) {
+    case 1: return run(fs.ao, fs.ao.rc2f);
+    case 2: {
+        auto fixed = [&](auto p) {
+            static_cast<LJPair&>(p) = fs.lj;
+            return run(p, fs.lj.rc2f);
+        };
+        if (fs.lj_pure) {
+            switch (fs.lj.n) {
+            case 6: return fixed(LJPure<6>{});
+            case 12: return fixed(LJPure<12>{});
+            case 18: return fixed(LJPure<18>{});
+            }
+        }
+        if (fs.lj.n == 0) return fixed(LJFixed<0>{});
+        return run(fs.lj, fs.lj.rc2f);
+    }
+    case 3: return run(fs.cal, fs.cal.rc2f);
+    case 4: {
+        const float rc2f = fs.ao.rc2f > fs.lj.rc2f ? fs.ao.rc2f : fs.lj.rc2f;
+        return run(ComboPairF{fs.ao, fs.lj}, rc2f);
+    }
+    }
+    return cudaErrorInvalidValue;
+}
+
 
 }  // namespace psim

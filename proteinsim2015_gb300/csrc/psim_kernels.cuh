@@ -171,6 +171,7 @@ struct VgbSystemArgs {
     const double* mx; const double* my; const double* mz;    // memX/Y/Z
     const double* fx; const double* fy; const double* fz;    // F, current order
     const double* gx; const double* gy; const double* gz;    // F0, previous order
+    double* ofx; double* ofy; double* ofz;                   // F (out, launch_step_list)
     double* vel;                // 3n, original order (tag-indexed)
     double* ox; double* oy; double* oz;                      // new pos, current order
     double* ox0; double* oy0; double* oz0;
@@ -210,6 +211,12 @@ cudaError_t launch_vgb_system(const VgbSystemArgs& a, const VgbParams& p, const 
 // The same update with FMA contraction (psim_mixed.cu), for the mixed form.
 cudaError_t launch_vgb_system_fast(const VgbSystemArgs& a, const VgbParams& p, const DevGeom& g,
                                    const NoiseView& nz, cudaStream_t st);
+
+// The list force pass and the update of a normal step in one kernel (psim_step.cu):
+// reads the records pl.pos and writes the new ones to a.lpos, another buffer.
+cudaError_t launch_step_list(const ForceSetup& fs, const DevGeom& g, const PairList& pl,
+                             const VgbSystemArgs& a, const VgbParams& p, const NoiseView& nz,
+                             cudaStream_t st);
 
 // Reference-layout integrator (brownianIntegrator::nextSystem on AoS arrays
 // in original order).  mem/mem_corr: 3n device arrays owned by the integrator.

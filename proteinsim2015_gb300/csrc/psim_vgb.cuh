@@ -358,6 +358,35 @@ __device__ __forceinline__ void vgb_system_one(const VgbSystemArgs& a, const Vgb
     if (err) atomicOr(a.err, err);
 }
 
+// vgb_system_one for a normal step of the mixed form between two list rebuilds (no
+// permutation, hash, velocities or image counts) with the force F in hand.
+__device__ __forceinline__ void vgb_normal_one(const VgbSystemArgs& a, const VgbParams& p,
+                                               const DevGeom& g, const NoiseView& nz, int f,
+                                               const double F[3], uint32_t err) {
+    const long long step = a.state->step;
+    const int tag = a.tag[f];
+    const double m = a.inv_mass[f];
+    const double x[3] = {a.x[f], a.y[f], a.z[f]};
+    const double x0[3] = {a.x0[f], a.y0[f], a.z0[f]};
+    double mx[3] = {a.mx[f], a.my[f], a.mz[f]};
+    const double F0[3] = {a.gx[f], a.gy[f], a.gz[f]};
+    const float4 lb = __ldg(a.lbuild + f);
+    const int lhal = __ldg(a.lhalo + f);
+    float xf[6];
+    load_noise_f(nz, p.seed, a.n, tag, tag - g.p0, step, xf, err);
+    double xn[3], x0n[3];
+    vgb_normal_fast(p, g.L, g.half, x, x0, mx, F, F0, xf, m, xn, x0n, err);
+    a.ox[f] = xn[0]; a.oy[f] = xn[1]; a.oz[f] = xn[2];
+    a.ox0[f] = x0n[0]; a.oy0[f] = x0n[1]; a.oz0[f] = x0n[2];
+    a.omx[f] = mx[0]; a.omy[f] = mx[1]; a.omz[f] = mx[2];
+    list_position(a, f, lb, lhal, xn, g);
+    if (f == 0) {
+        *a.lflag_clear = 0;
+        *a.lhcount = 0;   // halo records are handed out afresh at the next build
+    }
+    if (err) atomicOr(a.err, err);
+}
+
 // One system (the geometry is a kernel parameter) or, with kBatch, each
 // particle's replica of a batch (its geometry and Philox seed from tables).
 template <class Tag, bool kBatch>
