@@ -619,8 +619,11 @@ class System:
         _check(lib().psim_system_clusters(self._h, r_contact, int(min_size), _p(root),
                                           C.byref(nc), C.byref(avg)))
         order = np.argsort(root, kind="stable")
-        bounds = np.flatnonzero(np.diff(root[order])) + 1
-        groups = [g for g in np.split(order, bounds) if len(g) > min_size]
+        ends = np.append(np.flatnonzero(np.diff(root[order])) + 1, self.n)
+        starts = np.append(0, ends[:-1])
+        # slices of the clusters asked for only: a state has many small ones
+        big = np.flatnonzero(ends - starts > min_size)
+        groups = [order[i:j] for i, j in zip(starts[big].tolist(), ends[big].tolist())]
         assert len(groups) == nc.value
         return root, groups, avg.value
 

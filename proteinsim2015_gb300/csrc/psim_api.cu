@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -453,6 +454,34 @@ struct DevBuf {
 // A temporary device buffer freed when it leaves scope.
 struct ScopedBuf : DevBuf {
     ~ScopedBuf() { release(); }
+};
+
+// Device scratch of one host-facing call, in the owner's buffer: a cudaMalloc and
+// cudaFree pair costs ~100 us, more than most of what these calls run.  The
+// buffer is kept for the next call up to kKeep bytes and goes with its owner.
+class Scratch {
+public:
+    explicit Scratch(DevBuf& b) : buf_(b) {}
+    ~Scratch() {
+        if (buf_.bytes > kKeep) buf_.release();
+    }
+    // room for blocks of the given sizes; a block's address: at()
+    cudaError_t ensure(std::initializer_list<size_t> sizes) {
+        size_t total = 0;
+        for (size_t b : sizes) {
+            off_.push_back(total);
+            total += (b + 255) & ~(size_t)255;
+        }
+        return buf_.ensure(total);
+    }
+    template <class T> T* at(int k) const {
+        return reinterpret_cast<T*>(buf_.as<char>() + off_[(size_t)k]);
+    }
+
+private:
+    static constexpr size_t kKeep = (size_t)256 << 20;
+    DevBuf& buf_;
+    std::vector<size_t> off_;
 };
 
 // Scratch for the reference-layout drop-ins, grown on demand, one set per
@@ -1202,6 +1231,8 @@ struct psim_system {
     // displacement tracker: box images crossed per particle and the start
     // positions (original order), counted by the integrator once started
     DevBuf img, track_start;
+    DevBuf obs;               // scratch of the host-facing calls (Scratch)
+    uint32_t* host = nullptr; // pinned: the step state and the error word (settle)
 };
 
 namespace {
@@ -1680,11 +1711,12 @@ struct DeviceGuard {
 // Waits for the stream, reads the error word and the device step counter,
 // and re-aligns the host's step count with the steps the device completed.
 int settle(psim_system* s) {
+    PSIM_CUDA(cudaMemcpyAsync(s->host, s->state.p, sizeof(StepState), cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(s->host + 8, s->err.p, 4, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
-    uint32_t bits = 0;
-    StepState ss{};
-    PSIM_CUDA(cudaMemcpy(&bits, s->err.p, 4, cudaMemcpyDeviceToHost));
-    PSIM_CUDA(cudaMemcpy(&ss, s->state.p, sizeof ss, cudaMemcpyDeviceToHost));
+    StepState ss;
+    std::memcpy(&ss, s->host, sizeof ss);
+    const uint32_t bits = s->host[8];
     s->total = ss.step;
     if (bits) {
         s->latched = bits;
@@ -2013,6 +2045,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
               cudaEventCreateWithFlags(&s->ev_snap_ready, cudaEventDisableTiming) == cudaSuccess &&
               cudaEventCreateWithFlags(&s->ev_snap_done, cudaEventDisableTiming) == cudaSuccess;
     for (auto& e : s->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
+    ok = ok && cudaMallocHost(&s->host, 64) == cudaSuccess;
     for (int k = 0; k < 2 && ok; ++k) {
         ok = !s->pos[k].ensure(24 * n) && !s->pos0[k].ensure(24 * n) && !s->mem[k].ensure(24 * n) &&
              !s->tag[k].ensure(4 * n) && !s->radius[k].ensure(8 * n) &&
@@ -2095,7 +2128,7 @@ void psim_system_destroy(psim_system* s) {
                       &s->snap, &s->lslot[0], &s->lslot[1], &s->lbuild, &s->lpos[0], &s->lpos[1], &s->list,
                       &s->lcount, &s->lflag, &s->lhalo, &s->lhcount, &s->pscratch, &s->b_tasks,
                       &s->b_geoms, &s->b_pairs, &s->b_pre, &s->b_rep, &s->b_seeds,
-                      &s->img, &s->track_start, &s->b_lpre, &s->b_hr};
+                      &s->img, &s->track_start, &s->b_lpre, &s->b_hr, &s->obs};
     for (DevBuf* b : arrs) b->release();
     for (int k = 0; k < 2; ++k) {
         s->pos[k].release(); s->pos0[k].release(); s->mem[k].release(); s->tag[k].release();
@@ -2108,6 +2141,7 @@ void psim_system_destroy(psim_system* s) {
     if (s->ev_snap_done) cudaEventDestroy(s->ev_snap_done);
     if (s->st) cudaStreamDestroy(s->st);
     if (s->side) cudaStreamDestroy(s->side);
+    if (s->host) cudaFreeHost(s->host);
     delete s;
 }
 
@@ -2300,13 +2334,14 @@ int psim_system_download(psim_system* s, double* pos, double* pos0, double* vel,
     cudaStream_t st = s->st;
     // storage order is the previous cell order: its tags are tag[1 - ob]
     const int* tg = store_tags(s);
-    ScopedBuf stage;
-    PSIM_CUDA(stage.ensure(b));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({b}));
+    double* stage = mem.at<double>(0);
     auto get3 = [&](DevBuf& src, const int* perm, double* dst) -> int {
         if (!dst) return PSIM_OK;
         PSIM_CUDA(launch_merge_xyz(n, d3(src, n, 0), d3(src, n, 1), d3(src, n, 2), tg, perm,
-                                   stage.as<double>(), st));
-        PSIM_CUDA(cudaMemcpyAsync(dst, stage.p, b, cudaMemcpyDeviceToHost, st));
+                                   stage, st));
+        PSIM_CUDA(cudaMemcpyAsync(dst, stage, b, cudaMemcpyDeviceToHost, st));
         PSIM_CUDA(cudaStreamSynchronize(st));
         return PSIM_OK;
     };
@@ -2319,7 +2354,6 @@ int psim_system_download(psim_system* s, double* pos, double* pos0, double* vel,
         PSIM_CUDA(cudaMemcpyAsync(vel, s->vel.p, b, cudaMemcpyDeviceToHost, st));
         PSIM_CUDA(cudaStreamSynchronize(st));
     }
-    stage.release();
     return s->latched ? code_from_bits(s->latched) : PSIM_OK;
 }
 
@@ -2333,27 +2367,27 @@ int psim_system_download_cells(psim_system* s, int32_t* hash_index, uint32_t* cs
     const Phase ph = phase_of(s->total);
     const int n = s->n;
     cudaStream_t st = s->st;
-    ScopedBuf hb, cb, sb, pd;
-    PSIM_CUDA(hb.ensure(8 * (size_t)n));
-    PSIM_CUDA(cb.ensure(8 * (size_t)s->ncell));
-    PSIM_CUDA(sb.ensure(32 * (size_t)n));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({8 * (size_t)n, 8 * (size_t)s->ncell, 32 * (size_t)n, 32 * (size_t)n}));
+    int32_t* hb = mem.at<int32_t>(0);
+    uint32_t* cb = mem.at<uint32_t>(1);
+    double* sb = mem.at<double>(2);
     CellRefs c;
     if ((rc = cell_refs(s, c))) return rc;
     const double4_32a* posd = s->posd.as<double4_32a>();
     if (s->cfg.precision != PSIM_PRECISION_FP64) {
         // the mixed form keeps no FP64 sorted copy: gather one from the storage order
-        PSIM_CUDA(pd.ensure(32 * (size_t)n));
+        posd = mem.at<double4_32a>(3);
         PSIM_CUDA(launch_gather_posd(n, c.perm, d3(s->pos[ph.sb], n, 0), d3(s->pos[ph.sb], n, 1),
-                                     d3(s->pos[ph.sb], n, 2), c.radius, pd.as<double4_32a>(), st));
-        posd = pd.as<double4_32a>();
+                                     d3(s->pos[ph.sb], n, 2), c.radius, mem.at<double4_32a>(3), st));
     }
     PSIM_CUDA(launch_export_cells(n, s->ncell, s->cellid.as<int>(), c.tag, posd,
                                   s->start.as<int>(), c.count,
-                                  hb.as<int32_t>(), cb.as<uint32_t>(), sb.as<double>(), st));
+                                  hb, cb, sb, st));
     if (hash_index)
-        PSIM_CUDA(cudaMemcpyAsync(hash_index, hb.p, 8 * (size_t)n, cudaMemcpyDeviceToHost, st));
-    if (cse) PSIM_CUDA(cudaMemcpyAsync(cse, cb.p, 8 * (size_t)s->ncell, cudaMemcpyDeviceToHost, st));
-    if (sorted) PSIM_CUDA(cudaMemcpyAsync(sorted, sb.p, 32 * (size_t)n, cudaMemcpyDeviceToHost, st));
+        PSIM_CUDA(cudaMemcpyAsync(hash_index, hb, 8 * (size_t)n, cudaMemcpyDeviceToHost, st));
+    if (cse) PSIM_CUDA(cudaMemcpyAsync(cse, cb, 8 * (size_t)s->ncell, cudaMemcpyDeviceToHost, st));
+    if (sorted) PSIM_CUDA(cudaMemcpyAsync(sorted, sb, 32 * (size_t)n, cudaMemcpyDeviceToHost, st));
     PSIM_CUDA(cudaStreamSynchronize(st));
     return PSIM_OK;
 }
@@ -2406,18 +2440,16 @@ int psim_system_forces(psim_system* s, double* force) {
     if (rc) return rc;
     const Phase ph = phase_of(s->total);
     const int n = s->n;
-    ScopedBuf f3, out;
-    PSIM_CUDA(f3.ensure(24 * (size_t)n));
-    PSIM_CUDA(out.ensure(24 * (size_t)n));
-    ForceOut fo{f3.as<double>(), f3.as<double>() + n, f3.as<double>() + 2 * (size_t)n,
-                s->err.as<uint32_t>(), nullptr};
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({24 * (size_t)n, 24 * (size_t)n}));
+    double *f3 = mem.at<double>(0), *out = mem.at<double>(1);
+    ForceOut fo{f3, f3 + n, f3 + 2 * (size_t)n, s->err.as<uint32_t>(), nullptr};
     PSIM_CUDA(enqueue_force(s, ph, fo));
     // the pass writes in its order: the next cell order, or with a pair list
     // the storage order
     PSIM_CUDA(launch_unsort_force(n, s->list_on ? store_tags(s) : s->tag[ph.ob].as<int>(),
-                                  fo.fx, fo.fy, fo.fz,
-                                  out.as<double>(), s->st));
-    PSIM_CUDA(cudaMemcpyAsync(force, out.p, 24 * (size_t)n, cudaMemcpyDeviceToHost, s->st));
+                                  fo.fx, fo.fy, fo.fz, out, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(force, out, 24 * (size_t)n, cudaMemcpyDeviceToHost, s->st));
     return settle(s);
 }
 
@@ -2446,28 +2478,28 @@ int reduce(psim_system* s, ObserveArgs& a, double* out) {
     a.perm_prev = prev_perm(s);
     a.tag = store_tags(s);   // the storage order's tags (as download)
     a.L = s->g.L;
-    ScopedBuf scratch, res;
-    PSIM_CUDA(scratch.ensure(8 * (size_t)observe_scratch_doubles()));
-    PSIM_CUDA(res.ensure(8));
-    PSIM_CUDA(launch_observe(a, scratch.as<double>(), res.as<double>(), s->st));
-    PSIM_CUDA(cudaMemcpyAsync(out, res.p, 8, cudaMemcpyDeviceToHost, s->st));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({8 * (size_t)observe_scratch_doubles(), 8}));
+    PSIM_CUDA(launch_observe(a, mem.at<double>(0), mem.at<double>(1), s->st));
+    PSIM_CUDA(cudaMemcpyAsync(out, mem.at<double>(1), 8, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     return PSIM_OK;
 }
 
-// The sorted FP64 positions of the current cell list (into pd) and the cell
-// ranges, for a 27-cell walk.
-int sorted_view(psim_system* s, ScopedBuf& pd, PairScanArgs& a) {
+// The sorted FP64 positions of the current cell list (into pd, n of them) and the
+// cell ranges, for a walk of the pairs within r.
+int sorted_view(psim_system* s, double4_32a* pd, double r, PairScanArgs& a) {
     if (s->n_reps) return fail(PSIM_ERR_INPUT, "pair observables are per system, not per batch");
     const Phase ph = phase_of(s->total);
-    PSIM_CUDA(pd.ensure(32 * (size_t)s->n));
     CellRefs c;
     if (int rc = cell_refs(s, c)) return rc;
     PSIM_CUDA(launch_gather_posd(s->n, c.perm, d3(s->pos[ph.sb], s->n, 0),
                                  d3(s->pos[ph.sb], s->n, 1), d3(s->pos[ph.sb], s->n, 2),
-                                 c.radius, pd.as<double4_32a>(), s->st));
+                                 c.radius, pd, s->st));
     a.g = s->g;
-    a.posd = pd.as<double4_32a>();
+    a.posd = pd;
+    a.posh = s->posh.as<float4>();
+    a.pre_r2 = prefilter_r2(r, s->g.L);
     a.cellid = s->cellid.as<int>();
     a.cstart = s->start.as<int>();
     a.ccount = c.count;
@@ -2475,12 +2507,10 @@ int sorted_view(psim_system* s, ScopedBuf& pd, PairScanArgs& a) {
     return PSIM_OK;
 }
 
-int pair_scan(psim_system* s, PairScanArgs& a) {
-    ScopedBuf pd;
-    int rc = sorted_view(s, pd, a);
+int pair_scan(psim_system* s, double4_32a* pd, double r, PairScanArgs& a) {
+    int rc = sorted_view(s, pd, r, a);
     if (rc) return rc;
     PSIM_CUDA(launch_pair_scan(a, s->st));
-    PSIM_CUDA(cudaStreamSynchronize(s->st));
     return PSIM_OK;
 }
 
@@ -2491,13 +2521,12 @@ int psim_system_temperature(psim_system* s, double* kT) {
     if (rc) return rc;
     DeviceGuard dg(s->device);
     if ((rc = settle(s))) return rc;
-    ScopedBuf scratch, res;
-    PSIM_CUDA(scratch.ensure(8 * (size_t)observe_scratch_doubles()));
-    PSIM_CUDA(res.ensure(8));
-    PSIM_CUDA(launch_sum_squares(3LL * s->n, s->vel.as<double>(), scratch.as<double>(),
-                                 res.as<double>(), s->st));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({8 * (size_t)observe_scratch_doubles(), 8}));
+    PSIM_CUDA(launch_sum_squares(3LL * s->n, s->vel.as<double>(), mem.at<double>(0),
+                                 mem.at<double>(1), s->st));
     double v2 = 0.0;
-    PSIM_CUDA(cudaMemcpyAsync(&v2, res.p, 8, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(&v2, mem.at<double>(1), 8, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     *kT = s->n ? v2 / 3.0 / s->n : 0.0;
     return PSIM_OK;
@@ -2573,8 +2602,9 @@ int psim_system_interactions(psim_system* s, double r_contact, int32_t* coor, in
     DeviceGuard dg(s->device);
     int rc = settle(s);
     if (rc) return rc;
-    ScopedBuf cb, tot;
-    PSIM_CUDA(cb.ensure(4 * (size_t)s->n));
+    Scratch mem(s->obs);   // counts, total, and forces or sorted positions
+    PSIM_CUDA(mem.ensure({4 * (size_t)s->n, 8, 32 * (size_t)s->n}));
+    int* cb = mem.at<int>(0);
     // updateInteractions fused into one force pass on the current state: the
     // FP64 walk (the reference's own test, sqrt(r^2) < r_contact), the mixed
     // walk, or the mixed pair list when every pair closer than r_contact is
@@ -2585,11 +2615,9 @@ int psim_system_interactions(psim_system* s, double r_contact, int32_t* coor, in
         (!s->list_on || r_contact <= max_cutoff(&s->cfg.force))) {
         const Phase ph = phase_of(s->total);
         const int n = s->n;
-        ScopedBuf f3;
-        PSIM_CUDA(f3.ensure(24 * (size_t)n));
-        ForceOut fo{f3.as<double>(), f3.as<double>() + n, f3.as<double>() + 2 * (size_t)n,
-                    s->err.as<uint32_t>(), nullptr};
-        fo.coor = cb.as<int>();
+        double* f3 = mem.at<double>(2);
+        ForceOut fo{f3, f3 + n, f3 + 2 * (size_t)n, s->err.as<uint32_t>(), nullptr};
+        fo.coor = cb;
         fo.cont = r_contact;
         fo.cont2f = (float)(r_contact * r_contact);
         const float keep = s->fs.pre_rc2f;   // the candidate bound must cover r_contact
@@ -2599,7 +2627,7 @@ int psim_system_interactions(psim_system* s, double r_contact, int32_t* coor, in
         PSIM_CUDA(e);
         if ((rc = settle(s))) return rc;
         std::vector<int> c((size_t)n), tg((size_t)n);
-        PSIM_CUDA(cudaMemcpy(c.data(), cb.p, 4 * (size_t)n, cudaMemcpyDeviceToHost));
+        PSIM_CUDA(cudaMemcpy(c.data(), cb, 4 * (size_t)n, cudaMemcpyDeviceToHost));
         PSIM_CUDA(cudaMemcpy(tg.data(), s->list_on ? store_tags(s) : s->tag[ph.ob].as<int>(),
                              4 * (size_t)n, cudaMemcpyDeviceToHost));
         int64_t t = 0;
@@ -2610,16 +2638,18 @@ int psim_system_interactions(psim_system* s, double r_contact, int32_t* coor, in
         if (total) *total = t;
         return PSIM_OK;
     }
-    PSIM_CUDA(tot.ensure(8));
-    PSIM_CUDA(cudaMemsetAsync(tot.p, 0, 8, s->st));
+    unsigned long long* tot = mem.at<unsigned long long>(1);
+    PSIM_CUDA(cudaMemsetAsync(tot, 0, 8, s->st));
     PairScanArgs a{};
     a.r_contact = r_contact;
-    a.coor = cb.as<int>();
-    a.n_pairs = tot.as<unsigned long long>();
-    if ((rc = pair_scan(s, a))) return rc;
-    if (coor) PSIM_CUDA(cudaMemcpy(coor, cb.p, 4 * (size_t)s->n, cudaMemcpyDeviceToHost));
+    a.coor = cb;
+    a.n_pairs = tot;
+    if ((rc = pair_scan(s, mem.at<double4_32a>(2), r_contact, a))) return rc;
+    if (coor)
+        PSIM_CUDA(cudaMemcpyAsync(coor, cb, 4 * (size_t)s->n, cudaMemcpyDeviceToHost, s->st));
     unsigned long long t = 0;
-    PSIM_CUDA(cudaMemcpy(&t, tot.p, 8, cudaMemcpyDeviceToHost));
+    PSIM_CUDA(cudaMemcpyAsync(&t, tot, 8, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaStreamSynchronize(s->st));
     if (total) *total = (int64_t)t;
     return PSIM_OK;
 }
@@ -2633,23 +2663,21 @@ int psim_system_clusters(psim_system* s, double r_contact, int32_t min_size, int
     int rc = settle(s);
     if (rc) return rc;
     const size_t n = (size_t)s->n;
-    ScopedBuf pd, lab, rt, sz, eb;
-    PSIM_CUDA(lab.ensure(4 * n));
-    PSIM_CUDA(rt.ensure(4 * n));
-    PSIM_CUDA(sz.ensure(4 * n));
-    PSIM_CUDA(eb.ensure(4));
-    PSIM_CUDA(cudaMemsetAsync(sz.p, 0, 4 * n, s->st));
-    PSIM_CUDA(cudaMemsetAsync(eb.p, 0, 4, s->st));
+    Scratch mem(s->obs);   // positions, labels, roots, sizes and the error word
+    PSIM_CUDA(mem.ensure({32 * n, 4 * n, 4 * n, 4 * n, 4}));
+    int *lab = mem.at<int>(1), *rt = mem.at<int>(2), *sz = mem.at<int>(3);
+    uint32_t* eb = mem.at<uint32_t>(4);
+    PSIM_CUDA(cudaMemsetAsync(sz, 0, 4 * n, s->st));
+    PSIM_CUDA(cudaMemsetAsync(eb, 0, 4, s->st));
     PairScanArgs a{};
     a.r_contact = r_contact;
-    if ((rc = sorted_view(s, pd, a))) return rc;
-    PSIM_CUDA(launch_clusters(a, lab.as<int>(), rt.as<int>(), sz.as<int>(), eb.as<uint32_t>(),
-                              s->st));
+    if ((rc = sorted_view(s, mem.at<double4_32a>(0), r_contact, a))) return rc;
+    PSIM_CUDA(launch_clusters(a, lab, rt, sz, eb, s->st));
     std::vector<int> hroot(n), hsize(n);
     uint32_t bits = 0;
-    PSIM_CUDA(cudaMemcpyAsync(hroot.data(), rt.p, 4 * n, cudaMemcpyDeviceToHost, s->st));
-    PSIM_CUDA(cudaMemcpyAsync(hsize.data(), sz.p, 4 * n, cudaMemcpyDeviceToHost, s->st));
-    PSIM_CUDA(cudaMemcpyAsync(&bits, eb.p, 4, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(hroot.data(), rt, 4 * n, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(hsize.data(), sz, 4 * n, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(&bits, eb, 4, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     if (bits) return fail(PSIM_ERR_INPUT, "cluster search did not converge");
     if (root) std::copy(hroot.begin(), hroot.end(), root);
@@ -2674,19 +2702,21 @@ int psim_system_rdf(psim_system* s, double r_min, double r_max, int32_t n_bins, 
     DeviceGuard dg(s->device);
     int rc = settle(s);
     if (rc) return rc;
-    ScopedBuf hb;
-    PSIM_CUDA(hb.ensure(8 * (size_t)n_bins));
-    PSIM_CUDA(cudaMemsetAsync(hb.p, 0, 8 * (size_t)n_bins, s->st));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({8 * (size_t)n_bins, 32 * (size_t)s->n}));
+    unsigned long long* hb = mem.at<unsigned long long>(0);
+    PSIM_CUDA(cudaMemsetAsync(hb, 0, 8 * (size_t)n_bins, s->st));
     PairScanArgs a{};
     a.r_contact = 0.0;
     a.r_min = r_min;
     a.r_max = r_max;
     a.inv_dr = n_bins / (r_max - r_min);
     a.n_bins = n_bins;
-    a.hist = hb.as<unsigned long long>();
-    if ((rc = pair_scan(s, a))) return rc;
+    a.hist = hb;
+    if ((rc = pair_scan(s, mem.at<double4_32a>(1), r_max, a))) return rc;
     std::vector<unsigned long long> h((size_t)n_bins);
-    PSIM_CUDA(cudaMemcpy(h.data(), hb.p, 8 * (size_t)n_bins, cudaMemcpyDeviceToHost));
+    PSIM_CUDA(cudaMemcpyAsync(h.data(), hb, 8 * (size_t)n_bins, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaStreamSynchronize(s->st));
     // ordered pairs per particle in each shell over the ideal-gas count
     const double rho = s->n / (s->g.L * s->g.L * s->g.L);
     const double dr = (r_max - r_min) / n_bins;
@@ -2721,13 +2751,13 @@ int psim_system_energy(psim_system* s, double* potential, double* virial) {
     int rc = settle(s);
     if (rc) return rc;
     PairScanArgs a{};
-    ScopedBuf pd, scratch, res;
-    if ((rc = sorted_view(s, pd, a))) return rc;
-    PSIM_CUDA(scratch.ensure(16 * (size_t)((s->n + 127) / 128 + 1)));
-    PSIM_CUDA(res.ensure(16));
-    PSIM_CUDA(launch_energy(s->fs, a, scratch.as<double>(), res.as<double>(), s->st));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({32 * (size_t)s->n, 8 * energy_scratch_doubles(s->n), 16}));
+    if ((rc = sorted_view(s, mem.at<double4_32a>(0), max_cutoff(&s->cfg.force), a))) return rc;
+    double* res = mem.at<double>(2);
+    PSIM_CUDA(launch_energy(s->fs, a, mem.at<double>(1), res, s->st));
     double out[2] = {0.0, 0.0};
-    PSIM_CUDA(cudaMemcpyAsync(out, res.p, 16, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(out, res, 16, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     if (potential) *potential = s->n ? out[0] / s->n : 0.0;
     if (virial) *virial = s->n ? out[1] / s->n : 0.0;
@@ -2824,23 +2854,24 @@ int psim_system_pair_count(psim_system* s, double cutoff, double* mean_pairs) {
     int rc = settle(s);
     if (rc) return rc;
     const Phase ph = phase_of(s->total);
-    ScopedBuf tot, ph4;
-    PSIM_CUDA(tot.ensure(8));
-    PSIM_CUDA(ph4.ensure(16 * (size_t)s->n));
-    PSIM_CUDA(cudaMemsetAsync(tot.p, 0, 8, s->st));
+    Scratch mem(s->obs);
+    PSIM_CUDA(mem.ensure({8, 16 * (size_t)s->n}));
+    unsigned long long* tot = mem.at<unsigned long long>(0);
+    float4* ph4 = mem.at<float4>(1);
+    PSIM_CUDA(cudaMemsetAsync(tot, 0, 8, s->st));
     // sorted positions gathered from the FP64 state (with a pair list the
     // float copies are in list order)
     CellRefs c;
     if ((rc = cell_refs(s, c))) return rc;
     PSIM_CUDA(launch_gather_posh(s->n, c.perm, d3(s->pos[ph.sb], s->n, 0),
                                  d3(s->pos[ph.sb], s->n, 1), d3(s->pos[ph.sb], s->n, 2),
-                                 c.radius, ph4.as<float4>(), s->st));
-    CellView cv{nullptr, ph4.as<float4>(), nullptr, s->cellid.as<int>(), s->start.as<int>(),
+                                 c.radius, ph4, s->st));
+    CellView cv{nullptr, ph4, nullptr, s->cellid.as<int>(), s->start.as<int>(),
                 c.count};
-    PSIM_CUDA(launch_pair_count(s->g, cv, (float)(cutoff * cutoff), tot.as<unsigned long long>(),
+    PSIM_CUDA(launch_pair_count(s->g, cv, (float)(cutoff * cutoff), tot,
                                 s->st));
     unsigned long long h = 0;
-    PSIM_CUDA(cudaMemcpyAsync(&h, tot.p, 8, cudaMemcpyDeviceToHost, s->st));
+    PSIM_CUDA(cudaMemcpyAsync(&h, tot, 8, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
     *mean_pairs = s->n ? (double)h / s->n : 0.0;
     return PSIM_OK;

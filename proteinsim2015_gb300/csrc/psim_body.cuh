@@ -148,6 +148,10 @@ struct F64Body {
             a.n2 = __fma_rn(f, d2, a.n2);
         }
     }
+    __device__ __forceinline__ void eval_quad(int, const double4_32a& pj, const Home& h, Acc& a,
+                                              uint32_t& err) const {
+        eval(make_float4(0.f, 0.f, 0.f, 0.f), pj, h, a, err);
+    }
     // L for d < 0, else -L
     static __device__ __forceinline__ double toward(double L, double d) {
         return __hiloint2double(__double2hiint(L) | (~__double2hiint(d) & 0x80000000),

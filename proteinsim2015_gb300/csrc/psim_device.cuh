@@ -366,6 +366,7 @@ __host__ __device__ __forceinline__ T pow36(T rinv) {
 struct AOPair {
     double rc2, c1, c2;
     float rc2f, c1f, c2f;
+    double rc, e37;   // the cutoff and rc^-37 (u64)
     static constexpr bool kCheckNan = true;
     __host__ __device__ __forceinline__ double fnet64(double r2, double r, double rinv, double) const {
         double r36 = pow36(rinv);
@@ -390,8 +391,7 @@ struct AOPair {
     // the pair energy whose derivative is fnet64 (u' = fNet), zero at the
     // cutoff: 36/37 (r^-37 - rc^-37) + coEff1 ln(rc/r) + coEff2 (rc^2 - r^2)/2
     __host__ __device__ __forceinline__ double u64(double r2, double, double rinv, double) const {
-        const double rc = sqrt(rc2), rcinv = 1.0 / rc;
-        return (36.0 / 37.0) * (pow36(rinv) * rinv - pow36(rcinv) * rcinv) + c1 * log(rc * rinv) +
+        return (36.0 / 37.0) * (pow36(rinv) * rinv - e37) + c1 * log(rc * rinv) +
                0.5 * c2 * (rc2 - r2);
     }
 };
@@ -491,6 +491,8 @@ inline AOPair make_ao_pair(double kT, double wd, double rc) {
     AOPair p{};
     ao_coeffs(kT, wd, rc, &p.c1, &p.c2);
     p.rc2 = rc * rc;
+    p.rc = rc;
+    p.e37 = pow36(1.0 / rc) * (1.0 / rc);
     p.rc2f = (float)p.rc2;
     p.c1f = (float)p.c1;
     p.c2f = (float)p.c2;

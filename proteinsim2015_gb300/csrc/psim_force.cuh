@@ -364,11 +364,14 @@ __device__ __forceinline__ bool quad_rows(const DevGeom& g) {
     return g.n < 8ll * g.ncell;
 }
 
+// The walk of the warp's eight particles (i: the lane's): body.eval_quad(j, aux of j,
+// home, acc, err) for every neighbour j within sqrt(pre_rc2), FP32 positions
+// deciding.  acc gets this lane's sums.
 template <class Body>
-__device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom& g,
-                                                const CellView& cv, const ForceOut& out,
-                                                float pre_rc2, int i, int lane,
-                                                uint32_t (*qs)[kQuadStride]) {
+__device__ __forceinline__ void quad_walk(const Body& body, const DevGeom& g, const CellView& cv,
+                                          float pre_rc2, int i, int lane,
+                                          uint32_t (*qs)[kQuadStride], typename Body::Acc& acc,
+                                          uint32_t& err) {
     using Aux = typename Body::Aux;
     const Aux* g_aux = body.aux(cv);
     const int m = lane & 3;
@@ -377,14 +380,12 @@ __device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom&
     float4 hi = make_float4(0.f, 0.f, 0.f, 0.f);
     int cx = 0, cy = 0, cz = 0;
     typename Body::Home home;
-    typename Body::Acc acc;
     body.init(acc);
     if (active) {
         hi = cv.posh[i];
         cell_xyz(cv.cellid[i] - g.c0, g, cx, cy, cz);
         body.load_home(cv, i, home);
     }
-    uint32_t err = 0;
     int cnt = 0;    // entries in the particle's queue
     int done = 0;   // entries evaluated before them
     auto drain = [&]() {
@@ -393,12 +394,21 @@ __device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom&
         const int last = __reduce_max_sync(0xffffffffu, cnt);
         // the next neighbour is loaded while this one's terms are formed
         Aux aj{};
-        if (k < cnt) aj = g_aux[q[k]];
+        uint32_t j = 0u;
+        if (k < cnt) {
+            j = q[k];
+            aj = g_aux[j];
+        }
         for (int it = 0; it < last; it += 4, k += 4) {
             Aux an{};
-            if (k + 4 < cnt) an = g_aux[q[k + 4]];
-            if (k < cnt) body.eval(hi, aj, home, acc, err);
+            uint32_t jn = 0u;
+            if (k + 4 < cnt) {
+                jn = q[k + 4];
+                an = g_aux[jn];
+            }
+            if (k < cnt) body.eval_quad((int)j, aj, home, acc, err);
             aj = an;
+            j = jn;
         }
         done += cnt;
         cnt = 0;
@@ -459,8 +469,18 @@ __device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom&
         }
     }
     drain();
+}
+
+template <class Body>
+__device__ __forceinline__ void force_quad_warp(const Body& body, const DevGeom& g,
+                                                const CellView& cv, const ForceOut& out,
+                                                float pre_rc2, int i, int lane,
+                                                uint32_t (*qs)[kQuadStride]) {
+    typename Body::Acc acc;
+    uint32_t err = 0;
+    quad_walk(body, g, cv, pre_rc2, i, lane, qs, acc, err);
     body.add_quad(acc);
-    if (active && m == 0) body.store(out, i, acc);
+    if (i < g.p1 && (lane & 3) == 0) body.store(out, i, acc);
     if (err) atomicOr(out.err, err);
 }
 

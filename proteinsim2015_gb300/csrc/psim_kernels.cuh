@@ -449,6 +449,8 @@ int observe_scratch_doubles();
 struct PairScanArgs {
     DevGeom g;
     const double4_32a* posd;
+    const float4* posh;             // the same positions in FP32
+    float pre_r2;                   // FP32 bound on r^2 for every pair wanted
     const int* cellid;
     const int* cstart;
     const int* ccount;
@@ -463,8 +465,9 @@ struct PairScanArgs {
 cudaError_t launch_pair_scan(const PairScanArgs& a, cudaStream_t st);
 // FP64 potential energy and virial of the plugin's pair force over the 27-cell
 // walk of a: out[0] = sum over pairs of u(r), out[1] = sum over pairs of
-// r_ij . f_ij (f_ij the force on i from j).  scratch: 2 * ceil(n / 128) doubles.
+// r_ij . f_ij (f_ij the force on i from j).  scratch: energy_scratch_doubles(n).
 // cudaErrorInvalidValue for a force kind without an energy.
+size_t energy_scratch_doubles(int n);
 cudaError_t launch_energy(const ForceSetup& fs, const PairScanArgs& a, double* scratch,
                           double* out, cudaStream_t st);
 // Clusters of the contact graph (r < a.r_contact): root[original index] = the

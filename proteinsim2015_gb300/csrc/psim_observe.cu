@@ -11,7 +11,9 @@
 //
 // Sums are deterministic: each block writes its partial, one block adds the
 // partials in block order.
-#include "psim_kernels.cuh"
+#include <algorithm>
+
+#include "psim_force.cuh"
 
 namespace psim {
 
@@ -33,13 +35,14 @@ __device__ double block_sum(double v, double* sh) {
     return t;  // valid in thread 0
 }
 
+// out[b] = the sum of partials b n .. b n + n - 1 (block b)
 __global__ void __launch_bounds__(kRedThreads) finish_kernel(const double* part, int n, double* out) {
     __shared__ double sh[kRedThreads / 32];
     // each thread adds a fixed stride of partials, then the block in lane order
     double v = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) v += part[k];
+    for (int k = threadIdx.x; k < n; k += blockDim.x) v += part[(size_t)blockIdx.x * n + k];
     const double t = block_sum(v, sh);
-    if (threadIdx.x == 0) *out = t;
+    if (threadIdx.x == 0) out[blockIdx.x] = t;
 }
 
 // sum of |v|^2 over count values
@@ -88,48 +91,83 @@ __global__ void __launch_bounds__(kRedThreads) observe_kernel(ObserveArgs a, dou
     if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
-// The 27-cell walk of updateInteractions (systemHandling.cpp:126-161) on
-// the sorted FP64 positions: neighbours closer than r_contact are counted
-// (pbcDist's minimum image, utilities.cpp:79-104), and distances in
-// [r_min, r_max) are binned for g(r).
-__global__ void __launch_bounds__(128) pairs_kernel(PairScanArgs a) {
+// ------------------------------------------------------------ pair walks
+//
+// The pairs of the current cell list through the four-lane walk of the FP64 force
+// pass (force_quad_kernel): FP32 positions with a margin reject the candidates out of
+// range, so that the FP64 distance, pbcDist's minimum image (utilities.cpp:79-104), is
+// formed for the others only, with full warps.  At 131072 particles, a thread per
+// particle with FP64 distances to all 27 cells before, and now (whole calls): energy
+// 1050 -> 175 us, coordination 1251 -> 141, g(r) 1314 -> 166.
+
+__device__ __forceinline__ CellView scan_cells(const PairScanArgs& a) {
+    return CellView{a.posd, a.posh, nullptr, a.cellid, a.cstart, a.ccount};
+}
+__device__ __forceinline__ double scan_r2(const DevGeom& g, const double4_32a& pi,
+                                          const double4_32a& pj) {
+    double d0 = fabs(pj.x - pi.x), d1 = fabs(pj.y - pi.y), d2 = fabs(pj.z - pi.z);
+    if (d0 > g.half) d0 -= g.L;
+    if (d1 > g.half) d1 -= g.L;
+    if (d2 > g.half) d2 -= g.L;
+    return d0 * d0 + d1 * d1 + d2 * d2;
+}
+
+constexpr int kScanBlocks = 152 * 12;   // at most; each block takes every gridDim-th group
+
+// updateInteractions' count (systemHandling.cpp:94-161): neighbours closer than
+// r_contact; distances in [r_min, r_max) are binned for g(r).
+struct ScanBody {
+    PairScanArgs a;
+    unsigned int* hist;
+    using Aux = double4_32a;
+    struct Home {
+        double4_32a p;
+    };
+    struct Acc {
+        int coor;
+    };
+    __device__ __forceinline__ const Aux* aux(const CellView& cv) const { return cv.posd; }
+    __device__ __forceinline__ void init(Acc& c) const { c.coor = 0; }
+    __device__ __forceinline__ void load_home(const CellView& cv, int i, Home& h) const {
+        h.p = cv.posd[i];
+    }
+    __device__ __forceinline__ void eval_quad(int, const double4_32a& pj, const Home& h, Acc& c,
+                                              uint32_t&) const {
+        const double r = sqrt(scan_r2(a.g, h.p, pj));
+        if (r < a.r_contact) ++c.coor;
+        if (a.n_bins > 0 && r >= a.r_min && r < a.r_max) {
+            const int b = (int)((r - a.r_min) * a.inv_dr);
+            atomicAdd(&hist[b < a.n_bins ? b : a.n_bins - 1], 1u);
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kQuadWarps * 32) pairs_kernel(PairScanArgs a) {
     extern __shared__ unsigned int hist[];
+    __shared__ uint32_t s_q[kQuadWarps][8][kQuadStride];
     for (int b = threadIdx.x; b < a.n_bins; b += blockDim.x) hist[b] = 0u;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.g.n) {
-        const double4_32a pi = a.posd[i];
-        const int c = a.cellid[i];
-        const int cx = c % a.g.s, cy = (c / a.g.s) % a.g.s, cz = c / a.g.s2;
-        int coor = 0;
-        for (int dx = -1; dx <= 1; ++dx)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dz = -1; dz <= 1; ++dz) {
-                    int sh;
-                    const int x = wrap_cell(cx + dx, a.g.s, sh);
-                    const int y = wrap_cell(cy + dy, a.g.s, sh);
-                    const int z = wrap_cell(cz + dz, a.g.s, sh);
-                    const int cell = x + a.g.s * y + a.g.s2 * z;
-                    const int st = a.cstart[cell], en = st + a.ccount[cell];
-                    for (int j = st; j < en; ++j) {
-                        if (j == i) continue;
-                        const double4_32a pj = a.posd[j];
-                        double d0 = fabs(pj.x - pi.x), d1 = fabs(pj.y - pi.y),
-                               d2 = fabs(pj.z - pi.z);
-                        if (d0 > a.g.half) d0 -= a.g.L;
-                        if (d1 > a.g.half) d1 -= a.g.L;
-                        if (d2 > a.g.half) d2 -= a.g.L;
-                        const double r = sqrt(d0 * d0 + d1 * d1 + d2 * d2);
-                        if (r < a.r_contact) ++coor;
-                        if (a.n_bins > 0 && r >= a.r_min && r < a.r_max) {
-                            int b = (int)((r - a.r_min) * a.inv_dr);
-                            b = b < a.n_bins ? b : a.n_bins - 1;
-                            atomicAdd(&hist[b], 1u);
-                        }
-                    }
-                }
-        if (a.coor) a.coor[a.tag[i]] = coor;
-        if (a.n_pairs) atomicAdd(a.n_pairs, (unsigned long long)coor);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const ScanBody body{a, hist};
+    const CellView cv = scan_cells(a);
+    const int per = 8 * kQuadWarps, groups = (a.g.n + per - 1) / per;
+    long long total = 0;
+    for (int k = blockIdx.x; k < groups; k += gridDim.x) {
+        const int i = k * per + 8 * w + (lane >> 2);
+        ScanBody::Acc c;
+        uint32_t err = 0;
+        quad_walk(body, a.g, cv, a.pre_r2, i, lane, s_q[w], c, err);
+        int coor = c.coor + __shfl_xor_sync(0xffffffffu, c.coor, 1);
+        coor += __shfl_xor_sync(0xffffffffu, coor, 2);
+        if (i < a.g.n && (lane & 3) == 0) {
+            if (a.coor) a.coor[a.tag[i]] = coor;
+            total += coor;
+        }
+    }
+    if (a.n_pairs) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        if (lane == 0 && total) atomicAdd(a.n_pairs, (unsigned long long)total);
     }
     __syncthreads();
     for (int b = threadIdx.x; b < a.n_bins; b += blockDim.x)
@@ -180,36 +218,37 @@ __global__ void __launch_bounds__(256) uf_init_kernel(int n, int* label) {
     if (i < n) label[i] = i;
 }
 
-__global__ void __launch_bounds__(128) uf_edges_kernel(PairScanArgs a, int* label,
-                                                        uint32_t* err_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.g.n) return;
+struct EdgeBody {
+    PairScanArgs a;
+    int* label;
+    using Aux = double4_32a;
+    struct Home {
+        double4_32a p;
+        int tag;
+    };
+    struct Acc {};
+    __device__ __forceinline__ const Aux* aux(const CellView& cv) const { return cv.posd; }
+    __device__ __forceinline__ void init(Acc&) const {}
+    __device__ __forceinline__ void load_home(const CellView& cv, int i, Home& h) const {
+        h.p = cv.posd[i];
+        h.tag = a.tag[i];
+    }
+    __device__ __forceinline__ void eval_quad(int j, const double4_32a& pj, const Home& h, Acc&,
+                                              uint32_t& err) const {
+        const int tj = a.tag[j];
+        if (tj <= h.tag) return;   // each undirected edge once
+        if (sqrt(scan_r2(a.g, h.p, pj)) < a.r_contact) uf_union(label, h.tag, tj, a.g.n, err);
+    }
+};
+
+__global__ void __launch_bounds__(kQuadWarps * 32)
+uf_edges_kernel(PairScanArgs a, int* label, uint32_t* err_out) {
+    __shared__ uint32_t s_q[kQuadWarps][8][kQuadStride];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    EdgeBody::Acc c;
     uint32_t err = 0;
-    const double4_32a pi = a.posd[i];
-    const int ti = a.tag[i];
-    const int c = a.cellid[i];
-    const int cx = c % a.g.s, cy = (c / a.g.s) % a.g.s, cz = c / a.g.s2;
-    for (int dx = -1; dx <= 1; ++dx)
-        for (int dy = -1; dy <= 1; ++dy)
-            for (int dz = -1; dz <= 1; ++dz) {
-                int sh;
-                const int x = wrap_cell(cx + dx, a.g.s, sh);
-                const int y = wrap_cell(cy + dy, a.g.s, sh);
-                const int z = wrap_cell(cz + dz, a.g.s, sh);
-                const int cell = x + a.g.s * y + a.g.s2 * z;
-                const int st = a.cstart[cell], en = st + a.ccount[cell];
-                for (int j = st; j < en; ++j) {
-                    const int tj = a.tag[j];
-                    if (tj <= ti) continue;   // each undirected edge once
-                    const double4_32a pj = a.posd[j];
-                    double d0 = fabs(pj.x - pi.x), d1 = fabs(pj.y - pi.y), d2 = fabs(pj.z - pi.z);
-                    if (d0 > a.g.half) d0 -= a.g.L;
-                    if (d1 > a.g.half) d1 -= a.g.L;
-                    if (d2 > a.g.half) d2 -= a.g.L;
-                    if (sqrt(d0 * d0 + d1 * d1 + d2 * d2) < a.r_contact)
-                        uf_union(label, ti, tj, a.g.n, err);
-                }
-            }
+    quad_walk(EdgeBody{a, label}, a.g, scan_cells(a), a.pre_r2,
+              (blockIdx.x * kQuadWarps + w) * 8 + (lane >> 2), lane, s_q[w], c, err);
     if (err) atomicOr(err_out, err);
 }
 
@@ -256,61 +295,76 @@ struct ComboTerms {  // the AO + LJ(n) composite: each part inside its own cutof
 };
 
 // Per particle i: half the sum over its neighbours j of u(r_ij) and of
-// r_ij . f_ij = -fNet(r_ij) r_ij (pbcDist's minimum image), in FP64; block
-// partials of both, added in block order by finish_kernel.
+// r_ij . f_ij = -fNet(r_ij) r_ij, in FP64, then summed over the particles in a fixed
+// order.
 template <class Terms>
-__global__ void __launch_bounds__(128) energy_kernel(PairScanArgs a, Terms t, double* part,
-                                                     int stride) {
-    __shared__ double sh[4];
-    double eu = 0.0, ew = 0.0;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.g.n) {
-        const double4_32a pi = a.posd[i];
-        const int c = a.cellid[i];
-        const int cx = c % a.g.s, cy = (c / a.g.s) % a.g.s, cz = c / a.g.s2;
-        const double rc2 = t.rc2();
-        for (int dx = -1; dx <= 1; ++dx)
-            for (int dy = -1; dy <= 1; ++dy)
-                for (int dz = -1; dz <= 1; ++dz) {
-                    int sh_;
-                    const int x = wrap_cell(cx + dx, a.g.s, sh_);
-                    const int y = wrap_cell(cy + dy, a.g.s, sh_);
-                    const int z = wrap_cell(cz + dz, a.g.s, sh_);
-                    const int cell = x + a.g.s * y + a.g.s2 * z;
-                    const int st = a.cstart[cell], en = st + a.ccount[cell];
-                    for (int j = st; j < en; ++j) {
-                        if (j == i) continue;
-                        const double4_32a pj = a.posd[j];
-                        double d0 = fabs(pj.x - pi.x), d1 = fabs(pj.y - pi.y),
-                               d2 = fabs(pj.z - pi.z);
-                        if (d0 > a.g.half) d0 -= a.g.L;
-                        if (d1 > a.g.half) d1 -= a.g.L;
-                        if (d2 > a.g.half) d2 -= a.g.L;
-                        const double r2 = d0 * d0 + d1 * d1 + d2 * d2;
-                        if (!(r2 < rc2)) continue;
-                        const double r = sqrt(r2), rinv = 1.0 / r;
-                        double u = 0.0, f = 0.0;
-                        t.eval(r2, r, rinv, pi.w + pj.w, u, f);
-                        eu += u;
-                        ew -= f * r;
-                    }
-                }
+struct EnergyBody {
+    Terms t;
+    DevGeom g;
+    double rc2;
+    using Aux = double4_32a;
+    struct Home {
+        double4_32a p;
+    };
+    struct Acc {
+        double u, w;
+    };
+    __device__ __forceinline__ const Aux* aux(const CellView& cv) const { return cv.posd; }
+    __device__ __forceinline__ void init(Acc& c) const { c.u = c.w = 0.0; }
+    __device__ __forceinline__ void load_home(const CellView& cv, int i, Home& h) const {
+        h.p = cv.posd[i];
     }
-    const double su = block_sum(0.5 * eu, sh);
-    const double sw = block_sum(0.5 * ew, sh);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = su;
-        part[stride + blockIdx.x] = sw;
+    __device__ __forceinline__ void eval_quad(int, const double4_32a& pj, const Home& h, Acc& c,
+                                              uint32_t&) const {
+        const double r2 = scan_r2(g, h.p, pj);
+        if (!(r2 < rc2)) return;
+        const double r = sqrt(r2), rinv = 1.0 / r;
+        double u = 0.0, f = 0.0;
+        t.eval(r2, r, rinv, h.p.w + pj.w, u, f);
+        c.u += u;
+        c.w -= f * r;
     }
+};
+
+template <class Terms>
+__global__ void __launch_bounds__(kQuadWarps * 32)
+energy_kernel(PairScanArgs a, Terms t, double* part) {
+    __shared__ uint32_t s_q[kQuadWarps][8][kQuadStride];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = (blockIdx.x * kQuadWarps + w) * 8 + (lane >> 2);
+    const EnergyBody<Terms> body{t, a.g, t.rc2()};
+    typename EnergyBody<Terms>::Acc c;
+    uint32_t err = 0;
+    quad_walk(body, a.g, scan_cells(a), a.pre_r2, i, lane, s_q[w], c, err);
+#pragma unroll
+    for (int k = 1; k < 4; k <<= 1) {
+        c.u += __shfl_xor_sync(0xffffffffu, c.u, k);
+        c.w += __shfl_xor_sync(0xffffffffu, c.w, k);
+    }
+    if (i < a.g.n && (lane & 3) == 0) {
+        part[i] = 0.5 * c.u;
+        part[a.g.n + i] = 0.5 * c.w;
+    }
+}
+
+// block partials of the two rows of v[2][n]
+__global__ void __launch_bounds__(kRedThreads) rows_kernel(int n, const double* v, double* part) {
+    __shared__ double sh[kRedThreads / 32];
+    double t = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        t += v[(size_t)blockIdx.y * n + i];
+    t = block_sum(t, sh);
+    if (threadIdx.x == 0) part[blockIdx.y * gridDim.x + blockIdx.x] = t;
 }
 
 template <class Terms>
 cudaError_t run_energy(const Terms& t, const PairScanArgs& a, double* scratch, double* out,
                        cudaStream_t st) {
-    const int blocks = (a.g.n + 127) / 128;
-    energy_kernel<Terms><<<blocks, 128, 0, st>>>(a, t, scratch, blocks);
-    finish_kernel<<<1, kRedThreads, 0, st>>>(scratch, blocks, out);
-    finish_kernel<<<1, kRedThreads, 0, st>>>(scratch + blocks, blocks, out + 1);
+    const int per = 8 * kQuadWarps, n = a.g.n;
+    energy_kernel<Terms><<<(n + per - 1) / per, kQuadWarps * 32, 0, st>>>(a, t, scratch);
+    double* part = scratch + 2 * (size_t)n;
+    rows_kernel<<<dim3(kRedBlocks, 2), kRedThreads, 0, st>>>(n, scratch, part);
+    finish_kernel<<<2, kRedThreads, 0, st>>>(part, kRedBlocks, out);
     return cudaGetLastError();
 }
 
@@ -333,7 +387,8 @@ cudaError_t launch_clusters(const PairScanArgs& a, int* label, int* root, int* s
     const int n = a.g.n;
     if (n == 0) return cudaSuccess;
     uf_init_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, label);
-    uf_edges_kernel<<<(n + 127) / 128, 128, 0, st>>>(a, label, err);
+    const int per = 8 * kQuadWarps;
+    uf_edges_kernel<<<(n + per - 1) / per, kQuadWarps * 32, 0, st>>>(a, label, err);
     uf_final_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, label, root, size, err);
     return cudaGetLastError();
 }
@@ -352,11 +407,13 @@ cudaError_t launch_observe(const ObserveArgs& a, double* scratch, double* out, c
 }
 
 int observe_scratch_doubles() { return kRedBlocks; }
+size_t energy_scratch_doubles(int n) { return 2 * (size_t)n + 2 * kRedBlocks; }
 
 cudaError_t launch_pair_scan(const PairScanArgs& a, cudaStream_t st) {
     if (a.g.n == 0) return cudaSuccess;
     const size_t smem = sizeof(unsigned int) * (size_t)(a.n_bins > 0 ? a.n_bins : 1);
-    pairs_kernel<<<(a.g.n + 127) / 128, 128, smem, st>>>(a);
+    const int per = 8 * kQuadWarps, groups = (a.g.n + per - 1) / per;
+    pairs_kernel<<<std::min(groups, kScanBlocks), kQuadWarps * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
