@@ -567,7 +567,8 @@ int psim_system_profile(psim_system* sys, int32_t n_steps, double* out_ms);
 int psim_system_launches_per_step(psim_system* sys);
 /* Kernel launches of a step's pair-list rebuild (0 without a pair list): with
  * a pair list a step launches psim_system_launches_per_step kernels, and the
- * steps that rebuild the list this many more. */
+ * steps that rebuild the list this many more (0 where a small system's steps and
+ * rebuilds are one kernel). */
 int psim_system_launches_per_rebuild(psim_system* sys);
 
 /* Occupancy of the current cell list: max and mean particles per cell. */

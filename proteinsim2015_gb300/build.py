@@ -5,6 +5,7 @@ Translation units are compiled in parallel with one -gencode each:
                  reference's two-rounding a*b+c)
   psim_mixed.cu  FP32 pair math (contraction allowed)
   psim_step.cu   the mixed form's list step as one kernel (as psim_mixed.cu)
+  psim_run.cu    the mixed form's list steps of a small system in one kernel
   psim_list_build.cu  the pair list's build
   psim_cells.cu  integer counting sort and layout conversions
   psim_api.cu    host side of the C ABI
@@ -30,6 +31,7 @@ SOURCES = {
     "psim_mixed.cu": [],
     "psim_step.cu": [],
     "psim_list_build.cu": [],
+    "psim_run.cu": [],
     "psim_cells.cu": [],
     "psim_api.cu": [],
     "psim_noalloc.cu": [],

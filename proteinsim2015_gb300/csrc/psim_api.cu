@@ -1196,6 +1196,7 @@ struct psim_system {
     // (fused: normal steps in the one kernel of psim_step.cu)
     cudaGraphExec_t graph[6] = {}, fused[6] = {};
     cudaGraphExec_t graph_multi = nullptr;
+    int small = -1;           // whether stretches of normal steps run in one kernel (-1: not asked)
     uint32_t latched = 0;
     // Verlet pair list of the mixed form (list_on): list slot of each storage
     // slot (ping-pong with the order), positions at the build, entries,
@@ -1282,11 +1283,12 @@ void set_halo_args(psim_system* s, CanonArgs& ca, long long t) {
     }
 }
 
-// The pair-list build on the cell order just made (count buffer cb), run
-// only when *gate != 0.
-cudaError_t enqueue_list_build(psim_system* s, int cb, const int* gate) {
-    CellView cv{nullptr, s->posh.as<float4>(), s->posl.as<float4>(), s->cellid.as<int>(),
-                s->start.as<int>(), s->count[cb].as<int>()};
+// The cell order a pair list is built on (count buffer cb), and its build.
+CellView list_cells(psim_system* s, int cb) {
+    return CellView{nullptr, s->posh.as<float4>(), s->posl.as<float4>(), s->cellid.as<int>(),
+                    s->start.as<int>(), s->count[cb].as<int>()};
+}
+ListBuild list_build(psim_system* s, const int* gate) {
     ListBuild lb{s->list.as<uint32_t>(), s->lcount.as<int>(), s->n, s->lcap, s->lpre, gate,
                  s->lhalo.as<int>(), s->n};
     lb.xsorted = 1;   // the order set_halo_args asks the canonicalisation for
@@ -1295,7 +1297,14 @@ cudaError_t enqueue_list_build(psim_system* s, int cb, const int* gate) {
         lb.geoms = s->b_geoms.as<DevGeom>();
         lb.pre = s->b_lpre.as<float>();
     }
-    return launch_list_build(s->g, cv, lb, s->err.as<uint32_t>(), s->st);
+    return lb;
+}
+
+// The pair-list build on the cell order just made (count buffer cb), run
+// only when *gate != 0.
+cudaError_t enqueue_list_build(psim_system* s, int cb, const int* gate) {
+    return launch_list_build(s->g, list_cells(s, cb), list_build(s, gate), s->err.as<uint32_t>(),
+                             s->st);
 }
 
 // The pair list of the state at phase ph (the storage order is the list order: no
@@ -1349,6 +1358,32 @@ cudaError_t enqueue_force(psim_system* s, const Phase& ph, const ForceOut& fo) {
 // the trajectory are those of the cell list rebuilt every step: the same
 // pair terms in the same list order, the same per-particle arithmetic.
 
+// The canonicalisation of the rebuild before a step of parity q: list records, build
+// positions and halo images on the new order.
+CanonArgs canon_args(psim_system* s, int q) {
+    const int n = s->n;
+    CanonArgs ca{};
+    ca.n = n;
+    ca.tmp = s->tmp.as<int>();
+    ca.key = s->key.as<int>();
+    ca.start = s->start.as<int>();
+    ca.count = s->count[0].as<int>();
+    ca.tag_in = s->tag[0].as<int>();
+    ca.radius_in = s->radius[0].as<double>();
+    ca.inv_mass_in = s->inv_mass[0].as<double>();
+    ca.x = d3(s->pos[q], n, 0); ca.y = d3(s->pos[q], n, 1); ca.z = d3(s->pos[q], n, 2);
+    ca.perm = s->perm[0].as<int>();
+    ca.tag_out = s->tag[1].as<int>();
+    ca.radius_out = s->radius[1].as<double>();
+    ca.inv_mass_out = s->inv_mass[1].as<double>();
+    ca.cellid = s->cellid.as<int>();
+    ca.posh = s->posh.as<float4>();
+    ca.vel_freq = s->vp.vel_freq;
+    ca.err = s->err.as<uint32_t>();
+    set_halo_args(s, ca, q);
+    return ca;
+}
+
 // The rebuild after step t (phase of t): the state the integrator wrote (in
 // the storage order) sorted into the new cell order.
 int enqueue_rebuild_lazy(psim_system* s, long long t) {
@@ -1366,25 +1401,7 @@ int enqueue_rebuild_lazy(psim_system* s, long long t) {
                           s->scratch.as<int>(), st));
     PSIM_CUDA(launch_scatter(n, s->key.as<int>(), s->rank.as<int>(), s->start.as<int>(),
                              s->tmp.as<int>(), err, st));
-    CanonArgs ca{};
-    ca.n = n;
-    ca.tmp = s->tmp.as<int>();
-    ca.key = s->key.as<int>();
-    ca.start = s->start.as<int>();
-    ca.count = s->count[0].as<int>();
-    ca.tag_in = s->tag[0].as<int>();
-    ca.radius_in = s->radius[0].as<double>();
-    ca.inv_mass_in = s->inv_mass[0].as<double>();
-    ca.x = d3(s->pos[nsb], n, 0); ca.y = d3(s->pos[nsb], n, 1); ca.z = d3(s->pos[nsb], n, 2);
-    ca.perm = s->perm[0].as<int>();
-    ca.tag_out = s->tag[1].as<int>();
-    ca.radius_out = s->radius[1].as<double>();
-    ca.inv_mass_out = s->inv_mass[1].as<double>();
-    ca.cellid = s->cellid.as<int>();
-    ca.posh = s->posh.as<float4>();
-    ca.vel_freq = s->vp.vel_freq;
-    ca.err = err;
-    set_halo_args(s, ca, t + 1);   // list records, build positions and halo images on the new order
+    const CanonArgs ca = canon_args(s, nsb);
     PSIM_CUDA(launch_canonicalize(ca, st));
     // the state into the new order: positions, previous positions, noise
     // memory, and the forces of this step and the one before
@@ -1671,34 +1688,100 @@ void drop_graphs(psim_system* s) {
     drop(s->graph_multi);
 }
 
-// The graphs of n_steps steps from the system's step on, in order: visit(graph,
-// phase, steps, fused).  kGraphSteps steps at a time where a buffer period begins
+constexpr int kRunSteps = 1024;   // of one such launch
+
+// Whether stretches of its normal steps run in the one kernel of psim_run.cu: up to the
+// sizes its cluster holds, where it takes 5.6 to 8.5 us a step of the AO colloids and a
+// graph of single steps 17.4 (the LJ liquid of 6912: 19.3 against 27.7), so wherever it can.
+bool small_system(psim_system* s) {
+    if (!fused_steps(s) || s->n_reps) return false;
+    if (s->small < 0) s->small = run_list_fits(s->fs, s->n, s->ncell) ? 1 : 0;
+    return s->small == 1;
+}
+
+// The launches of n_steps steps from the system's step on, in order: visit(graph,
+// phase, steps, fused).  A small system's stretches of normal steps are one launch each
+// (graph null).  Otherwise kGraphSteps steps at a time where a buffer period begins
 // and all of them are of one kind, else single steps.  (A system whose velocity
 // steps come at least every kGraphSteps steps has no run of fused ones that long:
 // its multi-step graph is unfused.)
 template <class Visit>
-int each_graph(psim_system* s, int n_steps, Visit&& visit) {
+int each_launch(psim_system* s, int n_steps, Visit&& visit) {
     const bool fuse = fused_steps(s), one_kind = !fuse || s->vp.vel_freq < kGraphSteps - 1;
-    const bool multi = s->graph_multi || n_steps >= kGraphSteps + 5;
+    const bool small = small_system(s), multi = s->graph_multi || n_steps >= kGraphSteps + 5;
     int rc = PSIM_OK;
     for (long long t = s->total, end = t + n_steps; t < end && !rc;) {
-        bool run = multi && t % 6 == 0 && end - t >= kGraphSteps;
+        const int phase = (int)(t % 6);
+        if (small && normal_step(s, t)) {
+            // up to the next velocity step, and a few milliseconds at most
+            const long long period = s->vp.vel_freq + 1LL, to = (t / period + 1) * period;
+            const int steps = (int)std::min({to - t, end - t, (long long)kRunSteps});
+            rc = visit(nullptr, phase, steps, true);
+            t += steps;
+            continue;
+        }
+        bool run = !small && multi && t % 6 == 0 && end - t >= kGraphSteps;
         for (int k = 0; run && !one_kind && k < kGraphSteps; ++k) run = normal_step(s, t + k);
         const bool fused = fuse && (run ? !one_kind : normal_step(s, t));
-        const int phase = (int)(t % 6), steps = run ? kGraphSteps : 1;
-        rc = visit(run ? s->graph_multi : (fused ? s->fused[phase] : s->graph[phase]), phase, steps,
-                   fused);
+        const int steps = run ? kGraphSteps : 1;
+        rc = visit(run ? &s->graph_multi : (fused ? &s->fused[phase] : &s->graph[phase]), phase,
+                   steps, fused);
         t += steps;
     }
     return rc;
 }
 
+// steps normal steps from step s->total on in one kernel
+int enqueue_run(psim_system* s, int steps) {
+    const int n = s->n;
+    // a step is not captured by a caller (its stream is handed out): the number of steps
+    // and the phase of the state would be frozen into the launch
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PSIM_CUDA(cudaStreamIsCapturing(s->st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) PSIM_CUDA(cudaErrorStreamCaptureUnsupported);
+    RunArgs a{};
+    a.n = n;
+    a.ncell = s->ncell;
+    a.n_steps = steps;
+    for (int k = 0; k < 2; ++k) {
+        a.pos[k] = s->pos[k].as<double>();
+        a.pos0[k] = s->pos0[k].as<double>();
+        a.mem[k] = s->mem[k].as<double>();
+        a.lpos[k] = s->lpos[k].as<float4>();
+        a.tag[k] = s->tag[k].as<int>();
+        a.radius[k] = s->radius[k].as<double>();
+        a.inv_mass[k] = s->inv_mass[k].as<double>();
+        // the rebuild before a step of parity k
+        a.canon[k] = canon_args(s, k);
+    }
+    for (int k = 0; k < 3; ++k) a.frc[k] = s->frc[k].as<double>();
+    a.perm = s->perm[0].as<int>();
+    a.key = s->key.as<int>();
+    a.tmp = s->tmp.as<int>();
+    a.count = s->count[0].as<int>();
+    a.start = s->start.as<int>();
+    a.cv = list_cells(s, 0);
+    a.lb = list_build(s, nullptr);
+    a.pl = pair_list(s, phase_of(s->total));
+    a.linv_unit = 1.0f / s->lunit;
+    a.ldisp2 = s->ldisp2;
+    a.lbuild = s->lbuild.as<float4>();
+    a.lhalo = s->lhalo.as<int>();
+    a.lhcount = s->lhcount.as<int>();
+    a.lflag = s->lflag.as<int>();
+    a.state = s->state.as<StepState>();
+    a.err = s->err.as<uint32_t>();
+    const NoiseView nz{s->cfg.noise_mode, s->noise.as<double>(), s->noise_first, s->noise_steps};
+    PSIM_CUDA(launch_run_list(s->fs, s->g, a, s->vp, nz, s->st));
+    return PSIM_OK;
+}
+
 // The graphs of the next n_steps steps that are not captured yet.
 int capture_graphs(psim_system* s, int n_steps) {
-    return each_graph(s, n_steps, [&](cudaGraphExec_t& g, int phase, int steps, bool fused) {
-        if (g) return (int)PSIM_OK;
+    return each_launch(s, n_steps, [&](cudaGraphExec_t* g, int phase, int steps, bool fused) {
+        if (!g || *g) return (int)PSIM_OK;
         PSIM_CUDA(cudaStreamSynchronize(s->st));
-        return graph_steps(s, phase, steps, fused, &g);
+        return graph_steps(s, phase, steps, fused, g);
     });
 }
 
@@ -2302,8 +2385,12 @@ int psim_system_step_async(psim_system* s, int32_t n_steps) {
     if (n_steps < 0) return fail(PSIM_ERR_INPUT, "negative step count");
     DeviceGuard dg(s->device);
     if (int rc = capture_graphs(s, n_steps)) return rc;   // before anything is in flight
-    return each_graph(s, n_steps, [&](cudaGraphExec_t& g, int, int steps, bool) {
-        PSIM_CUDA(cudaGraphLaunch(g, s->st));
+    return each_launch(s, n_steps, [&](cudaGraphExec_t* g, int, int steps, bool) {
+        if (g) {
+            PSIM_CUDA(cudaGraphLaunch(*g, s->st));
+        } else if (int rc = enqueue_run(s, steps)) {
+            return rc;
+        }
         s->total += steps;
         return (int)PSIM_OK;
     });
@@ -2800,14 +2887,19 @@ int psim_system_launches_per_step(psim_system* s) {
     // force, vGB, scan x3, scatter, canonicalise (+1 memset node); with a
     // pair list: force, vGB (one kernel on normal steps where fused_steps
     // allows), step end (the rebuild's kernels run on the steps that rebuild:
-    // psim_system_launches_per_rebuild)
-    return (s && s->list_on) ? (fused_steps(s) ? 2 : 3) : 7;
+    // psim_system_launches_per_rebuild); a small system's normal step alone, or a
+    // stretch of them, is one kernel with its rebuilds
+    if (!s || !s->list_on) return 7;
+    DeviceGuard dg(s->device);
+    return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
 }
 
 int psim_system_launches_per_rebuild(psim_system* s) {
     // hash + count, scan x3, scatter, canonicalise, state permutation, list
     // build (+ memset and copy nodes)
-    return (s && s->list_on) ? 8 : 0;
+    if (!s || !s->list_on) return 0;
+    DeviceGuard dg(s->device);
+    return small_system(s) ? 0 : 8;
 }
 
 int psim_system_cell_occupancy(psim_system* s, int32_t* max_occ, double* mean_occ) {

@@ -144,6 +144,14 @@ __device__ __forceinline__ double widen_f32(float f) {
     return __longlong_as_double((long long)(sign | (ed << 52) | m));
 }
 
+// *p through the read-only path (kNc: nothing writes it while the kernel runs) or
+// plainly.
+template <bool kNc, class T>
+__device__ __forceinline__ T load_as(const T* p) {
+    if constexpr (kNc) return __ldg(p);
+    return *p;
+}
+
 // 1/a and 1/sqrt(a) to about an ulp in 3 and 5 FP64 operations, from the
 // hardware's ~20-bit seeds (rcp.approx / rsqrt.approx, not on the FP64 unit) and
 // one third-order Householder iteration: with h = 1 - a y (1 - a y^2) the seed's

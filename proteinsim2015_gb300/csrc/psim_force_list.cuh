@@ -44,7 +44,13 @@ __device__ __forceinline__ void load_record(const float4* pos, uint32_t j, float
 // One group of kListFold = 8 list entries (32 bytes, 32-byte aligned) in a
 // single 256-bit load through the read-only path: a warp's request covers
 // its 1 KB once, where two 128-bit loads would each cover all of it.
+template <bool kNc>
 __device__ __forceinline__ void load_group(const uint32_t* p, uint4& a, uint4& b) {
+    if constexpr (!kNc) {
+        a = reinterpret_cast<const uint4*>(p)[0];
+        b = reinterpret_cast<const uint4*>(p)[1];
+        return;
+    }
     asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
         : "l"(p));
@@ -60,10 +66,12 @@ template <>
 struct ListRec<false> {
     float4 h, l;
 };
+template <bool kNc>
 __device__ __forceinline__ ListRec<true> load_rec(const float4* pos, uint32_t j,
                                                   ListRec<true>) {
-    return ListRec<true>{__ldg(pos + j)};
+    return ListRec<true>{load_as<kNc>(pos + j)};
 }
+template <bool kNc>
 __device__ __forceinline__ ListRec<false> load_rec(const float4* pos, uint32_t j,
                                                    ListRec<false>) {
     ListRec<false> r;
@@ -90,7 +98,8 @@ __device__ __forceinline__ ListRec<false> load_rec(const float4* pos, uint32_t j
 // exact for nearby values.  Either way d carries one FP32 rounding.  The
 // lanes of a particle are adjacent in one warp; lane 0 adds the others' sums
 // in lane order, so the result does not depend on scheduling.
-template <class Body, bool kCompact, bool kCount, int kLanes>
+// kNc: no one writes the list or the records while the kernel runs.
+template <class Body, bool kCompact, bool kCount, int kLanes, bool kNc = true>
 __device__ __forceinline__ void list_terms(const Body& body, const PairList& pl, int s, int lane,
                                            typename Body::Acc& acc, float& rmin, uint32_t& err) {
     constexpr int kBatch = 4;
@@ -147,7 +156,7 @@ __device__ __forceinline__ void list_terms(const Body& body, const PairList& pl,
     // (gp at the first; group kLanes m exists)
     auto load_view = [&](const uint32_t* p, int m, uint4& a, uint4& b) {
         if constexpr (kLanes == 1) {
-            load_group(p, a, b);
+            load_group<kNc>(p, a, b);
         } else if constexpr (kLanes == 2) {
             a = __ldg(reinterpret_cast<const uint4*>(p));
             b = 2 * m + 1 < groups ? __ldg(reinterpret_cast<const uint4*>(p + gs))
@@ -169,24 +178,24 @@ __device__ __forceinline__ void list_terms(const Body& body, const PairList& pl,
     uint4 ea = make_uint4(0u, 0u, 0u, 0u), eb = ea;
     Rec r[kBatch], rn[kBatch];
     if (views > 0) load_view(gp, 0, ea, eb);
-    r[0] = load_rec(pl.pos, ea.x, none);
-    r[1] = load_rec(pl.pos, ea.y, none);
-    r[2] = load_rec(pl.pos, ea.z, none);
-    r[3] = load_rec(pl.pos, ea.w, none);
+    r[0] = load_rec<kNc>(pl.pos, ea.x, none);
+    r[1] = load_rec<kNc>(pl.pos, ea.y, none);
+    r[2] = load_rec<kNc>(pl.pos, ea.z, none);
+    r[3] = load_rec<kNc>(pl.pos, ea.w, none);
     for (int m = 0; m < views; ++m) {
         const bool more = m + 1 < views;
         gp += gs * kLanes;
         uint4 na = make_uint4(0u, 0u, 0u, 0u), nb = na;
         if (more) load_view(gp, m + 1, na, nb);
-        rn[0] = load_rec(pl.pos, eb.x, none);
-        rn[1] = load_rec(pl.pos, eb.y, none);
-        rn[2] = load_rec(pl.pos, eb.z, none);
-        rn[3] = load_rec(pl.pos, eb.w, none);
+        rn[0] = load_rec<kNc>(pl.pos, eb.x, none);
+        rn[1] = load_rec<kNc>(pl.pos, eb.y, none);
+        rn[2] = load_rec<kNc>(pl.pos, eb.z, none);
+        rn[3] = load_rec<kNc>(pl.pos, eb.w, none);
         terms(r);
-        r[0] = load_rec(pl.pos, na.x, none);
-        r[1] = load_rec(pl.pos, na.y, none);
-        r[2] = load_rec(pl.pos, na.z, none);
-        r[3] = load_rec(pl.pos, na.w, none);
+        r[0] = load_rec<kNc>(pl.pos, na.x, none);
+        r[1] = load_rec<kNc>(pl.pos, na.y, none);
+        r[2] = load_rec<kNc>(pl.pos, na.z, none);
+        r[3] = load_rec<kNc>(pl.pos, na.w, none);
         terms(rn);
         body.fold(acc);
         eb = nb;

@@ -325,6 +325,45 @@ struct CanonArgs {
 };
 cudaError_t launch_canonicalize(const CanonArgs& a, cudaStream_t st);
 
+// Many normal steps of a small system with a pair list in one kernel
+// (psim_run.cu): the buffers of every phase, the rebuild's arguments for the two
+// parities of the records, and the steps to take.  The state after them is where
+// that many single steps would have put it; the step state is advanced, and an error
+// is latched with the state of the failing step.
+constexpr int kRunMaxN = 16 * 512;
+constexpr int kRunMaxCells = 1 << 16;
+struct RunArgs {
+    int n, ncell, n_steps;
+    double* pos[2];
+    double* pos0[2];
+    double* mem[2];
+    double* frc[3];
+    float4* lpos[2];
+    int* tag[2];
+    double* radius[2];
+    double* inv_mass[2];
+    int* perm;
+    int* key;
+    int* tmp;
+    int* count;
+    int* start;
+    CanonArgs canon[2];     // positions and records of the step's parity
+    CellView cv;
+    ListBuild lb;
+    PairList pl;            // pos is set per step
+    float linv_unit, ldisp2;
+    const float4* lbuild;
+    const int* lhalo;
+    int* lhcount;
+    int* lflag;
+    StepState* state;
+    uint32_t* err;
+};
+// Whether a system of these sizes can run so on the current device.
+bool run_list_fits(const ForceSetup& fs, int n, int ncell);
+cudaError_t launch_run_list(const ForceSetup& fs, const DevGeom& g, const RunArgs& a,
+                            const VgbParams& p, const NoiseView& nz, cudaStream_t st);
+
 // Full 32-byte pair-list records of the sorted positions (posh, posl) and
 // the halo images of the particles within hr of a face (lhalo per slot,
 // records n + 1 + [0, hcap) handed out by *lhcount, zeroed by the caller).

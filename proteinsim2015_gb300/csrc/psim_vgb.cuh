@@ -260,11 +260,13 @@ __device__ __forceinline__ void load_noise_f(const NoiseView& nz, uint32_t seed,
 // positions into the next grid.
 // The new position in pair-list order: the periodic image nearest the
 // position at the list build (|x - build| < L/2 picks it), as an exact float
-// pair; raises the rebuild flag when it has moved more than sqrt(ldisp2).
-// s, b, hal: the particle's list slot, its position at the build and its halo
-// word, loaded before the update so that their latency overlaps it.
-__device__ __forceinline__ void list_position(const VgbSystemArgs& a, int s, const float4& b,
-                                              int hal, const double xn[3], const DevGeom& g) {
+// pair, into record s of lpos (n of them before the ghost) and its halo images;
+// whether it has moved more than sqrt(ldisp2) from the build.
+// b, hal: the particle's position at the build and its halo word, loaded before
+// the update so that their latency overlaps it.
+__device__ __forceinline__ bool list_record(float4* lpos, float linv_unit, int n, float ldisp2,
+                                            int s, const float4& b, int hal, const double xn[3],
+                                            const DevGeom& g) {
     const float bb[3] = {b.x, b.y, b.z};
     const float halff = 0.5f * g.Lhi;
     float h[3], l[3], d2 = 0.f;
@@ -278,11 +280,15 @@ __device__ __forceinline__ void list_position(const VgbSystemArgs& a, int s, con
         d2 += e * e;
     }
     const float4 hv = make_float4(h[0], h[1], h[2], b.w), lv = make_float4(l[0], l[1], l[2], 0.f);
-    store_record(a.lpos, a.linv_unit, (size_t)s, hv, lv);
+    store_record(lpos, linv_unit, (size_t)s, hv, lv);
     if (hal & 63)  // the particle's periodic images in the halo records
-        halo_write(a.lpos + (a.linv_unit != 0.f ? 1 : 2) * ((size_t)a.n + 1), a.linv_unit,
-                   hal >> 6, (uint32_t)(hal & 63), hv, lv, g.Lhi, g.Llo);
-    if (d2 > a.ldisp2) *a.lflag_set = 1;
+        halo_write(lpos + (linv_unit != 0.f ? 1 : 2) * ((size_t)n + 1), linv_unit, hal >> 6,
+                   (uint32_t)(hal & 63), hv, lv, g.Lhi, g.Llo);
+    return d2 > ldisp2;
+}
+__device__ __forceinline__ void list_position(const VgbSystemArgs& a, int s, const float4& b,
+                                              int hal, const double xn[3], const DevGeom& g) {
+    if (list_record(a.lpos, a.linv_unit, a.n, a.ldisp2, s, b, hal, xn, g)) *a.lflag_set = 1;
 }
 
 // One particle of the system-order update (slot f), with its system's
