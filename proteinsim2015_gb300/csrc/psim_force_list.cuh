@@ -250,20 +250,21 @@ force_list_kernel(Body body0, DevGeom g, PairList pl, ForceOut out) {
 template <class Body, bool kCompact, bool kReplicas, bool kCount, bool kMulti>
 cudaError_t launch_list_lanes(const Body& body, const DevGeom& g, const PairList& pl,
                               const ForceOut& out, int lanes, cudaStream_t st) {
+    const long long items = (long long)g.n * lanes;
+    const int threads = block_threads(items), blocks = (int)((items + threads - 1) / threads);
     if constexpr (kMulti) {
         if (lanes == 2 || lanes == 4) {
-            const int blocks = (int)(((long long)g.n * lanes + 255) / 256);
             if (lanes == 4)
                 force_list_kernel<Body, kCompact, kReplicas, kCount, 4>
-                    <<<blocks, 256, 0, st>>>(body, g, pl, out);
+                    <<<blocks, threads, 0, st>>>(body, g, pl, out);
             else
                 force_list_kernel<Body, kCompact, kReplicas, kCount, 2>
-                    <<<blocks, 256, 0, st>>>(body, g, pl, out);
+                    <<<blocks, threads, 0, st>>>(body, g, pl, out);
             return cudaGetLastError();
         }
     }
-    force_list_kernel<Body, kCompact, kReplicas, kCount, 1><<<(g.n + 255) / 256, 256, 0, st>>>(
-        body, g, pl, out);
+    force_list_kernel<Body, kCompact, kReplicas, kCount, 1><<<blocks, threads, 0, st>>>(body, g, pl,
+                                                                                    out);
     return cudaGetLastError();
 }
 

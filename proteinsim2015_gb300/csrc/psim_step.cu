@@ -62,15 +62,15 @@ cudaError_t launch_step_list(const ForceSetup& fs, const DevGeom& g, const PairL
     return with_pair(fs, [&](auto pair, float rc2f) -> cudaError_t {
         using Body = MixedBody<decltype(pair)>;
         const Body body{pair, rc2f};
-        const int blocks = (a.n + 255) / 256;
+        const int threads = block_threads(a.n), blocks = (a.n + threads - 1) / threads;
         if (pl.rep) {
             if constexpr (Body::kBatchable) {
-                step_list_kernel<Body, true><<<blocks, 256, 0, st>>>(body, g, pl, a, p, nz);
+                step_list_kernel<Body, true><<<blocks, threads, 0, st>>>(body, g, pl, a, p, nz);
                 return cudaGetLastError();
             }
             return cudaErrorInvalidValue;
         }
-        step_list_kernel<Body, false><<<blocks, 256, 0, st>>>(body, g, pl, a, p, nz);
+        step_list_kernel<Body, false><<<blocks, threads, 0, st>>>(body, g, pl, a, p, nz);
         return cudaGetLastError();
     });
 }

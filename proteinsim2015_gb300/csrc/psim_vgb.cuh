@@ -414,11 +414,11 @@ template <class Tag>
 cudaError_t launch_vgb_system_t(const VgbSystemArgs& a, const VgbParams& p, const DevGeom& g,
                                 const NoiseView& nz, cudaStream_t st) {
     if (a.n == 0) return cudaSuccess;
-    const int blocks = (a.n + 255) / 256;
+    const int threads = block_threads(a.n), blocks = (a.n + threads - 1) / threads;
     if (a.rep)
-        vgb_system_kernel<Tag, true><<<blocks, 256, 0, st>>>(a, p, g, nz);
+        vgb_system_kernel<Tag, true><<<blocks, threads, 0, st>>>(a, p, g, nz);
     else
-        vgb_system_kernel<Tag, false><<<blocks, 256, 0, st>>>(a, p, g, nz);
+        vgb_system_kernel<Tag, false><<<blocks, threads, 0, st>>>(a, p, g, nz);
     return cudaGetLastError();
 }
 
