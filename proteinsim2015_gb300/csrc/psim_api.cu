@@ -1283,6 +1283,12 @@ void set_halo_args(psim_system* s, CanonArgs& ca, long long t) {
     }
 }
 
+// Whether the cell order is made by one kernel.
+bool one_order(const psim_system* s) { return order_fits(s->n, s->ncell); }
+OrderArgs order_args(psim_system* s, int cb) {
+    return OrderArgs{s->ncell, s->key.as<int>(), s->count[cb].as<int>(), s->start.as<int>()};
+}
+
 // The cell order a pair list is built on (count buffer cb), and its build.
 CellView list_cells(psim_system* s, int cb) {
     return CellView{nullptr, s->posh.as<float4>(), s->posl.as<float4>(), s->cellid.as<int>(),
@@ -1391,9 +1397,9 @@ int enqueue_rebuild_lazy(psim_system* s, long long t) {
     const int n = s->n, nsb = 1 - ph.sb;
     cudaStream_t st = s->st;
     uint32_t* err = s->err.as<uint32_t>();
+    const CanonArgs ca = canon_args(s, nsb);
     PSIM_CUDA(cudaMemsetAsync(s->count[0].p, 0, 4 * (size_t)s->ncell, st));
-    PSIM_CUDA(launch_hash_count(n, d3(s->pos[nsb], n, 0), d3(s->pos[nsb], n, 1),
-                                d3(s->pos[nsb], n, 2), s->g, s->key.as<int>(), s->rank.as<int>(),
+    PSIM_CUDA(launch_hash_count(n, ca.x, ca.y, ca.z, s->g, s->key.as<int>(), s->rank.as<int>(),
                                 s->count[0].as<int>(), err, st,
                                 s->n_reps ? s->b_rep.as<int>() : nullptr,
                                 s->n_reps ? s->b_geoms.as<DevGeom>() : nullptr));
@@ -1401,7 +1407,6 @@ int enqueue_rebuild_lazy(psim_system* s, long long t) {
                           s->scratch.as<int>(), st));
     PSIM_CUDA(launch_scatter(n, s->key.as<int>(), s->rank.as<int>(), s->start.as<int>(),
                              s->tmp.as<int>(), err, st));
-    const CanonArgs ca = canon_args(s, nsb);
     PSIM_CUDA(launch_canonicalize(ca, st));
     // the state into the new order: positions, previous positions, noise
     // memory, and the forces of this step and the one before
@@ -1513,8 +1518,10 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
                 s->err.as<uint32_t>(), nullptr};
     PSIM_CUDA(enqueue_force(s, ph, fo));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[1], st));
-    // integrator: pushParticleForce + nextSystem, hash + count into the next grid
-    PSIM_CUDA(cudaMemsetAsync(s->count[ncb].p, 0, 4 * (size_t)s->ncell, st));
+    // integrator: pushParticleForce + nextSystem, hash + count into the next grid (left to
+    // the kernel of the whole order where there is one)
+    const bool one = one_order(s);
+    if (!one) PSIM_CUDA(cudaMemsetAsync(s->count[ncb].p, 0, 4 * (size_t)s->ncell, st));
     VgbSystemArgs a{};
     a.n = n;
     a.perm = s->perm[pb].as<int>();
@@ -1532,7 +1539,7 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     a.omx = d3(s->mem[nsb], n, 0); a.omy = d3(s->mem[nsb], n, 1); a.omz = d3(s->mem[nsb], n, 2);
     a.key = s->key.as<int>();
     a.rank = s->rank.as<int>();
-    a.count = s->count[ncb].as<int>();
+    a.count = one ? nullptr : s->count[ncb].as<int>();
     a.err = s->err.as<uint32_t>();
     a.state = s->state.as<StepState>();
     if (s->n_reps) {
@@ -1548,10 +1555,12 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
         PSIM_CUDA(launch_vgb_system_fast(a, s->vp, s->g, nz, st));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[2], st));
     // rebuild: scan, scatter, canonicalise into the next order
-    PSIM_CUDA(launch_scan(s->count[ncb].as<int>(), s->start.as<int>(), s->ncell,
-                          s->scratch.as<int>(), st));
-    PSIM_CUDA(launch_scatter(n, s->key.as<int>(), s->rank.as<int>(), s->start.as<int>(),
-                             s->tmp.as<int>(), s->err.as<uint32_t>(), st));
+    if (!one) {
+        PSIM_CUDA(launch_scan(s->count[ncb].as<int>(), s->start.as<int>(), s->ncell,
+                              s->scratch.as<int>(), st));
+        PSIM_CUDA(launch_scatter(n, s->key.as<int>(), s->rank.as<int>(), s->start.as<int>(),
+                                 s->tmp.as<int>(), s->err.as<uint32_t>(), st));
+    }
     CanonArgs ca{};
     ca.n = n;
     ca.tmp = s->tmp.as<int>();
@@ -1574,7 +1583,10 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     ca.advance = 1;
     ca.vel_freq = s->vp.vel_freq;
     ca.err = s->err.as<uint32_t>();
-    PSIM_CUDA(launch_canonicalize(ca, st));
+    if (one)
+        PSIM_CUDA(launch_order(order_args(s, ncb), ca, st));
+    else
+        PSIM_CUDA(launch_canonicalize(ca, st));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[3], st));
     return PSIM_OK;
 }
@@ -1757,9 +1769,7 @@ int enqueue_run(psim_system* s, int steps) {
     for (int k = 0; k < 3; ++k) a.frc[k] = s->frc[k].as<double>();
     a.perm = s->perm[0].as<int>();
     a.key = s->key.as<int>();
-    a.tmp = s->tmp.as<int>();
-    a.count = s->count[0].as<int>();
-    a.start = s->start.as<int>();
+    a.order = order_args(s, 0);
     a.cv = list_cells(s, 0);
     a.lb = list_build(s, nullptr);
     a.pl = pair_list(s, phase_of(s->total));
@@ -2884,12 +2894,13 @@ int psim_system_profile(psim_system* s, int32_t n_steps, double* out_ms) {
 }
 
 int psim_system_launches_per_step(psim_system* s) {
-    // force, vGB, scan x3, scatter, canonicalise (+1 memset node); with a
-    // pair list: force, vGB (one kernel on normal steps where fused_steps
+    // force, vGB, scan x3, scatter, canonicalise (+1 memset node), or force, vGB and
+    // the one kernel of a small system's cell order; with a pair list: force, vGB (one kernel on normal steps where fused_steps
     // allows), step end (the rebuild's kernels run on the steps that rebuild:
     // psim_system_launches_per_rebuild); a small system's normal step alone, or a
     // stretch of them, is one kernel with its rebuilds
-    if (!s || !s->list_on) return 7;
+    if (!s) return 7;
+    if (!s->list_on) return one_order(s) ? 3 : 7;
     DeviceGuard dg(s->device);
     return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
 }

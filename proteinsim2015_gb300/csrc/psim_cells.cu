@@ -19,6 +19,8 @@ namespace {
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanBlock * kScanItems;
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderMaxN = 3 << 13;
 
 __device__ __forceinline__ int block_scan_exclusive(int v, int* warp_tot, int& total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -129,20 +131,43 @@ __global__ void __launch_bounds__(256) canonicalize_kernel(CanonArgs a, int vel_
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.err && *a.err) return;
     if (p < a.n) canon_slot(a, p);
-    if (a.state && a.advance && p == 0) {
-        // end of a step: brownianIntegrator's velCounter bookkeeping
-        // (brownianIntegrator.cpp:291-292) runs only after normal steps
-        StepState s = *a.state;
-        if (s.step > 0) s.vel_counter = (s.vel_counter == vel_freq) ? 0 : s.vel_counter + 1;
-        s.step += 1;
-        if (a.rebuild && *a.rebuild) s.list_builds += 1;
-        *a.state = s;
-    }
+    if (a.state && a.advance && p == 0) step_advance(a, vel_freq);
 }
 
 cudaError_t launch_canonicalize(const CanonArgs& a, cudaStream_t st) {
     const int blocks = a.n > 0 ? (a.n + 255) / 256 : 1;
     canonicalize_kernel<<<blocks, 256, 0, st>>>(a, a.vel_freq);
+    return cudaGetLastError();
+}
+
+// The cell order of a small system and the end of its step (block_order), where the
+// cells and the particles' 16-bit records fit a block's shared memory.  Latency bounds it:
+// one kernel takes the place of five and a memset.  us a step of AO colloids in FP64, the
+// chain of kernels and this one: 1001 particles 27.7 -> 20.0, 4000 28.0 -> 22.0, 8000
+// 28.6 -> 23.4, 16000 30.5 -> 28.1, 20001 32.4 -> 29.8 (every block counts all particles:
+// near 30000 the two meet); the LJ liquid of 13500 75.7 -> 71.0.
+__global__ void __launch_bounds__(kOrderThreads)
+order_kernel(OrderArgs o, CanonArgs c, int vel_freq) {
+    extern __shared__ int smem[];
+    if (*c.err) return;
+    const int b = blockIdx.x, blocks = gridDim.x;
+    const int fs = (c.n + blocks - 1) / blocks, cs = (o.ncell + blocks - 1) / blocks;
+    const bool ok = block_order(o, c, min(c.n, b * fs), min(c.n, (b + 1) * fs),
+                                min(o.ncell, b * cs), min(o.ncell, (b + 1) * cs), smem);
+    if (ok && b == 0 && threadIdx.x == 0 && c.state && c.advance) step_advance(c, vel_freq);
+}
+
+bool order_fits(int n, int ncell) {
+    return n >= 1 && n <= kOrderMaxN && ncell <= kOrderIndex && order_smem(n, ncell) <= kOrderSmem;
+}
+
+cudaError_t launch_order(const OrderArgs& o, const CanonArgs& c, cudaStream_t st) {
+    if (!order_fits(c.n, o.ncell) || !c.err) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(
+        order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrderSmem);
+    if (e != cudaSuccess) return e;
+    const int blocks = std::min(32, (c.n + 255) / 256);
+    order_kernel<<<blocks, kOrderThreads, order_smem(c.n, o.ncell), st>>>(o, c, c.vel_freq);
     return cudaGetLastError();
 }
 

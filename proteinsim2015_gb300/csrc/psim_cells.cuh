@@ -1,18 +1,16 @@
-// psim_cells.cuh -- the canonical order of one slot of the counting sort, shared by
-// canonicalize_kernel and the kernel that runs small systems (psim_run.cu).
+// psim_cells.cuh -- the canonical order within a cell, and the whole cell order of a
+// small system by one block, shared by psim_cells.cu and psim_run.cu.
 #pragma once
 
 #include "psim_kernels.cuh"
 
 namespace psim {
 
-// Slot p of the scattered order: its particle's place inside its cell, and there
-// everything the force pass reads.
-__device__ __forceinline__ void canon_slot(const CanonArgs& a, int p) {
-    const int f = a.tmp[p];
-    const int c = a.key[f];
-    const int st = a.start[c];
-    const int cnt = a.count[c];
+// Particle f's place inside its cell c, whose cnt slots from st on hold the particles
+// tmp(st) .. (scattered in any order), and there everything the force pass reads.
+template <class Tmp>
+__device__ __forceinline__ void canon_place(const CanonArgs& a, int f, int c, int st, int cnt,
+                                            Tmp tmp) {
     const int mine = a.tag_in[f];
     int r = 0;
     if (a.xorder) {
@@ -20,12 +18,12 @@ __device__ __forceinline__ void canon_slot(const CanonArgs& a, int p) {
         // order like their values, and every pattern is comparable
         const long long mx = __double_as_longlong(a.x[f]);
         for (int q = st; q < st + cnt; ++q) {
-            const int fq = a.tmp[q];
+            const int fq = tmp(q);
             const long long xq = __double_as_longlong(a.x[fq]);
             r += (xq < mx || (xq == mx && a.tag_in[fq] < mine)) ? 1 : 0;
         }
     } else {
-        for (int q = st; q < st + cnt; ++q) r += (a.tag_in[a.tmp[q]] < mine) ? 1 : 0;
+        for (int q = st; q < st + cnt; ++q) r += (a.tag_in[tmp(q)] < mine) ? 1 : 0;
     }
     const int g = st + r;
     a.perm[g] = f;
@@ -79,6 +77,92 @@ __device__ __forceinline__ void canon_slot(const CanonArgs& a, int p) {
             a.lhalo[g] = (base << 6) | (int)fl;
         }
     }
+}
+
+__device__ __forceinline__ void canon_slot(const CanonArgs& a, int p) {
+    const int f = a.tmp[p], c = a.key[f];
+    canon_place(a, f, c, a.start[c], a.count[c], [&](int q) { return a.tmp[q]; });
+}
+
+// The whole order by one block that holds the cells and the particles' keys in shared
+// memory.  The blocks of a kernel each count and scatter every particle -- a few
+// microseconds of shared-memory work that needs no other block -- and place only their
+// own: particles [f0, f1) and, in o.start and o.count, cells [c0, c1).  False, in every
+// thread of every block, when a particle has no cell (a negative key): nothing is
+// written.
+// The block's shared memory: starts of the cells, then key, rank and scattered order.
+__host__ __device__ inline size_t order_smem(int n, int ncell) {
+    return 4 * (size_t)(ncell + 1 + 32) + 6 * (size_t)n;
+}
+constexpr int kOrderIndex = 1 << 16;   // keys and particles are 16-bit
+__device__ __forceinline__ bool block_order(const OrderArgs& o, const CanonArgs& c,
+                                            int f0, int f1, int c0, int c1, int* smem) {
+    const int T = blockDim.x, tid = threadIdx.x, n = c.n, ncell = o.ncell;
+    int* start = smem;
+    int* warp = smem + ncell + 1;
+    uint16_t* key = reinterpret_cast<uint16_t*>(warp + 32);
+    uint16_t* rank = key + n;
+    uint16_t* tmp = rank + n;
+    for (int k = tid; k < ncell; k += T) start[k] = 0;
+    __syncthreads();
+    bool bad = false;
+    for (int i0 = tid; i0 < n; i0 += 4 * T) {   // four loads in flight
+        int k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = o.key[min(i0 + u * T, n - 1)];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * T;
+            bad = bad || k[u] < 0;
+            if (i >= n || k[u] < 0) continue;
+            key[i] = (uint16_t)k[u];
+            rank[i] = (uint16_t)atomicAdd(&start[k[u]], 1);
+        }
+    }
+    if (__syncthreads_or(bad)) return false;
+    // counts to starts, a run of cells per thread
+    const int per = (ncell + T - 1) / T, b0 = min(ncell, tid * per), b1 = min(ncell, b0 + per);
+    int sum = 0;
+    for (int k = b0; k < b1; ++k) sum += start[k];
+    const int lane = tid & 31, w = tid >> 5;
+    int x = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31) warp[w] = x;
+    __syncthreads();
+    int run = x - sum;
+    for (int k = 0; k < w; ++k) run += warp[k];
+    for (int k = b0; k < b1; ++k) {
+        const int m = start[k];
+        start[k] = run;
+        run += m;
+    }
+    if (tid == 0) start[ncell] = n;
+    __syncthreads();
+    for (int i = tid; i < n; i += T) tmp[start[key[i]] + rank[i]] = (uint16_t)i;
+    for (int k = c0 + tid; k < c1; k += T) {
+        o.start[k] = start[k];
+        o.count[k] = start[k + 1] - start[k];
+    }
+    __syncthreads();
+    for (int f = f0 + tid; f < f1; f += T) {
+        const int k = key[f], st = start[k];
+        canon_place(c, f, k, st, start[k + 1] - st, [&](int q) { return (int)tmp[q]; });
+    }
+    return true;
+}
+
+// The end of a step: brownianIntegrator's velCounter bookkeeping
+// (brownianIntegrator.cpp:291-292) runs only after normal steps.
+__device__ __forceinline__ void step_advance(const CanonArgs& a, int vel_freq) {
+    StepState s = *a.state;
+    if (s.step > 0) s.vel_counter = (s.vel_counter == vel_freq) ? 0 : s.vel_counter + 1;
+    s.step += 1;
+    if (a.rebuild && *a.rebuild) s.list_builds += 1;
+    *a.state = s;
 }
 
 }  // namespace psim

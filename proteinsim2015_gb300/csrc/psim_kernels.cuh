@@ -337,13 +337,26 @@ struct CanonArgs {
 };
 cudaError_t launch_canonicalize(const CanonArgs& a, cudaStream_t st);
 
+// The cell order of a small system in one kernel (order_kernel): counts of the keys,
+// start, and the canonical order -- what launch_scan, launch_scatter and
+// launch_canonicalize leave.
+struct OrderArgs {
+    int ncell;
+    const int* key;         // cell of each particle (negative: none, an error)
+    int* count;
+    int* start;
+};
+constexpr int kOrderSmem = 220 << 10;   // shared memory of a block at most
+// Whether a system of these sizes is ordered so.
+bool order_fits(int n, int ncell);
+cudaError_t launch_order(const OrderArgs& o, const CanonArgs& c, cudaStream_t st);
+
 // Many normal steps of a small system with a pair list in one kernel
 // (psim_run.cu): the buffers of every phase, the rebuild's arguments for the two
 // parities of the records, and the steps to take.  The state after them is where
 // that many single steps would have put it; the step state is advanced, and an error
 // is latched with the state of the failing step.
 constexpr int kRunMaxN = 16 * 512;
-constexpr int kRunMaxCells = 1 << 16;
 struct RunArgs {
     int n, ncell, n_steps;
     double* pos[2];
@@ -356,9 +369,7 @@ struct RunArgs {
     double* inv_mass[2];
     int* perm;
     int* key;
-    int* tmp;
-    int* count;
-    int* start;
+    OrderArgs order;
     CanonArgs canon[2];     // positions and records of the step's parity
     CellView cv;
     ListBuild lb;

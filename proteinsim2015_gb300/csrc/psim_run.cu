@@ -83,92 +83,58 @@ __device__ __forceinline__ void store_state(const RunArgs& a, long long t, int f
     }
 }
 
-struct RunShared {
-    uint32_t flags[3];                // reports of the cluster, by step number mod 3
-    int totals[kRunBlocks];           // scan: every block's cells
-    int warp[32];
-};
-
-// start[c] = the counts of the cells before c, each block a contiguous share of the
-// cells.  A cluster barrier is passed in the middle.
-__device__ __forceinline__ void run_scan(const RunArgs& a, RunShared& sh,
-                                         cg::cluster_group& cluster) {
-    const int rank = (int)cluster.block_rank(), T = blockDim.x;
-    const int share = (a.ncell + kRunBlocks - 1) / kRunBlocks, per = (share + T - 1) / T;
-    const int c0 = rank * share, c1 = min(a.ncell, c0 + share);
-    const int b0 = min(c1, c0 + (int)threadIdx.x * per), b1 = min(c1, b0 + per);
-    int sum = 0;
-    for (int c = b0; c < b1; ++c) sum += a.count[c];
-    // exclusive scan of the threads' sums over the block
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) sh.warp[w] = x;
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int k = 0; k < T / 32; ++k) {
-        if (k < w) before += sh.warp[k];
-        total += sh.warp[k];
-    }
-    if (threadIdx.x < kRunBlocks) *cluster.map_shared_rank(&sh.totals[rank], threadIdx.x) = total;
-    cluster_barrier();
-    int run = before + x - sum;
-    for (int k = 0; k < rank; ++k) run += sh.totals[k];
-    for (int c = b0; c < b1; ++c) {
-        a.start[c] = run;
-        run += a.count[c];
-    }
-}
 
 // The rebuild before step t: the state into the new cell order, the list on it.
-__device__ __forceinline__ void run_rebuild(const RunArgs& a, const DevGeom& g, long long t,
-                                            int f, bool active, RunShared& sh,
+// False, in every thread, where it failed.
+__device__ __forceinline__ bool run_rebuild(const RunArgs& a, const DevGeom& g, long long t,
+                                            int f, bool active, int* smem,
                                             cg::cluster_group& cluster, RunState& s, int& tag,
-                                            double& m, uint32_t& err) {
-    const int q = (int)(t & 1), threads = kRunBlocks * blockDim.x;
+                                            double& m) {
+    const int q = (int)(t & 1);
     if (active) store_state(a, t, f, s);
-    for (int c = f; c < a.ncell; c += threads) a.count[c] = 0;
+    if (active) {
+        uint32_t err = 0;
+        const int key = hash_pos(s.x, g, err);
+        if (err) atomicOr(a.err, err);
+        a.key[f] = err ? -1 : key;
+    }
     if (f == 0) *a.lhcount = 0;
     cluster_barrier();
-    int key = 0, rank = 0;
-    if (active) {
-        key = hash_pos(s.x, g, err);
-        rank = atomicAdd(&a.count[key], 1);
-        a.key[f] = key;
-    }
+    const int block = (int)cluster.block_rank(), T = blockDim.x;
+    const int share = (a.order.ncell + kRunBlocks - 1) / kRunBlocks;
+    const bool ok = block_order(a.order, a.canon[q], min(a.n, block * T),
+                                min(a.n, (block + 1) * T), min(a.order.ncell, block * share),
+                                min(a.order.ncell, (block + 1) * share), smem);
     cluster_barrier();
-    run_scan(a, sh, cluster);
-    cluster_barrier();
-    if (active) a.tmp[a.start[key] + rank] = f;
-    cluster_barrier();
-    if (active) canon_slot(a.canon[q], f);
-    cluster_barrier();
+    if (!ok) return false;   // the same in every block
+    uint32_t err = 0;
     if (active) {
         load_state(a, t, a.perm[f], s);
         tag = a.tag[1][f];
         m = a.inv_mass[1][f];
         list_build_one<false>(g, a.cv, a.lb, a.lb.pre_r2, f, err);
     }
+    if (err) atomicOr(a.err, err);
     cluster_barrier();   // every slot's state is read
     if (active) {
         a.tag[0][f] = tag;
         a.inv_mass[0][f] = m;
         a.radius[0][f] = a.radius[1][f];
     }
+    const uint32_t bad = *(volatile const uint32_t*)a.err;
+    cluster_barrier();   // all have read it before a step may write it
+    return bad == 0;
 }
 
 template <class Body>
 __global__ void __launch_bounds__(kRunThreads, 1)
 run_list_kernel(Body body, DevGeom g, RunArgs a, VgbParams p, NoiseView nz) {
-    __shared__ RunShared sh;
+    __shared__ uint32_t flags[3];   // reports of the cluster, by step number mod 3
+    extern __shared__ int smem[];   // of a rebuild
     cg::cluster_group cluster = cg::this_cluster();
     const int f = (int)cluster.block_rank() * blockDim.x + threadIdx.x;
     const bool active = f < a.n;
-    if (threadIdx.x < 3) sh.flags[threadIdx.x] = 0u;
+    if (threadIdx.x < 3) flags[threadIdx.x] = 0u;
     const uint32_t failed = *(volatile const uint32_t*)a.err;
     const StepState at = *a.state;
     // every block has read the words before any writes them
@@ -222,28 +188,22 @@ run_list_kernel(Body body, DevGeom g, RunArgs a, VgbParams p, NoiseView nz) {
         // to every block: flags of this step number; those of the next are free, as
         // every warp has read the ones of two steps ago before the last barrier
         const int slot = done % 3;
-        if (threadIdx.x == 0) sh.flags[(slot + 1) % 3] = 0u;
+        if (threadIdx.x == 0) flags[(slot + 1) % 3] = 0u;
         report = __reduce_or_sync(0xffffffffu, report);
         if (report && (threadIdx.x & 31) < kRunBlocks)
-            atomicOr(cluster.map_shared_rank(&sh.flags[slot], threadIdx.x & 31), report);
+            atomicOr(cluster.map_shared_rank(&flags[slot], threadIdx.x & 31), report);
         cluster_arrive();
         nerr = 0;
         if (active && done + 1 < a.n_steps)
             load_noise_f(nz, p.seed, a.n, tag, tag, t + 1, xf, nerr);
         cluster_wait();
-        report = *(volatile uint32_t*)&sh.flags[slot];
+        report = *(volatile uint32_t*)&flags[slot];
         if (report & kRunError) break;   // the state stays that of the failing step
         s = v;
         ++done;
         if (report & kRunMoved) {
             ++builds;
-            uint32_t berr = 0;
-            run_rebuild(a, g, t + 1, f, active, sh, cluster, s, tag, m, berr);
-            if (berr) atomicOr(a.err, berr);
-            cluster_barrier();
-            const uint32_t bad = *(volatile const uint32_t*)a.err;
-            cluster_barrier();   // all have read it before a step may write it
-            if (bad) break;
+            if (!run_rebuild(a, g, t + 1, f, active, smem, cluster, s, tag, m)) break;
             if (active) {
                 lb = a.lbuild[f];
                 hal = a.lhalo[f];
@@ -272,11 +232,13 @@ cudaError_t launch(const Body& body, const DevGeom& g, const RunArgs& a, const V
     auto* kernel = run_list_kernel<Body>;
     cudaError_t e =
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOrderSmem);
     if (e != cudaSuccess) return e;
-    const int threads = ((a.n + kRunBlocks - 1) / kRunBlocks + 31) / 32 * 32;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(kRunBlocks);
-    cfg.blockDim = dim3(clusters ? kRunThreads : threads);
+    cfg.blockDim = dim3(((a.n + kRunBlocks - 1) / kRunBlocks + 31) / 32 * 32);
+    cfg.dynamicSmemBytes = order_smem(a.n, a.order.ncell);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -300,11 +262,13 @@ cudaError_t dispatch(const ForceSetup& fs, const DevGeom& g, const RunArgs& a, c
 }  // namespace
 
 bool run_list_fits(const ForceSetup& fs, int n, int ncell) {
-    if (n < 1 || n > kRunMaxN || ncell > kRunMaxCells) return false;
+    if (n < 1 || n > kRunMaxN || !order_fits(n, ncell)) return false;
     // the device holds a cluster of this kernel's blocks
     int clusters = 0;
-    if (dispatch(fs, DevGeom{}, RunArgs{}, VgbParams{}, NoiseView{}, nullptr, &clusters) !=
-        cudaSuccess) {
+    RunArgs a{};
+    a.n = n;
+    a.order.ncell = ncell;
+    if (dispatch(fs, DevGeom{}, a, VgbParams{}, NoiseView{}, nullptr, &clusters) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -356,10 +356,10 @@ __device__ __forceinline__ void vgb_system_one(const VgbSystemArgs& a, const Vgb
         *a.lflag_clear = 0;
         *a.lhcount = 0;   // halo records are handed out afresh at the next build
     }
-    if (a.count) {   // the next cell list (not when it is rebuilt only with the pair list)
+    if (a.key) {   // the next cell list (not when it is rebuilt only with the pair list)
         const int key = hash_pos(xn, g, err);
         a.key[f] = key;
-        a.rank[f] = atomicAdd(&a.count[key], 1);
+        if (a.count) a.rank[f] = atomicAdd(&a.count[key], 1);   // (order_kernel counts itself)
     }
     if (err) atomicOr(a.err, err);
 }

@@ -50,10 +50,11 @@ def both(psim, n, box, scale, force, steps, vel_freq, noise=None):
 
 
 # one particle; one warp a block and one more; the most it takes and one more; the
-# most cells it takes (64000 of 65536) and more (41^3); three cells a side
+# most cells it takes with 700 particles and more (38^3, 39^3); three cells a side
 @pytest.mark.parametrize("n,box,scale", [(1, 9.0, 5), (33, 9.0, 5), (512, 14.0, 9), (513, 14.0, 9),
                                          (4097, 28.0, 18), (8192, 34.0, 22), (8193, 34.0, 22),
-                                         (700, 64.0, 40), (700, 65.6, 41), (64, 7.0, 3)])
+                                         (700, 64.0, 40), (700, 65.6, 41), (700, 60.8, 38),
+                                         (700, 62.4, 39), (64, 7.0, 3)])
 @pytest.mark.parametrize("vel_freq", [1, 25, 1000])
 def test_same_bits(psim, n, box, scale, vel_freq):
     builds, at = both(psim, n, box, scale, psim.make_force("AO", 1.2, kT=1.0, well_depth=0.3),
