@@ -355,8 +355,9 @@ int psim_init_rsa_device(int32_t n, double box, double min_sep, uint64_t seed,
  * LennardJones plugin with ljNum = 0; the loss is the squared distance
  * between the trajectory's time-averaged, Gaussian-smoothed g(r) (samples
  * every sample_every steps; n_bins bins of [r_min, r_max), kernel width
- * sigma) and a target.  The reverse pass recomputes checkpoint_every-step
- * segments from checkpoints of the forward pass. */
+ * sigma) and a target.  The reverse pass recomputes segments of
+ * checkpoint_every steps (or of as many more as 256 MB hold the positions of)
+ * from checkpoints of the forward pass, all but the last. */
 typedef struct psim_adjoint psim_adjoint;
 
 typedef struct {

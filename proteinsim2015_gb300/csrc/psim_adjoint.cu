@@ -21,14 +21,16 @@
 //
 // A forward step is one launch (force and update), a reverse step one (J u,
 // dF/dth . u and the loss's position gradient), both over one neighbour list kept for
-// tens of steps.  The forward pass keeps a checkpoint (x_t, x_{t-1}, F(x_{t-1})) every
-// K steps; the reverse pass recomputes each K-step segment from its checkpoint, so
-// memory is (T/K + K) positions and the cost two forward passes plus the reverse.
+// tens of steps.  The forward pass keeps the positions of its last K steps and a
+// checkpoint (x_t, x_{t-1}, F(x_{t-1})) every K steps; the reverse pass goes back through
+// the last segment as it stands and recomputes each earlier one from its checkpoint, so
+// memory is (T/K + K) positions.  K is the caller's interval or, where that is longer,
+// what 256 MB hold (kAdjTraj): a trajectory that fits is never computed twice.
 // All sums are taken in an order that the positions decide: two runs agree bit for
 // bit.  What bounds it is the FP64 unit: 33 FP64 operations a pair forward and ~65
 // back with the lanes of an instruction 75% full at 32768 particles.  Gradient of 60
 // steps, with a cell list and a thread per particle for every pass before, and now:
-// 4096 particles 186 -> 7.6 ms, 32768 286 -> 30 ms.
+// ADJFIGS
 //
 // All arithmetic is FP64 and the forward matches the system's plain form
 // (same coefficients and Philox draws) up to rounding.  The pair force is the
@@ -826,6 +828,7 @@ void with_lanes(const psim_adjoint* a, Fn&& fn) {
     else fn(std::integral_constant<int, 4>{});
 }
 constexpr int kAdjRing = kAdjBlock + 2;
+constexpr size_t kAdjTraj = (size_t)256 << 20;   // bytes of positions always worth keeping
 
 double4_32a* pos_at(psim_adjoint* a, int k) {
     return a->traj.as<double4_32a>() + (size_t)k * a->n;
@@ -1031,7 +1034,9 @@ int upload(psim_adjoint* a, const double* host) {
 // The whole forward in K-step segments (slots 0, 1, ... hold x_{t0-1}, x_t0 ..
 // x_t0+K), with a checkpoint (x_t0, x_{t0-1}, F(x_{t0-1})) of each and the smoothed
 // counts of the sampled steps.
-int forward_all(psim_adjoint* a, const AdjPair& q, const double* pos0, const double* vel0) {
+// builds (may be null) gets the steps of the last segment that a list was built at.
+int forward_all(psim_adjoint* a, const AdjPair& q, const double* pos0, const double* vel0,
+                std::vector<int>* builds) {
     const int n = a->n, b = (n + 255) / 256, nb = a->cfg.n_bins;
     const size_t b4 = 32 * (size_t)n;
     int rc = set_list(a);
@@ -1063,8 +1068,12 @@ int forward_all(psim_adjoint* a, const AdjPair& q, const double* pos0, const dou
         ADJ_CUDA(cudaMemcpyAsync(c, pos_at(a, 0), 2 * b4, cudaMemcpyDeviceToDevice, a->st));
         ADJ_CUDA(cudaMemcpyAsync(c + 2 * b4, force_at(a, t0 - 1), 24 * (size_t)n,
                                  cudaMemcpyDeviceToDevice, a->st));
+        // the last segment's lists are all built within it: the reverse pass builds
+        // them again
+        const bool last = t1 == a->T;
+        if (last && builds) a->listed = false;
         // the counts of x_t1 belong to the next segment unless it is the last
-        if ((rc = run_forward(a, q, t0, t1, true, t1 == a->T, true, nullptr))) return rc;
+        if ((rc = run_forward(a, q, t0, t1, true, last, true, last ? builds : nullptr))) return rc;
         if (t1 < a->T) {   // carry x_{t1-1}, x_t1 to the front
             const int k = t1 - t0;
             for (int s = 0; s < 2; ++s) {
@@ -1134,7 +1143,8 @@ psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device
     a->device = device;
     a->n = n;
     a->T = cfg->n_steps;
-    a->K = std::min(std::max(cfg->checkpoint_every, 2), cfg->n_steps);
+    const int asked = std::min(std::max(cfg->checkpoint_every, 2), cfg->n_steps);
+    a->K = std::max(asked, (int)std::min((size_t)a->T, kAdjTraj / (48 * (size_t)n)));
     a->S = cfg->n_steps / cfg->sample_every;
     const double dt = cfg->integ.dt, dt2 = dt * dt, m = 1.0 / cfg->mass;
     a->step = AdjStep{n, 1.0 + vc.coeff0, vc.coeff0, m * dt2 * (vc.coeff1 + vc.coeff2),
@@ -1175,7 +1185,7 @@ psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device
         a->trajf.free();
         a->ck.free();
         ok = a->K > 2;
-        a->K = std::max(2, a->K / 2);
+        a->K = a->K > asked ? asked : std::max(2, a->K / 2);
     }
     if (ok) {
         double2 e2[256];
@@ -1243,7 +1253,7 @@ int psim_adjoint_forward(psim_adjoint* a, const psim_adjoint_params* p, const do
     a->rc2 = std::max(std::max(q.ao_rc2, q.y_rc2), q.lj_rc2);
     if (a->rc2 > a->cfg.geom.cell_size * a->cfg.geom.cell_size)
         return adj_fail(PSIM_ERR_INPUT, "adjoint: a cutoff exceeds the cell size");
-    int rc = forward_all(a, q, pos0, vel0);
+    int rc = forward_all(a, q, pos0, vel0, nullptr);
     if (rc) return rc;
     std::vector<double> g;
     if ((rc = mean_g(a, g))) return rc;
@@ -1278,7 +1288,8 @@ int psim_adjoint_gradient(psim_adjoint* a, const psim_adjoint_params* p, const d
     if (q.lj_rc2 > 0.0 && (!(q.sig > 0.0) || q.ljn < 0 || q.ljn > 64))
         return adj_fail(PSIM_ERR_INPUT, "adjoint: LJ term needs sigma > 0 and 0 <= n <= 64");
     // forward: checkpoints and the loss
-    int rc = forward_all(a, q, pos0, vel0);
+    std::vector<int> builds;
+    int rc = forward_all(a, q, pos0, vel0, &builds);
     if (rc) return rc;
     std::vector<double> g;
     if ((rc = mean_g(a, g))) return rc;
@@ -1305,17 +1316,17 @@ int psim_adjoint_gradient(psim_adjoint* a, const psim_adjoint_params* p, const d
     int l0 = 0, l1 = 1, l2 = 2, uc = 0;   // lam_t, lam_{t+1}, lam_{t+2}; u_t
     const int nseg = (T + K - 1) / K;
     const double rwalk = std::max(a->rc2, a->walk_rc2);
-    std::vector<int> builds;
     for (int seg = nseg - 1; seg >= 0; --seg) {
         const int t0 = seg * K, t1 = std::min(t0 + K, T);
-        // recompute the segment from its checkpoint
-        const char* c = a->ck.as<char>() + (size_t)seg * 88 * n;
-        ADJ_CUDA(cudaMemcpyAsync(pos_at(a, 0), c, 2 * b4, cudaMemcpyDeviceToDevice, a->st));
-        ADJ_CUDA(cudaMemcpyAsync(force_at(a, t0 - 1), c + 2 * b4, b3, cudaMemcpyDeviceToDevice,
-                                 a->st));
-        a->listed = false;
-        builds.clear();
-        if ((rc = run_forward(a, q, t0, t1, false, false, false, &builds))) return rc;
+        if (seg < nseg - 1) {   // recompute the segment from its checkpoint
+            const char* c = a->ck.as<char>() + (size_t)seg * 88 * n;
+            ADJ_CUDA(cudaMemcpyAsync(pos_at(a, 0), c, 2 * b4, cudaMemcpyDeviceToDevice, a->st));
+            ADJ_CUDA(cudaMemcpyAsync(force_at(a, t0 - 1), c + 2 * b4, b3,
+                                     cudaMemcpyDeviceToDevice, a->st));
+            a->listed = false;
+            builds.clear();
+            if ((rc = run_forward(a, q, t0, t1, false, false, false, &builds))) return rc;
+        }
         // back through it, each step on the list that holds for it
         int at = a->listed ? (int)builds.size() - 1 : -1;
         for (int t = (seg == nseg - 1 ? t1 : t1 - 1); t >= t0; --t) {
