@@ -7,6 +7,7 @@ Translation units are compiled in parallel with one -gencode each:
   psim_step.cu   the mixed form's list step as one kernel (as psim_mixed.cu)
   psim_run.cu    the mixed form's list steps of a small system in one kernel
   psim_list_build.cu  the pair list's build
+  psim_rebuild.cu  the end of a step with a pair list and its rebuild
   psim_cells.cu  integer counting sort and layout conversions
   psim_api.cu    host side of the C ABI
   psim_noalloc.cu  the cell-list build on a static device scratch array
@@ -32,6 +33,7 @@ SOURCES = {
     "psim_step.cu": [],
     "psim_list_build.cu": [],
     "psim_run.cu": [],
+    "psim_rebuild.cu": [],
     "psim_cells.cu": [],
     "psim_api.cu": [],
     "psim_noalloc.cu": [],

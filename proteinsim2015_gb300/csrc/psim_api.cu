@@ -50,6 +50,7 @@ int code_from_bits(uint32_t bits) {
     if (bits & EBIT_NAN) return PSIM_ERR_NAN_FORCE;
     if (bits & EBIT_BOUNDS) return PSIM_ERR_PARTICLE_BOUNDS;
     if (bits & EBIT_CELL) return PSIM_ERR_CELL_BOUNDS;
+    if (bits & EBIT_WAIT) return PSIM_ERR_CUDA;
     if (bits & (EBIT_NOISE | EBIT_INDEX | EBIT_LIST)) return PSIM_ERR_INPUT;
     return PSIM_OK;
 }
@@ -59,6 +60,7 @@ const char* bits_text(uint32_t bits) {
     if (bits & EBIT_NAN) return "non-finite force";
     if (bits & EBIT_BOUNDS) return "particle out of bounds after the periodic wrap";
     if (bits & EBIT_CELL) return "particle hashed outside the cell grid";
+    if (bits & EBIT_WAIT) return "a barrier inside a kernel gave up";
     if (bits & EBIT_NOISE) return "injected noise does not cover the step";
     if (bits & EBIT_INDEX) return "an index or cell range in the input is out of bounds";
     if (bits & EBIT_LIST)
@@ -877,7 +879,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
                                       w.lpos.as<float4>(), w.lhalo.as<int>(),
                                       w.lhcount.as<int>(), z.hcap, z.hr, g,
                                       w.err.as<uint32_t>(), st, compact ? 1.0f / unit : 0.f));
-        ListBuild lb{w.list.as<uint32_t>(), w.lcount.as<int>(), g.n, z.cap, z.pre, nullptr,
+        ListBuild lb{w.list.as<uint32_t>(), w.lcount.as<int>(), g.n, z.cap, z.pre,
                      w.lhalo.as<int>(), g.n};
         PSIM_CUDA(launch_list_build(g, cv, lb, w.err.as<uint32_t>(), st));
         PSIM_CUDA(cudaMemcpyAsync(&bits, w.err.p, 4, cudaMemcpyDeviceToHost, st));
@@ -1215,7 +1217,7 @@ struct psim_system {
     // per-slot arrays live in buffer 0 (buffer 1 receives a new order or the
     // cell view of the current positions that refresh_cells computes).
     DevBuf pscratch;
-    cudaGraphConditionalHandle cond = 0;   // the rebuild's conditional node (graph capture)
+    DevBuf rebuild;                        // the rebuild kernel's barrier counter and sums
     // compact 16-byte records when every particle has one radius (set by the upload)
     int lcompact = 0;
     float lradius = 0.f, lunit = 0.f;
@@ -1294,8 +1296,8 @@ CellView list_cells(psim_system* s, int cb) {
     return CellView{nullptr, s->posh.as<float4>(), s->posl.as<float4>(), s->cellid.as<int>(),
                     s->start.as<int>(), s->count[cb].as<int>()};
 }
-ListBuild list_build(psim_system* s, const int* gate) {
-    ListBuild lb{s->list.as<uint32_t>(), s->lcount.as<int>(), s->n, s->lcap, s->lpre, gate,
+ListBuild list_build(psim_system* s) {
+    ListBuild lb{s->list.as<uint32_t>(), s->lcount.as<int>(), s->n, s->lcap, s->lpre,
                  s->lhalo.as<int>(), s->n};
     lb.xsorted = 1;   // the order set_halo_args asks the canonicalisation for
     if (s->n_reps) {   // each replica's own grid and list radius
@@ -1306,10 +1308,9 @@ ListBuild list_build(psim_system* s, const int* gate) {
     return lb;
 }
 
-// The pair-list build on the cell order just made (count buffer cb), run
-// only when *gate != 0.
-cudaError_t enqueue_list_build(psim_system* s, int cb, const int* gate) {
-    return launch_list_build(s->g, list_cells(s, cb), list_build(s, gate), s->err.as<uint32_t>(),
+// The pair-list build on the cell order just made (count buffer cb).
+cudaError_t enqueue_list_build(psim_system* s, int cb) {
+    return launch_list_build(s->g, list_cells(s, cb), list_build(s), s->err.as<uint32_t>(),
                              s->st);
 }
 
@@ -1355,12 +1356,12 @@ cudaError_t enqueue_force(psim_system* s, const Phase& ph, const ForceOut& fo) {
 
 // ---- the step with a pair list: the cell list is rebuilt with the list only
 //
-// force (list) -> vGB (no permutation, no hash) -> step end, then, on the
-// steps whose integrator raised the rebuild flag, the rebuild: hash + count,
+// force (list) -> vGB (no permutation, no hash) -> step end, which on the steps
+// whose integrator raised the rebuild flag is also the rebuild: hash + count,
 // scan, scatter, canonicalisation into the new cell order (list records and
 // halo images included), the state carried into that order, the list build.
-// In a graph the rebuild is the body of a conditional node that the step end
-// sets; so a step without a rebuild launches three kernels.  The forces and
+// So a step launches three kernels, or two where one does the first two's work
+// (psim_step.cu).  The forces and
 // the trajectory are those of the cell list rebuilt every step: the same
 // pair terms in the same list order, the same per-particle arithmetic.
 
@@ -1390,55 +1391,45 @@ CanonArgs canon_args(psim_system* s, int q) {
     return ca;
 }
 
-// The rebuild after step t (phase of t): the state the integrator wrote (in
-// the storage order) sorted into the new cell order.
-int enqueue_rebuild_lazy(psim_system* s, long long t) {
+// The end of step t (phase of t): the step state, and the rebuild on the state the
+// integrator wrote (in the storage order) where the step asked for one.
+int enqueue_step_rebuild(psim_system* s, long long t) {
     const Phase ph = phase_of(t);
-    const int n = s->n, nsb = 1 - ph.sb;
-    cudaStream_t st = s->st;
-    uint32_t* err = s->err.as<uint32_t>();
-    const CanonArgs ca = canon_args(s, nsb);
-    PSIM_CUDA(cudaMemsetAsync(s->count[0].p, 0, 4 * (size_t)s->ncell, st));
-    PSIM_CUDA(launch_hash_count(n, ca.x, ca.y, ca.z, s->g, s->key.as<int>(), s->rank.as<int>(),
-                                s->count[0].as<int>(), err, st,
-                                s->n_reps ? s->b_rep.as<int>() : nullptr,
-                                s->n_reps ? s->b_geoms.as<DevGeom>() : nullptr));
-    PSIM_CUDA(launch_scan(s->count[0].as<int>(), s->start.as<int>(), s->ncell,
-                          s->scratch.as<int>(), st));
-    PSIM_CUDA(launch_scatter(n, s->key.as<int>(), s->rank.as<int>(), s->start.as<int>(),
-                             s->tmp.as<int>(), err, st));
-    PSIM_CUDA(launch_canonicalize(ca, st));
-    // the state into the new order: positions, previous positions, noise
-    // memory, and the forces of this step and the one before
+    const int nsb = 1 - ph.sb;
+    RebuildArgs a{};
+    a.n = s->n;
+    a.ncell = s->ncell;
+    a.vel_freq = s->vp.vel_freq;
+    a.state = s->state.as<StepState>();
+    a.lflag = s->lflag.as<int>() + (t & 1);
+    a.err = s->err.as<uint32_t>();
+    a.counter = s->rebuild.as<unsigned long long>();
+    a.next = s->rebuild.as<int>() + 2;
+    a.sums = s->rebuild.as<int>() + 4;
+    a.key = s->key.as<int>();
+    a.rank = s->rank.as<int>();
+    a.count = s->count[0].as<int>();
+    a.start = s->start.as<int>();
+    a.tmp = s->tmp.as<int>();
+    a.canon = canon_args(s, nsb);
     DevBuf* arrs[5] = {&s->pos[nsb], &s->pos0[nsb], &s->mem[nsb], &s->frc[ph.fcur],
                        &s->frc[ph.fprev]};
-    PermuteArgs pa{};
-    pa.n = n;
-    pa.perm = s->perm[0].as<int>();
-    pa.narr = 15;
-    double* scr = s->pscratch.as<double>();
-    for (int a = 0; a < 5; ++a)
-        for (int k = 0; k < 3; ++k) {
-            pa.src[3 * a + k] = d3(*arrs[a], n, k);
-            pa.dst[3 * a + k] = scr + (size_t)(3 * a + k) * n;
-        }
-    PSIM_CUDA(launch_permute(pa, err, st));
-    for (int a = 0; a < 5; ++a)
-        PSIM_CUDA(cudaMemcpyAsync(arrs[a]->p, scr + (size_t)3 * a * n, 24 * (size_t)n,
-                                  cudaMemcpyDeviceToDevice, st));
-    PSIM_CUDA(cudaMemcpyAsync(s->tag[0].p, s->tag[1].p, 4 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-    PSIM_CUDA(cudaMemcpyAsync(s->radius[0].p, s->radius[1].p, 8 * (size_t)n,
-                              cudaMemcpyDeviceToDevice, st));
-    PSIM_CUDA(cudaMemcpyAsync(s->inv_mass[0].p, s->inv_mass[1].p, 8 * (size_t)n,
-                              cudaMemcpyDeviceToDevice, st));
-    PSIM_CUDA(enqueue_list_build(s, 0, nullptr));
+    for (int k = 0; k < 5; ++k) a.arr[k] = arrs[k]->as<double>();
+    a.scratch = s->pscratch.as<double>();
+    for (int k = 0; k < 2; ++k) {
+        a.tag[k] = s->tag[k].as<int>();
+        a.radius[k] = s->radius[k].as<double>();
+        a.inv_mass[k] = s->inv_mass[k].as<double>();
+    }
+    a.cv = list_cells(s, 0);
+    a.lb = list_build(s);
+    PSIM_CUDA(launch_step_rebuild(a, s->g, s->st));
     return PSIM_OK;
 }
 
 // Step t with a pair list.  In a graph (evs null) this enqueues the force
-// pass and the integrator (or, fused, the one kernel of both) and the step end;
-// the caller adds the conditional rebuild.  Timed directly (evs: 4 events), the
-// rebuild decision is read back.
+// pass and the integrator (or, fused, the one kernel of both) and the step end
+// with its rebuild; evs: 4 events around the phases.
 int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs, bool fused = false) {
     const Phase ph = phase_of(t);
     const int n = s->n, sb = ph.sb, nsb = 1 - ph.sb;
@@ -1489,25 +1480,13 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs, bool fused 
     else
         PSIM_CUDA(launch_vgb_system_fast(a, s->vp, s->g, nz, st));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[2], st));
-    PSIM_CUDA(launch_step_end(s->state.as<StepState>(), lflag, s->err.as<uint32_t>(),
-                              s->vp.vel_freq, s->cond, evs ? 0 : 1, st));
-    if (evs) {
-        int flag = 0;
-        uint32_t bits = 0;
-        PSIM_CUDA(cudaMemcpyAsync(&flag, lflag, 4, cudaMemcpyDeviceToHost, st));
-        PSIM_CUDA(cudaMemcpyAsync(&bits, s->err.p, 4, cudaMemcpyDeviceToHost, st));
-        PSIM_CUDA(cudaStreamSynchronize(st));
-        if (flag && !bits) {
-            const int rc = enqueue_rebuild_lazy(s, t);
-            if (rc) return rc;
-        }
-        PSIM_CUDA(cudaEventRecord(evs[3], st));
-    }
+    if (int rc = enqueue_step_rebuild(s, t)) return rc;
+    if (evs) PSIM_CUDA(cudaEventRecord(evs[3], st));
     return PSIM_OK;
 }
 
-int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
-    if (s->list_on) return enqueue_step_lazy(s, t, evs);
+int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs, bool fused = false) {
+    if (s->list_on) return enqueue_step_lazy(s, t, evs, fused);
     const Phase ph = phase_of(t);
     const int n = s->n;
     cudaStream_t st = s->st;
@@ -1591,88 +1570,12 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs) {
     return PSIM_OK;
 }
 
-// The step graph with a pair list: the step, then a conditional node (set by
-// the step end) whose body is the rebuild.
-// Steps phase .. phase + steps - 1 with a pair list, captured into one graph:
-// each step's kernels followed by a conditional node whose body is that
-// step's rebuild (the step end sets the node's condition).
-int graph_lazy_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_t* out) {
-    cudaGraph_t g = nullptr;
-    PSIM_CUDA(cudaGraphCreate(&g, 0));
-    auto done = [&](int rc) {
-        if (g) cudaGraphDestroy(g);
-        return rc;
-    };
-    // a condition handle per conditional node: the step end that sets it is
-    // captured with s->cond holding that step's handle
-    std::vector<cudaGraphConditionalHandle> conds(steps);
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < steps && e == cudaSuccess; ++k)
-        e = cudaGraphConditionalHandleCreate(&conds[k], g, 0, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess)
-        return done(fail(PSIM_ERR_CUDA, "conditional handle: %s", cudaGetErrorString(e)));
-    std::vector<cudaGraph_t> bodies;
-    e = cudaStreamBeginCaptureToGraph(s->st, g, nullptr, nullptr, 0,
-                                      cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return done(fail(PSIM_ERR_CUDA, "capture: %s", cudaGetErrorString(e)));
-    int rc = PSIM_OK;
-    for (int k = 0; k < steps && !rc; ++k) {
-        s->cond = conds[k];
-        rc = enqueue_step_lazy(s, phase + k, nullptr, fused);
-        if (rc) break;
-        cudaStreamCaptureStatus cs;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t nd = 0;
-        cudaGraph_t cg = nullptr;
-        e = cudaStreamGetCaptureInfo(s->st, &cs, nullptr, &cg, &deps, nullptr, &nd);
-        cudaGraphNode_t cn = nullptr;
-        cudaGraphNodeParams cp{};
-        if (e == cudaSuccess) {
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = s->cond;
-            cp.conditional.type = cudaGraphCondTypeIf;
-            cp.conditional.size = 1;
-            std::vector<cudaGraphNode_t> dv(deps, deps + nd);
-            e = cudaGraphAddNode(&cn, cg, dv.data(), nullptr, dv.size(), &cp);
-        }
-        if (e == cudaSuccess)
-            e = cudaStreamUpdateCaptureDependencies(s->st, &cn, nullptr, 1,
-                                                    cudaStreamSetCaptureDependencies);
-        if (e != cudaSuccess)
-            rc = fail(PSIM_ERR_CUDA, "conditional node: %s", cudaGetErrorString(e));
-        else
-            bodies.push_back(cp.conditional.phGraph_out[0]);
-    }
-    cudaGraph_t captured = g;
-    e = cudaStreamEndCapture(s->st, &captured);
-    if (rc) return done(rc);
-    if (e != cudaSuccess) return done(fail(PSIM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e)));
-    // the bodies: each step's rebuild, captured into its node's own graph
-    for (int k = 0; k < steps; ++k) {
-        cudaGraph_t body = bodies[k];
-        e = cudaStreamBeginCaptureToGraph(s->st, body, nullptr, nullptr, 0,
-                                          cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return done(fail(PSIM_ERR_CUDA, "capture: %s", cudaGetErrorString(e)));
-        rc = enqueue_rebuild_lazy(s, phase + k);
-        cudaGraph_t bcap = body;
-        e = cudaStreamEndCapture(s->st, &bcap);
-        if (rc) return done(rc);
-        if (e != cudaSuccess)
-            return done(fail(PSIM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e)));
-    }
-    e = cudaGraphInstantiate(out, g, 0);
-    if (e != cudaSuccess)
-        return done(fail(PSIM_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e)));
-    return done(PSIM_OK);
-}
-
 // Steps phase .. phase + steps - 1, captured into one graph.
 int graph_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_t* out) {
-    if (s->list_on) return graph_lazy_steps(s, phase, steps, fused, out);
     cudaGraph_t g = nullptr;
     PSIM_CUDA(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSIM_OK;
-    for (int k = 0; k < steps && !rc; ++k) rc = enqueue_step(s, phase + k, nullptr);
+    for (int k = 0; k < steps && !rc; ++k) rc = enqueue_step(s, phase + k, nullptr, fused);
     cudaError_t e = cudaStreamEndCapture(s->st, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (e != cudaSuccess) return fail(PSIM_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
@@ -1700,11 +1603,13 @@ void drop_graphs(psim_system* s) {
     drop(s->graph_multi);
 }
 
-constexpr int kRunSteps = 1024;   // of one such launch
+constexpr int kRunSteps = 1024, kRunLeast = 4;   // of one such launch
 
 // Whether stretches of its normal steps run in the one kernel of psim_run.cu: up to the
-// sizes its cluster holds, where it takes 5.6 to 8.5 us a step of the AO colloids and a
-// graph of single steps 17.4 (the LJ liquid of 6912: 19.3 against 27.7), so wherever it can.
+// sizes its cluster holds, where it takes 5.5 to 8.3 us a step of the AO colloids and a
+// graph of single steps 8.4 to 9.5 (the LJ liquid of 6912: 19.3 against 19.6).  A stretch
+// of kRunLeast steps at least: alone a step of 4000 takes 15.4 against 13.7, of 8192 18.7
+// against 14.0.
 bool small_system(psim_system* s) {
     if (!fused_steps(s) || s->n_reps) return false;
     if (s->small < 0) s->small = run_list_fits(s->fs, s->n, s->ncell) ? 1 : 0;
@@ -1728,9 +1633,11 @@ int each_launch(psim_system* s, int n_steps, Visit&& visit) {
             // up to the next velocity step, and a few milliseconds at most
             const long long period = s->vp.vel_freq + 1LL, to = (t / period + 1) * period;
             const int steps = (int)std::min({to - t, end - t, (long long)kRunSteps});
-            rc = visit(nullptr, phase, steps, true);
-            t += steps;
-            continue;
+            if (steps >= kRunLeast) {
+                rc = visit(nullptr, phase, steps, true);
+                t += steps;
+                continue;
+            }
         }
         bool run = !small && multi && t % 6 == 0 && end - t >= kGraphSteps;
         for (int k = 0; run && !one_kind && k < kGraphSteps; ++k) run = normal_step(s, t + k);
@@ -1746,11 +1653,6 @@ int each_launch(psim_system* s, int n_steps, Visit&& visit) {
 // steps normal steps from step s->total on in one kernel
 int enqueue_run(psim_system* s, int steps) {
     const int n = s->n;
-    // a step is not captured by a caller (its stream is handed out): the number of steps
-    // and the phase of the state would be frozen into the launch
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    PSIM_CUDA(cudaStreamIsCapturing(s->st, &capture));
-    if (capture != cudaStreamCaptureStatusNone) PSIM_CUDA(cudaErrorStreamCaptureUnsupported);
     RunArgs a{};
     a.n = n;
     a.ncell = s->ncell;
@@ -1771,7 +1673,7 @@ int enqueue_run(psim_system* s, int steps) {
     a.key = s->key.as<int>();
     a.order = order_args(s, 0);
     a.cv = list_cells(s, 0);
-    a.lb = list_build(s, nullptr);
+    a.lb = list_build(s);
     a.pl = pair_list(s, phase_of(s->total));
     a.linv_unit = 1.0f / s->lunit;
     a.ldisp2 = s->ldisp2;
@@ -2162,6 +2064,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
              !s->list.ensure(4 * n * (size_t)(s->lcap + kListFold)) && !s->lcount.ensure(4 * n) &&
              !s->lflag.ensure(8) && !s->lhalo.ensure(4 * n) && !s->lhcount.ensure(4) &&
              !s->pscratch.ensure(15 * 8 * (size_t)n) &&
+             !s->rebuild.ensure(16 + 4 * (size_t)rebuild_sums()) &&
              cudaMemset(s->lflag.p, 0, 8) == cudaSuccess &&
              cudaMemset(s->lhcount.p, 0, 4) == cudaSuccess;
     }
@@ -2219,7 +2122,7 @@ void psim_system_destroy(psim_system* s) {
     DevBuf* arrs[] = {&s->cellid, &s->key, &s->rank, &s->tmp, &s->start, &s->scratch, &s->posd,
                       &s->posh, &s->posl, &s->vel, &s->err, &s->state, &s->occ, &s->noise,
                       &s->snap, &s->lslot[0], &s->lslot[1], &s->lbuild, &s->lpos[0], &s->lpos[1], &s->list,
-                      &s->lcount, &s->lflag, &s->lhalo, &s->lhcount, &s->pscratch, &s->b_tasks,
+                      &s->lcount, &s->lflag, &s->lhalo, &s->lhcount, &s->pscratch, &s->rebuild, &s->b_tasks,
                       &s->b_geoms, &s->b_pairs, &s->b_pre, &s->b_rep, &s->b_seeds,
                       &s->img, &s->track_start, &s->b_lpre, &s->b_hr, &s->obs};
     for (DevBuf* b : arrs) b->release();
@@ -2333,6 +2236,7 @@ int psim_system_upload(psim_system* s, const double* pos, const double* pos0, co
         // the first list, on the first cell order (the list slots are the
         // storage slots: the state is carried into that order below)
         PSIM_CUDA(cudaMemsetAsync(s->lflag.p, 0, 8, st));
+        PSIM_CUDA(cudaMemsetAsync(s->rebuild.p, 0, 8, st));
         set_halo_args(s, ca, 0);
         PSIM_CUDA(cudaMemsetAsync(s->lhcount.p, 0, 4, st));
     }
@@ -2355,7 +2259,7 @@ int psim_system_upload(psim_system* s, const double* pos, const double* pos0, co
         for (int a = 0; a < 5; ++a)
             PSIM_CUDA(cudaMemcpyAsync(arrs[a]->p, scr + (size_t)3 * a * n, 24 * (size_t)n,
                                       cudaMemcpyDeviceToDevice, st));
-        PSIM_CUDA(enqueue_list_build(s, ph.cb, nullptr));
+        PSIM_CUDA(enqueue_list_build(s, ph.cb));
     }
     uint32_t bits = 0;
     PSIM_CUDA(cudaMemcpyAsync(&bits, s->err.p, 4, cudaMemcpyDeviceToHost, st));
@@ -2394,6 +2298,11 @@ int psim_system_step_async(psim_system* s, int32_t n_steps) {
     if (s->latched) return fail(code_from_bits(s->latched), "%s", bits_text(s->latched));
     if (n_steps < 0) return fail(PSIM_ERR_INPUT, "negative step count");
     DeviceGuard dg(s->device);
+    if (s->list_on) {   // not in a caller's capture (the stream is handed out)
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        PSIM_CUDA(cudaStreamIsCapturing(s->st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) PSIM_CUDA(cudaErrorStreamCaptureUnsupported);
+    }
     if (int rc = capture_graphs(s, n_steps)) return rc;   // before anything is in flight
     return each_launch(s, n_steps, [&](cudaGraphExec_t* g, int, int steps, bool) {
         if (g) {
@@ -2894,23 +2803,18 @@ int psim_system_profile(psim_system* s, int32_t n_steps, double* out_ms) {
 }
 
 int psim_system_launches_per_step(psim_system* s) {
-    // force, vGB, scan x3, scatter, canonicalise (+1 memset node), or force, vGB and
-    // the one kernel of a small system's cell order; with a pair list: force, vGB (one kernel on normal steps where fused_steps
-    // allows), step end (the rebuild's kernels run on the steps that rebuild:
-    // psim_system_launches_per_rebuild); a small system's normal step alone, or a
-    // stretch of them, is one kernel with its rebuilds
+    // force, vGB, scan x3, scatter, canonicalise (+1 memset node), or force, vGB and the
+    // one kernel of a small system's cell order; with a pair list: force, vGB (one kernel
+    // on normal steps where fused_steps allows), the step end with its rebuild; a small
+    // system's normal step alone, or a stretch of them, is one kernel
     if (!s) return 7;
     if (!s->list_on) return one_order(s) ? 3 : 7;
     DeviceGuard dg(s->device);
     return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
 }
 
-int psim_system_launches_per_rebuild(psim_system* s) {
-    // hash + count, scan x3, scatter, canonicalise, state permutation, list
-    // build (+ memset and copy nodes)
-    if (!s || !s->list_on) return 0;
-    DeviceGuard dg(s->device);
-    return small_system(s) ? 0 : 8;
+int psim_system_launches_per_rebuild(psim_system*) {
+    return 0;   // part of the step's last kernel
 }
 
 int psim_system_cell_occupancy(psim_system* s, int32_t* max_occ, double* mean_occ) {

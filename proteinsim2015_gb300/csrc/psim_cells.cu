@@ -131,7 +131,8 @@ __global__ void __launch_bounds__(256) canonicalize_kernel(CanonArgs a, int vel_
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.err && *a.err) return;
     if (p < a.n) canon_slot(a, p);
-    if (a.state && a.advance && p == 0) step_advance(a, vel_freq);
+    if (a.state && a.advance && p == 0)
+        step_advance(a.state, vel_freq, a.rebuild && *a.rebuild);
 }
 
 cudaError_t launch_canonicalize(const CanonArgs& a, cudaStream_t st) {
@@ -154,7 +155,8 @@ order_kernel(OrderArgs o, CanonArgs c, int vel_freq) {
     const int fs = (c.n + blocks - 1) / blocks, cs = (o.ncell + blocks - 1) / blocks;
     const bool ok = block_order(o, c, min(c.n, b * fs), min(c.n, (b + 1) * fs),
                                 min(o.ncell, b * cs), min(o.ncell, (b + 1) * cs), smem);
-    if (ok && b == 0 && threadIdx.x == 0 && c.state && c.advance) step_advance(c, vel_freq);
+    if (ok && b == 0 && threadIdx.x == 0 && c.state && c.advance)
+        step_advance(c.state, vel_freq, false);
 }
 
 bool order_fits(int n, int ncell) {
@@ -645,28 +647,6 @@ invert_tags_kernel(int n, const int* tag, int* slot_of) {
 cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     invert_tags_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, tag, slot_of);
-    return cudaGetLastError();
-}
-
-__global__ void step_end_kernel(StepState* state, const int* lflag, const uint32_t* err,
-                                int vel_freq, cudaGraphConditionalHandle handle, int use_handle) {
-    const int rebuild = (*err == 0 && *lflag != 0) ? 1 : 0;
-    StepState s = *state;
-    if (*err == 0) {
-        // brownianIntegrator's velCounter bookkeeping (brownianIntegrator.cpp:291-292)
-        // runs only after normal steps
-        if (s.step > 0) s.vel_counter = (s.vel_counter == vel_freq) ? 0 : s.vel_counter + 1;
-        s.step += 1;
-        s.list_builds += rebuild;
-        *state = s;
-    }
-    if (use_handle) cudaGraphSetConditional(handle, (unsigned int)rebuild);
-}
-
-cudaError_t launch_step_end(StepState* state, const int* lflag, const uint32_t* err,
-                            int vel_freq, cudaGraphConditionalHandle handle, int use_handle,
-                            cudaStream_t st) {
-    step_end_kernel<<<1, 1, 0, st>>>(state, lflag, err, vel_freq, handle, use_handle);
     return cudaGetLastError();
 }
 

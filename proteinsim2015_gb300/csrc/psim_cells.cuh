@@ -157,12 +157,12 @@ __device__ __forceinline__ bool block_order(const OrderArgs& o, const CanonArgs&
 
 // The end of a step: brownianIntegrator's velCounter bookkeeping
 // (brownianIntegrator.cpp:291-292) runs only after normal steps.
-__device__ __forceinline__ void step_advance(const CanonArgs& a, int vel_freq) {
-    StepState s = *a.state;
+__device__ __forceinline__ void step_advance(StepState* state, int vel_freq, bool rebuild) {
+    StepState s = *state;
     if (s.step > 0) s.vel_counter = (s.vel_counter == vel_freq) ? 0 : s.vel_counter + 1;
     s.step += 1;
-    if (a.rebuild && *a.rebuild) s.list_builds += 1;
-    *a.state = s;
+    if (rebuild) s.list_builds += 1;
+    *state = s;
 }
 
 }  // namespace psim

@@ -24,6 +24,7 @@ enum : uint32_t {
     EBIT_NOISE = 16u,     // 7706 injected noise buffer does not cover the step
     EBIT_INDEX = 32u,     // 7706 a caller-supplied index or cell range is out of bounds
     EBIT_LIST = 64u,      // 7706 a pair list is full (more neighbours within rc + skin than it holds)
+    EBIT_WAIT = 128u,     // 7790 a barrier inside a kernel gave up
 };
 
 // ----------------------------------------------------------------- geometry

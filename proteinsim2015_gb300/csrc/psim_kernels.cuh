@@ -119,15 +119,14 @@ struct PairList {
 };
 cudaError_t launch_forces_list(const ForceSetup& fs, const DevGeom& g, const PairList& pl,
                                const ForceOut& out, cudaStream_t st);
-// Builds the list from the cell list of cv (list order = cell order) when
-// *gate != 0; pre_r2: FP32 bound on r^2 for (rc + skin) with the rounding margin.
+// Builds the list from the cell list of cv (list order = cell order);
+// pre_r2: FP32 bound on r^2 for (rc + skin) with the rounding margin.
 struct ListBuild {
     uint32_t* list;
     int* count;
     int stride;
     int cap;
     float pre_r2;
-    const int* gate;
     const int* lhalo;      // per list slot: first halo record << 6 | halo_flags
     int ghost;             // the ghost record (n); halo records follow it
     // a batch of replicas (rep null: one system): each slot's replica, the
@@ -409,13 +408,33 @@ cudaError_t launch_list_refresh(int n, const double4_32a* posd, const int* tag,
 // slot_of[tag[k]] = k (tag: every value in [0, n)).
 cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st);
 
-// End of a step whose cell list is rebuilt only with its pair list: advances
-// the step state (canonicalize_kernel's bookkeeping) and decides the rebuild
-// -- the flag the integrator raised, unless an error is latched.  In a graph
-// (use_handle) the decision sets the conditional node that runs the rebuild.
-cudaError_t launch_step_end(StepState* state, const int* lflag, const uint32_t* err,
-                            int vel_freq, cudaGraphConditionalHandle handle, int use_handle,
-                            cudaStream_t st);
+// End of a step with a pair list (psim_rebuild.cu): advances the step state and, where
+// the step raised the flag, rebuilds cell order and list on the positions canon.x..z
+// and carries the state into the new order.  Nothing is done once an error is latched.
+struct RebuildArgs {
+    int n, ncell, vel_freq;
+    StepState* state;
+    const int* lflag;
+    uint32_t* err;
+    unsigned long long* counter;   // of the grid's barriers; starts at 0
+    int* next;                     // the list build's next particle
+    int* sums;                     // rebuild_sums() of them
+    int* key;
+    int* rank;
+    int* count;
+    int* start;
+    int* tmp;
+    CanonArgs canon;
+    double* arr[5];                // positions, previous positions, noise, two forces: 3n
+    double* scratch;               // 15 n
+    int* tag[2];                   // [1] is written by the order, then carried to [0]
+    double* radius[2];
+    double* inv_mass[2];
+    CellView cv;
+    ListBuild lb;
+};
+int rebuild_sums();
+cudaError_t launch_step_rebuild(const RebuildArgs& a, const DevGeom& g, cudaStream_t st);
 
 // dst[k][g] = src[k][perm[g]] for the first narr arrays (the state carried
 // into a new cell order).

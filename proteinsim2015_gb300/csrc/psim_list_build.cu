@@ -1,15 +1,15 @@
-// psim_list_build.cu -- the Verlet pair list's build as a kernel.
+// psim_list_build.cu -- the Verlet pair list's build as a kernel: a system's first list, and
+// those of the host arrays' force pass.  (A step's rebuild is psim_rebuild.cu.)
 #include <algorithm>
 
 #include "psim_list_build.cuh"
 
 namespace psim {
 
-// A grid of a few blocks per SM striding over the particles, so that a step
-// whose rebuild gate is closed costs one short launch.
+// A grid of a few blocks per SM striding over the particles.
 __global__ void __launch_bounds__(128)
 list_build_kernel(DevGeom g, CellView cv, ListBuild lb, uint32_t* errp) {
-    if (*errp != 0 || (lb.gate && *lb.gate == 0)) return;
+    if (*errp != 0) return;
     uint32_t err = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
         if (lb.rep) {   // a batch: the particle's replica's grid and list radius

@@ -1,11 +1,10 @@
 // psim_run.cu -- many steps of a small system through its pair list in one kernel.
 //
-// A step of a few thousand particles is a few microseconds of work behind ~12 us of
-// launches and of the graph's conditional node for the list rebuild.  Here one cluster
-// of 16 blocks, a thread per particle, runs a whole stretch of normal steps: a
-// particle's state stays in its thread's registers, a step ends at one hardware
-// cluster barrier, and a rebuild (hash, scan, scatter, canonical order, list) runs in
-// the same kernel, a barrier between its phases.  The next step's random numbers are
+// A step of a few thousand particles is a few microseconds of work behind the launch
+// of its two kernels.  Here one cluster of 16 blocks, a thread per particle, runs a
+// whole stretch of normal steps: a particle's state stays in its thread's registers, a
+// step ends at one hardware cluster barrier, and a rebuild (hash, cell order, list) runs
+// in the same kernel, a barrier between its phases.  The next step's random numbers are
 // drawn while the barrier completes.  The arithmetic per particle, the list order and
 // the storage between calls are those of step_list_kernel and the rebuild kernels, so
 // the results are the same bit for bit.
@@ -16,11 +15,11 @@
 // What bounds a step is latency: a barrier, then per thread a chain of list groups,
 // records and pair terms in order (a particle's sum keeps one lane and its order), then
 // the update's FP64 chain.  Up to 8192 particles (a thread each in 16 blocks of 512:
-// the registers of an SM) and 65536 cells (the scan is a loop over a thread's share).
-// us a step, one kernel for stretches against a graph of single steps:
-//   AO 100 / 1001 / 4000 / 8192 particles   5.6 / 5.9 / 6.6 / 8.5 against 17.4
-//   LJ liquid (rc 2.5, density 0.38) 4000 / 6912   14.9 / 19.3 against 27.7
-// and 13.7 against 21.7 for a step called alone.
+// the registers of an SM) whose cells fit the order's shared memory.
+// us a step, one kernel for stretches of 25 against a graph of steps of two kernels:
+//   AO 100 / 1001 / 4000 / 8192 particles   5.5 / 5.9 / 6.5 / 8.3 against 8.4 / 9.3 / 9.5 / 9.2
+//   LJ liquid (rc 2.5, density 0.38) 4000 / 6912   14.9 / 19.3 against 20.2 / 19.6
+// (17.4 to 27.7 when each step had a conditional node for its rebuild).
 #include <cooperative_groups.h>
 
 #include "psim_body.cuh"
