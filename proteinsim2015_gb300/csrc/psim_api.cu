@@ -492,6 +492,7 @@ struct Workspace {
     std::mutex mu;
     int device = -1;
     cudaStream_t st = nullptr;
+    uint32_t* host = nullptr;   // pinned: the error word and two flags read back
     DevBuf pos, radius, radius_in, xyz, key, rank, tmp, perm, tag_in, tag_out, radius_out,
         cellid, count, start, scratch, posd, posh, posl, hash_index, cse, sorted, force, fxyz, err;
     // the mixed form's pair list (records, halo words and count, entries),
@@ -538,6 +539,7 @@ int ws_begin(Workspace& w) {
             cudaStreamSynchronize(w.st);
             for (DevBuf* b : all) b->release();
             cudaStreamDestroy(w.st);
+            cudaFreeHost(w.host);
         } else {
             // the old device is gone (reset or lost): its memory went with it
             cudaGetLastError();
@@ -546,7 +548,9 @@ int ws_begin(Workspace& w) {
         PSIM_CUDA(cudaSetDevice(dev));
         w.lkey.valid = false;
         w.st = nullptr;
+        w.host = nullptr;
     }
+    if (!w.host) PSIM_CUDA(cudaMallocHost(&w.host, 16));
     if (!w.st) {
         PSIM_CUDA(cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking));
         w.device = dev;
@@ -667,7 +671,7 @@ int psim_cells_build(const psim_geometry* gm, const double* pos, const double* r
     PSIM_CUDA(w.scratch.ensure(4 * scan_scratch_ints(g.ncell)));
     PSIM_CUDA(w.posd.ensure(32 * n));
     PSIM_CUDA(w.posh.ensure(16 * n));
-    PSIM_CUDA(w.err.ensure(4));
+    PSIM_CUDA(w.err.ensure(8));
     cudaStream_t st = w.st;
     double* x = w.xyz.as<double>();
     // the caller's arrays: read and written in place by the device, or copied
@@ -684,16 +688,26 @@ int psim_cells_build(const psim_geometry* gm, const double* pos, const double* r
         d_pos = w.pos.as<double>();
         d_radius = w.radius_in.as<double>();
     }
-    PSIM_CUDA(cudaMemsetAsync(w.count.p, 0, 4 * nc, st));
-    PSIM_CUDA(cudaMemsetAsync(w.err.p, 0, 4, st));
+    // A small system's order is one kernel where the chain is eight launches of ~2 us each
+    // on the host (20001 particles: three calls of one step 263 -> 234 us with the FP64
+    // pass's one wait fewer).  err[0]: particles outside the grid; err[1]: always 0, so
+    // that the order is made of such particles too (in the cells at the edge).
+    const bool one = order_fits(g.n, g.ncell);
+    PSIM_CUDA(cudaMemsetAsync(w.err.p, 0, 8, st));
     PSIM_CUDA(launch_import_positions(g.n, d_pos, d_radius, x, x + n, x + 2 * n,
-                                      w.radius.as<double>(), st));
-    PSIM_CUDA(launch_hash_count(g.n, x, x + n, x + 2 * n, g, w.key.as<int>(), w.rank.as<int>(),
-                                w.count.as<int>(), w.err.as<uint32_t>(), st));
-    PSIM_CUDA(launch_scan(w.count.as<int>(), w.start.as<int>(), g.ncell, w.scratch.as<int>(), st));
-    PSIM_CUDA(launch_scatter(g.n, w.key.as<int>(), w.rank.as<int>(), w.start.as<int>(),
-                             w.tmp.as<int>(), nullptr, st));
-    PSIM_CUDA(launch_fill_int_iota(g.n, w.tag_in.as<int>(), st));
+                                      w.radius.as<double>(), st, one ? w.key.as<int>() : nullptr,
+                                      &g, w.err.as<uint32_t>()));
+    if (!one) {
+        PSIM_CUDA(cudaMemsetAsync(w.count.p, 0, 4 * nc, st));
+        PSIM_CUDA(launch_hash_count(g.n, x, x + n, x + 2 * n, g, w.key.as<int>(),
+                                    w.rank.as<int>(), w.count.as<int>(), w.err.as<uint32_t>(),
+                                    st));
+        PSIM_CUDA(launch_scan(w.count.as<int>(), w.start.as<int>(), g.ncell,
+                              w.scratch.as<int>(), st));
+        PSIM_CUDA(launch_scatter(g.n, w.key.as<int>(), w.rank.as<int>(), w.start.as<int>(),
+                                 w.tmp.as<int>(), nullptr, st));
+        PSIM_CUDA(launch_fill_int_iota(g.n, w.tag_in.as<int>(), st));
+    }
     CanonArgs ca{};
     ca.n = g.n;
     ca.tmp = w.tmp.as<int>();
@@ -711,7 +725,14 @@ int psim_cells_build(const psim_geometry* gm, const double* pos, const double* r
     ca.cellid = w.cellid.as<int>();
     ca.posd = w.posd.as<double4_32a>();
     ca.posh = w.posh.as<float4>();
-    PSIM_CUDA(launch_canonicalize(ca, st));
+    if (one) {
+        ca.tag_in = nullptr;
+        ca.err = w.err.as<uint32_t>() + 1;
+        const OrderArgs o{g.ncell, w.key.as<int>(), w.count.as<int>(), w.start.as<int>()};
+        PSIM_CUDA(launch_order(o, ca, st));
+    } else {
+        PSIM_CUDA(launch_canonicalize(ca, st));
+    }
     if (w.direct) {
         PSIM_CUDA(launch_export_cells(g.n, g.ncell, w.cellid.as<int>(), w.tag_out.as<int>(),
                                       w.posd.as<double4_32a>(), w.start.as<int>(),
@@ -728,9 +749,9 @@ int psim_cells_build(const psim_geometry* gm, const double* pos, const double* r
         if (sorted)
             PSIM_CUDA(cudaMemcpyAsync(sorted, w.sorted.p, 32 * n, cudaMemcpyDeviceToHost, st));
     }
-    uint32_t bits = 0;
-    PSIM_CUDA(cudaMemcpyAsync(&bits, w.err.p, 4, cudaMemcpyDeviceToHost, st));
+    PSIM_CUDA(cudaMemcpyAsync(w.host, w.err.p, 4, cudaMemcpyDeviceToHost, st));
     PSIM_CUDA(cudaStreamSynchronize(st));
+    const uint32_t bits = *w.host;
     if (bits) return fail(code_from_bits(bits), "%s", bits_text(bits));
     return PSIM_OK;
 }
@@ -768,7 +789,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
     PSIM_CUDA(w.scratch.ensure(4 * scan_scratch_ints(g.ncell)));
     PSIM_CUDA(w.fxyz.ensure(24 * n));
     PSIM_CUDA(w.inv.ensure(4 * n));
-    PSIM_CUDA(w.err.ensure(4));
+    PSIM_CUDA(w.err.ensure(8));
     PSIM_CUDA(w.lflag.ensure(8));
     cudaStream_t st = w.st;
     // the caller's arrays: read in place by the device, or copied in
@@ -787,7 +808,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
         d_hi = w.hash_index.as<int32_t>();
         d_cse = w.cse.as<uint32_t>();
     }
-    PSIM_CUDA(cudaMemsetAsync(w.err.p, 0, 4, st));
+    PSIM_CUDA(cudaMemsetAsync(w.err.p, 0, 8, st));
     // flags: [0] a particle moved too far for the kept list, [1] mixed radii
     int* flags = w.lflag.as<int>();
     PSIM_CUDA(cudaMemsetAsync(flags, 0, 8, st));
@@ -840,12 +861,20 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
             PSIM_CUDA(cudaMemcpyAsync(force, w.force.p, 24 * n, cudaMemcpyDeviceToHost, st));
     }
     w.lcalls += precision == PSIM_PRECISION_MIXED ? 1 : 0;
-    // a position outside the grid has no home cell: stop before the force pass
+    // a position outside the grid has no home cell: stop before the force pass.  The
+    // FP64 pass stops by itself on the device, and this call need not wait here (a
+    // plugin's own pass, or a block per cell, might not).
+    const bool fp64 = precision == PSIM_PRECISION_FP64 && !plugin && !fs.tile;
     uint32_t bits = 0;
     int hflags[2] = {0, 0};
-    PSIM_CUDA(cudaMemcpyAsync(&bits, w.err.p, 4, cudaMemcpyDeviceToHost, st));
-    PSIM_CUDA(cudaMemcpyAsync(hflags, flags, 8, cudaMemcpyDeviceToHost, st));
-    PSIM_CUDA(cudaStreamSynchronize(st));
+    if (!fp64) {
+        PSIM_CUDA(cudaMemcpyAsync(w.host, w.err.p, 4, cudaMemcpyDeviceToHost, st));
+        PSIM_CUDA(cudaMemcpyAsync(w.host + 1, flags, 8, cudaMemcpyDeviceToHost, st));
+        PSIM_CUDA(cudaStreamSynchronize(st));
+        bits = w.host[0];
+        hflags[0] = (int)w.host[1];
+        hflags[1] = (int)w.host[2];
+    }
     if (bits) {
         w.lkey.valid = false;
         return fail(code_from_bits(bits), "%s", bits_text(bits));
@@ -882,8 +911,9 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
         ListBuild lb{w.list.as<uint32_t>(), w.lcount.as<int>(), g.n, z.cap, z.pre,
                      w.lhalo.as<int>(), g.n};
         PSIM_CUDA(launch_list_build(g, cv, lb, w.err.as<uint32_t>(), st));
-        PSIM_CUDA(cudaMemcpyAsync(&bits, w.err.p, 4, cudaMemcpyDeviceToHost, st));
+        PSIM_CUDA(cudaMemcpyAsync(w.host, w.err.p, 4, cudaMemcpyDeviceToHost, st));
         PSIM_CUDA(cudaStreamSynchronize(st));
+        bits = *w.host;
         w.lbuilds++;
         if (bits == EBIT_LIST) {
             // a denser neighbourhood than the list has room for: the cell walk
@@ -911,6 +941,11 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
             inv = w.lslot_of.as<int>();
         }
     } else if (precision == PSIM_PRECISION_FP64) {
+        if (fp64) {   // keeps the import's refusal apart from the pass's own errors
+            PSIM_CUDA(launch_invert_tags(g.n, w.tag_out.as<int>(), w.inv.as<int>(), st,
+                                         w.err.as<uint32_t>()));
+            inv = w.inv.as<int>();
+        }
         PSIM_CUDA(fr.run(PSIM_PASS_FP64, g, &cv, nullptr, out, st));
     } else {
         PSIM_CUDA(fr.run(PSIM_PASS_MIXED, g, &cv, nullptr, out, st));
@@ -920,11 +955,15 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
         inv = w.inv.as<int>();
     }
     PSIM_CUDA(launch_export_force(g.n, inv, f, f + n, f + 2 * n,
-                                  w.direct ? force : w.force.as<double>(), st));
-    PSIM_CUDA(cudaMemcpyAsync(&bits, w.err.p, 4, cudaMemcpyDeviceToHost, st));
-    if (!w.direct)
+                                  w.direct ? force : w.force.as<double>(), st,
+                                  fp64 ? w.err.as<uint32_t>() + 1 : nullptr));
+    PSIM_CUDA(cudaMemcpyAsync(w.host, w.err.p, 8, cudaMemcpyDeviceToHost, st));
+    if (!w.direct && !fp64)
         PSIM_CUDA(cudaMemcpyAsync(force, w.force.p, 24 * n, cudaMemcpyDeviceToHost, st));
     PSIM_CUDA(cudaStreamSynchronize(st));
+    bits = w.host[0];
+    if (!w.direct && fp64 && w.host[1] == 0)   // not when the arrays were refused
+        PSIM_CUDA(cudaMemcpy(force, w.force.p, 24 * n, cudaMemcpyDeviceToHost));
     if (bits) {
         w.lkey.valid = false;
         return fail(code_from_bits(bits), "%s", bits_text(bits));
@@ -986,6 +1025,7 @@ struct psim_integrator {
     int vel_counter = 0;
     long long steps = 0;
     DevBuf mem, mem_corr, pos, pos0, vel, frc, frc0, mass, noise, err;
+    uint32_t* host = nullptr;   // pinned: the error word read back
 };
 
 extern "C" {
@@ -1015,6 +1055,7 @@ psim_integrator* psim_integrator_create(const psim_integrator_config* cfg, int32
         it->mem.ensure(b) || it->mem_corr.ensure(b) || it->pos.ensure(b) || it->pos0.ensure(b) ||
         it->vel.ensure(b) || it->frc.ensure(b) || it->frc0.ensure(b) ||
         it->mass.ensure(8 * (size_t)n) || it->err.ensure(4) ||
+        cudaMallocHost(&it->host, 16) != cudaSuccess ||
         cudaMemset(it->mem.p, 0, b) || cudaMemset(it->mem_corr.p, 0, b)) {
         fail(PSIM_ERR_CUDA, "integrator allocation failed: %s", cudaGetErrorString(cudaGetLastError()));
         psim_integrator_destroy(it);
@@ -1031,6 +1072,7 @@ void psim_integrator_destroy(psim_integrator* it) {
     DevBuf* all[] = {&it->mem, &it->mem_corr, &it->pos, &it->pos0, &it->vel, &it->frc,
                      &it->frc0, &it->mass, &it->noise, &it->err};
     for (DevBuf* b : all) b->release();
+    if (it->host) cudaFreeHost(it->host);
     for (int k = 0; k < kAosChunks; ++k) {
         if (it->ev_in[k]) cudaEventDestroy(it->ev_in[k]);
         if (it->ev_run[k]) cudaEventDestroy(it->ev_run[k]);
@@ -1085,9 +1127,9 @@ int psim_integrator_next_system(psim_integrator* it, double current_time, double
         a.philox_step = it->steps;
         a.err = it->err.as<uint32_t>();
         PSIM_CUDA(launch_vgb_host(a, it->vp, box, st));
-        uint32_t bits = 0;
-        PSIM_CUDA(cudaMemcpyAsync(&bits, it->err.p, 4, cudaMemcpyDeviceToHost, st));
+        PSIM_CUDA(cudaMemcpyAsync(it->host, it->err.p, 4, cudaMemcpyDeviceToHost, st));
         PSIM_CUDA(cudaStreamSynchronize(st));
+        const uint32_t bits = *it->host;
         if (!first)  // brownianIntegrator.cpp:291-292
             it->vel_counter = (it->vel_counter == it->vp.vel_freq) ? 0 : it->vel_counter + 1;
         it->steps++;

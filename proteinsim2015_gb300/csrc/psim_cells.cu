@@ -12,6 +12,7 @@
 //      fused with the gather of everything the force pass reads
 // The cell hashes and memberships equal the reference's bit for bit.
 #include "psim_cells.cuh"
+#include "psim_vgb.cuh"
 
 namespace psim {
 
@@ -317,8 +318,9 @@ cudaError_t launch_import_sorted(int n, const double* sorted, const int32_t* has
 // written in place) through shared memory in coalesced runs.
 __global__ void __launch_bounds__(256)
 export_force_kernel(int n, const int* inv, const double* fx, const double* fy, const double* fz,
-                    double* out) {
+                    double* out, const uint32_t* refused) {
     __shared__ double so[3 * 256];
+    if (refused && *refused) return;
     const int b0 = blockIdx.x * blockDim.x;
     const int m = min((int)blockDim.x, n - b0);
     const int i = b0 + threadIdx.x;
@@ -333,9 +335,10 @@ export_force_kernel(int n, const int* inv, const double* fx, const double* fy, c
 }
 
 cudaError_t launch_export_force(int n, const int* inv, const double* fx, const double* fy,
-                                const double* fz, double* out, cudaStream_t st) {
+                                const double* fz, double* out, cudaStream_t st,
+                                const uint32_t* refused) {
     if (n == 0) return cudaSuccess;
-    export_force_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, inv, fx, fy, fz, out);
+    export_force_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, inv, fx, fy, fz, out, refused);
     return cudaGetLastError();
 }
 
@@ -387,10 +390,10 @@ split_xyz_kernel(int n, const double* aos, const int* tag, int gather, double* x
 
 // Positions (3n AoS) and radii of the caller, which may be host memory read
 // in place, into SoA coordinates and a device copy of the radii, each block
-// reading its spans as coalesced runs through shared memory.
+// reading its spans as coalesced runs through shared memory; with key, their cells too.
 __global__ void __launch_bounds__(256)
 import_positions_kernel(int n, const double* aos, const double* radius, double* x, double* y,
-                        double* z, double* radius_out) {
+                        double* z, double* radius_out, int* key, DevGeom g, uint32_t* err) {
     __shared__ double sp[3 * 256];
     const int b0 = blockIdx.x * blockDim.x;
     const int m = min((int)blockDim.x, n - b0);
@@ -402,12 +405,19 @@ import_positions_kernel(int n, const double* aos, const double* radius, double* 
     y[i] = sp[3 * threadIdx.x + 1];
     z[i] = sp[3 * threadIdx.x + 2];
     radius_out[i] = radius[i];
+    if (key) {
+        uint32_t bad = 0;
+        key[i] = hash_pos(&sp[3 * threadIdx.x], g, bad);
+        if (bad) atomicOr(err, bad);
+    }
 }
 
 cudaError_t launch_import_positions(int n, const double* aos, const double* radius, double* x,
-                                    double* y, double* z, double* radius_out, cudaStream_t st) {
+                                    double* y, double* z, double* radius_out, cudaStream_t st,
+                                    int* key, const DevGeom* g, uint32_t* err) {
     if (n == 0) return cudaSuccess;
-    import_positions_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, aos, radius, x, y, z, radius_out);
+    import_positions_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, aos, radius, x, y, z, radius_out,
+                                                             key, g ? *g : DevGeom{}, err);
     return cudaGetLastError();
 }
 
@@ -637,16 +647,24 @@ cudaError_t launch_list_refresh(int n, const double4_32a* posd, const int* tag,
     return cudaGetLastError();
 }
 
-// slot_of[tag[k]] = k: the slot of each original index in a sorted order
+// slot_of[tag[k]] = k: the slot of each original index in a sorted order.  With err,
+// nothing when *err says that the tags were refused, and err[1] keeps the word as it is
+// here, before the force pass adds to it.
 __global__ void __launch_bounds__(256)
-invert_tags_kernel(int n, const int* tag, int* slot_of) {
+invert_tags_kernel(int n, const int* tag, int* slot_of, uint32_t* err) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (err) {
+        const uint32_t refused = err[0];
+        if (k == 0) err[1] = refused;
+        if (refused) return;
+    }
     if (k < n) slot_of[tag[k]] = k;
 }
 
-cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st) {
+cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st,
+                               uint32_t* err) {
     if (n == 0) return cudaSuccess;
-    invert_tags_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, tag, slot_of);
+    invert_tags_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, tag, slot_of, err);
     return cudaGetLastError();
 }
 

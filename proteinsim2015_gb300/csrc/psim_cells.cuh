@@ -8,10 +8,12 @@ namespace psim {
 
 // Particle f's place inside its cell c, whose cnt slots from st on hold the particles
 // tmp(st) .. (scattered in any order), and there everything the force pass reads.
-template <class Tmp>
+// (kTags: a.tag_in holds the tags; otherwise a particle's index is its tag.)
+template <bool kTags, class Tmp>
 __device__ __forceinline__ void canon_place(const CanonArgs& a, int f, int c, int st, int cnt,
                                             Tmp tmp) {
-    const int mine = a.tag_in[f];
+    auto tag = [&](int i) { return kTags ? a.tag_in[i] : i; };
+    const int mine = tag(f);
     int r = 0;
     if (a.xorder) {
         // by x, then tag: the bit patterns of the (non-negative) positions
@@ -20,10 +22,10 @@ __device__ __forceinline__ void canon_place(const CanonArgs& a, int f, int c, in
         for (int q = st; q < st + cnt; ++q) {
             const int fq = tmp(q);
             const long long xq = __double_as_longlong(a.x[fq]);
-            r += (xq < mx || (xq == mx && a.tag_in[fq] < mine)) ? 1 : 0;
+            r += (xq < mx || (xq == mx && tag(fq) < mine)) ? 1 : 0;
         }
     } else {
-        for (int q = st; q < st + cnt; ++q) r += (a.tag_in[tmp(q)] < mine) ? 1 : 0;
+        for (int q = st; q < st + cnt; ++q) r += (tag(tmp(q)) < mine) ? 1 : 0;
     }
     const int g = st + r;
     a.perm[g] = f;
@@ -81,7 +83,7 @@ __device__ __forceinline__ void canon_place(const CanonArgs& a, int f, int c, in
 
 __device__ __forceinline__ void canon_slot(const CanonArgs& a, int p) {
     const int f = a.tmp[p], c = a.key[f];
-    canon_place(a, f, c, a.start[c], a.count[c], [&](int q) { return a.tmp[q]; });
+    canon_place<true>(a, f, c, a.start[c], a.count[c], [&](int q) { return a.tmp[q]; });
 }
 
 // The whole order by one block that holds the cells and the particles' keys in shared
@@ -150,7 +152,10 @@ __device__ __forceinline__ bool block_order(const OrderArgs& o, const CanonArgs&
     __syncthreads();
     for (int f = f0 + tid; f < f1; f += T) {
         const int k = key[f], st = start[k];
-        canon_place(c, f, k, st, start[k + 1] - st, [&](int q) { return (int)tmp[q]; });
+        const int m = start[k + 1] - st;
+        auto at = [&](int q) { return (int)tmp[q]; };
+        if (c.tag_in) canon_place<true>(c, f, k, st, m, at);
+        else canon_place<false>(c, f, k, st, m, at);
     }
     return true;
 }

@@ -292,7 +292,7 @@ struct CanonArgs {
     const int* key;         // cell of each previous-order index
     const int* start;
     const int* count;
-    const int* tag_in;      // previous order
+    const int* tag_in;      // previous order (launch_order: null, the index)
     const double* radius_in;
     const double* inv_mass_in;
     const double* x; const double* y; const double* z;   // positions, previous order
@@ -406,7 +406,8 @@ cudaError_t launch_list_refresh(int n, const double4_32a* posd, const int* tag,
                                 float4* lpos, float disp2, const DevGeom& g, float inv_unit,
                                 float radius, int* flag, cudaStream_t st);
 // slot_of[tag[k]] = k (tag: every value in [0, n)).
-cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st);
+cudaError_t launch_invert_tags(int n, const int* tag, int* slot_of, cudaStream_t st,
+                               uint32_t* err = nullptr);
 
 // End of a step with a pair list (psim_rebuild.cu): advances the step state and, where
 // the step raised the flag, rebuilds cell order and list on the positions canon.x..z
@@ -466,7 +467,8 @@ cudaError_t launch_import_sorted(int n, const double* sorted, const int32_t* has
 // out[3 i + k] = f_k[inv[i]]: forces from the force pass's order to the
 // original order (out may be host memory written in place).
 cudaError_t launch_export_force(int n, const int* inv, const double* fx, const double* fy,
-                                const double* fz, double* out, cudaStream_t st);
+                                const double* fz, double* out, cudaStream_t st,
+                                const uint32_t* refused = nullptr);
 // Counts from (start, end) pairs, starts re-derived by a scan (so empty
 // cells keep the back-to-back layout the row walk of the force pass needs);
 // a range beyond n, or a start that disagrees with that layout, sets
@@ -476,7 +478,9 @@ cudaError_t launch_import_cse(int ncell, int n, const uint32_t* cse, int* start,
 // Positions (3n AoS) and radii, possibly host memory read in place, into
 // SoA x, y, z and a device copy of the radii.
 cudaError_t launch_import_positions(int n, const double* aos, const double* radius, double* x,
-                                    double* y, double* z, double* radius_out, cudaStream_t st);
+                                    double* y, double* z, double* radius_out, cudaStream_t st,
+                                    int* key = nullptr, const DevGeom* g = nullptr,
+                                    uint32_t* err = nullptr);
 // AoS xyz -> three arrays, optionally scattered by tag (gather == 0) or
 // gathered (gather == 1: out[i] = in[tag[i]]).
 cudaError_t launch_split_xyz(int n, const double* aos, const int* tag, int gather, double* x,

@@ -4,6 +4,7 @@ the force pass on the oracle's sorted particles (cells in order, tags within a c
 import numpy as np
 import pytest
 
+from gpu_helpers import oracle_force
 from oracle import port
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +41,34 @@ def test_canonical_order(psim, n, box, scale):
         hi, cse, srt = port.build_cells(og, x, rad)
         assert np.array_equal(s.forces(), psim.force_evaluate(p, g, srt, hi, cse))
     s.close()
+
+
+@pytest.mark.parametrize("n,box,scale", [(1, 9.0, 5), (257, 9.0, 5), (ORDER_MAX, 45.0, 29),
+                                         (ORDER_MAX + 1, 45.0, 29)])
+def test_host_arrays_order(psim, n, box, scale):
+    rng = np.random.default_rng(n)
+    pos, rad = rng.uniform(0.0, box, 3 * n), rng.uniform(0.3, 0.5, n)
+    g = psim.geometry(n, box, box / scale, scale)
+    hi, cse, srt = port.build_cells(port.geom(n, box, box / scale, scale), pos, rad)
+    got = psim.cells_build(g, pos, rad)
+    assert np.array_equal(got[0], hi) and np.array_equal(got[2], srt)
+    assert np.array_equal(got[1], cse)
+    pos[3 * (n // 2)] = box * 1.5
+    with pytest.raises(psim.PsimError) as e:
+        psim.cells_build(g, pos, rad)
+    assert e.value.code == psim.ERR_CELL_BOUNDS
+
+
+def test_refused_arrays_leave_the_forces_alone(psim):
+    n, box, scale = 300, 9.0, 5
+    pos, rad = np.random.default_rng(1).uniform(0.0, box, 3 * n), np.full(n, 0.1)
+    p = psim.make_force("AO", 1.2, kT=1.0, well_depth=0.3)
+    g = psim.geometry(n, box, box / scale, scale)
+    hi, cse, srt, ref, err, _ = oracle_force(p.as_dict(), g, pos, rad)
+    for bad in (-1, n):
+        h = hi.copy()
+        h[1] = bad
+        out = np.full(3 * n, 7.0)
+        with pytest.raises(psim.PsimError) as e:
+            psim.force_evaluate(p, g, srt, h, cse, out=out)
+        assert e.value.code == psim.ERR_INPUT and np.all(out == 7.0)
