@@ -1537,7 +1537,7 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs, bool fused = fal
     if (evs) PSIM_CUDA(cudaEventRecord(evs[0], st));
     ForceOut fo{d3(s->frc[ph.fcur], n, 0), d3(s->frc[ph.fcur], n, 1), d3(s->frc[ph.fcur], n, 2),
                 s->err.as<uint32_t>(), nullptr};
-    PSIM_CUDA(enqueue_force(s, ph, fo));
+    if (!fused) PSIM_CUDA(enqueue_force(s, ph, fo));
     if (evs) PSIM_CUDA(cudaEventRecord(evs[1], st));
     // integrator: pushParticleForce + nextSystem, hash + count into the next grid (left to
     // the kernel of the whole order where there is one)
@@ -1570,7 +1570,11 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs, bool fused = fal
     }
     a.img = s->img.as<int>();   // null until the displacement tracker starts
     NoiseView nz{s->cfg.noise_mode, s->noise.as<double>(), s->noise_first, s->noise_steps};
-    if (s->cfg.precision == PSIM_PRECISION_FP64)
+    if (fused) {
+        CellView cv{s->posd.as<double4_32a>(), s->posh.as<float4>(), nullptr,
+                    s->cellid.as<int>(), s->start.as<int>(), s->count[cb].as<int>()};
+        PSIM_CUDA(launch_step_fp64(s->fs, s->g, cv, fo, a, s->vp, nz, st));
+    } else if (s->cfg.precision == PSIM_PRECISION_FP64)
         PSIM_CUDA(launch_vgb_system(a, s->vp, s->g, nz, st));
     else
         PSIM_CUDA(launch_vgb_system_fast(a, s->vp, s->g, nz, st));
@@ -1627,9 +1631,17 @@ int graph_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_
     return PSIM_OK;
 }
 
-// Whether the normal steps of s run in the one kernel of psim_step.cu.
+// FP64 systems whose normal steps are one kernel for force pass and update: at 16000
+// particles a step takes 26.5 us so and 27.6 as two, at 20001 33.6 and 29.5.
+constexpr int kStep64 = 1 << 14;
+
+// Whether the force pass and the update of a normal step of s are one kernel: that of
+// psim_step.cu with a pair list, step_quad_kernel for a small FP64 system without one.
 bool fused_steps(const psim_system* s) {
-    return s->list_on && s->lcompact && s->list_lanes == 1 && !s->cfg.force_launch && !s->img.p;
+    if (s->cfg.force_launch || s->img.p) return false;
+    if (s->list_on) return s->lcompact && s->list_lanes == 1;
+    return s->cfg.precision == PSIM_PRECISION_FP64 && !s->n_reps && !s->fs.tile &&
+           s->n <= kStep64 && one_order(s);
 }
 // The velocity counter's period: step t > 0 writes the velocities when it
 // divides t; step 0 is the first step.
@@ -1653,7 +1665,7 @@ constexpr int kRunSteps = 1024, kRunLeast = 4;   // of one such launch
 // of kRunLeast steps at least: alone a step of 4000 takes 15.4 against 13.7, of 8192 18.7
 // against 14.0.
 bool small_system(psim_system* s) {
-    if (!fused_steps(s) || s->n_reps) return false;
+    if (!s->list_on || !fused_steps(s) || s->n_reps) return false;
     if (s->small < 0) s->small = run_list_fits(s->fs, s->n, s->ncell) ? 1 : 0;
     return s->small == 1;
 }
@@ -2850,7 +2862,7 @@ int psim_system_launches_per_step(psim_system* s) {
     // on normal steps where fused_steps allows), the step end with its rebuild; a small
     // system's normal step alone, or a stretch of them, is one kernel
     if (!s) return 7;
-    if (!s->list_on) return one_order(s) ? 3 : 7;
+    if (!s->list_on) return fused_steps(s) ? 2 : (one_order(s) ? 3 : 7);
     DeviceGuard dg(s->device);
     return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
 }

@@ -217,6 +217,11 @@ struct VgbSystemArgs {
     // the unwrapped position is x + img L
     int* img;
 };
+// A normal step of a small FP64 system without a pair list: force pass and update in one
+// kernel (single systems; a.key receives the cells, a.count and a.img are null).
+cudaError_t launch_step_fp64(const ForceSetup& fs, const DevGeom& g, const CellView& cv,
+                             const ForceOut& out, const VgbSystemArgs& a, const VgbParams& p,
+                             const NoiseView& nz, cudaStream_t st);
 cudaError_t launch_vgb_system(const VgbSystemArgs& a, const VgbParams& p, const DevGeom& g,
                               const NoiseView& nz, cudaStream_t st);
 // The same update with FMA contraction (psim_mixed.cu), for the mixed form.

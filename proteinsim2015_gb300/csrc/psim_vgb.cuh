@@ -129,6 +129,29 @@ __device__ __forceinline__ void vgb_particle(const VgbParams& p, double L, doubl
     }
 }
 
+// One axis of vgb_particle's normal step: the same operations.  xk, xm: draws k and
+// 3 + k of axis k.
+__device__ __forceinline__ void vgb_normal_axis(const VgbParams& p, double L, double half_L,
+                                                double x, double x0, double& mx, double F,
+                                                double F0, double xk, double xm, double m,
+                                                double& xn, double& x0n, uint32_t& err) {
+    const double c1 = m * p.dt2 * p.coeff1;
+    const double c2 = m * p.dt2 * p.coeff2;
+    const double mc = p.sig2 * ((p.corr * mx) + (p.dev * xk));
+    mx = xm;
+    double t = (p.c0 * x);
+    t -= (p.coeff0 * x0);
+    t += (c1 * F);
+    t += (c2 * (F - F0));
+    t += (p.sig1 * mx) + (p.coeff0 * mc);
+    xn = t;
+    if (neg_d(t)) xn = t + L;
+    else if (ge_pos_d(t, L)) xn = t - L;
+    x0n = x;
+    if (abs_gt_d(xn - x, half_L)) x0n = (xn - x < 0) ? x - L : x + L;
+    if (neg_d(xn) || ge_pos_d(xn, L) || !(xn == xn)) err |= EBIT_BOUNDS;
+}
+
 // normalStep of the mixed form (brownianIntegrator.cpp:225-296), written as
 //   x_new = x + [coEff0 (x - x0) + dt^2 coEff1 F/m + dt^2 coEff2 (F - F0)/m + noise]
 // (c0 = 1 + coEff0): the bracket -- a displacement of ~v dt -- is summed in
@@ -201,17 +224,18 @@ __device__ __forceinline__ int cell_coord_fast(double x, const DevGeom& g) {
     return cell_coord(x, g);
 }
 
+__device__ __forceinline__ int hash_axis(double x, const DevGeom& g, uint32_t& err) {
+    int q = cell_coord_fast(x, g);
+    if (q < 0 || q >= g.s) {
+        err |= EBIT_CELL;
+        q = q < 0 ? 0 : g.s - 1;
+    }
+    return q;
+}
 __device__ __forceinline__ int hash_pos(const double xn[3], const DevGeom& g, uint32_t& err) {
     int c[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        int q = cell_coord_fast(xn[k], g);
-        if (q < 0 || q >= g.s) {
-            err |= EBIT_CELL;
-            q = q < 0 ? 0 : g.s - 1;
-        }
-        c[k] = q;
-    }
+    for (int k = 0; k < 3; ++k) c[k] = hash_axis(xn[k], g, err);
     return g.c0 + c[0] + g.s * c[1] + g.s2 * c[2];  // systemHandling.cpp:43 (+ the batch offset)
 }
 
