@@ -1552,6 +1552,7 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs, bool fused = fal
     a.x0 = d3(s->pos0[sb], n, 0); a.y0 = d3(s->pos0[sb], n, 1); a.z0 = d3(s->pos0[sb], n, 2);
     a.mx = d3(s->mem[sb], n, 0); a.my = d3(s->mem[sb], n, 1); a.mz = d3(s->mem[sb], n, 2);
     a.fx = fo.fx; a.fy = fo.fy; a.fz = fo.fz;
+    a.ofx = fo.fx; a.ofy = fo.fy; a.ofz = fo.fz;
     a.gx = d3(s->frc[ph.fprev], n, 0); a.gy = d3(s->frc[ph.fprev], n, 1);
     a.gz = d3(s->frc[ph.fprev], n, 2);
     a.vel = s->vel.as<double>();
@@ -1571,9 +1572,12 @@ int enqueue_step(psim_system* s, long long t, cudaEvent_t* evs, bool fused = fal
     a.img = s->img.as<int>();   // null until the displacement tracker starts
     NoiseView nz{s->cfg.noise_mode, s->noise.as<double>(), s->noise_first, s->noise_steps};
     if (fused) {
-        CellView cv{s->posd.as<double4_32a>(), s->posh.as<float4>(), nullptr,
+        CellView cv{s->posd.as<double4_32a>(), s->posh.as<float4>(), s->posl.as<float4>(),
                     s->cellid.as<int>(), s->start.as<int>(), s->count[cb].as<int>()};
-        PSIM_CUDA(launch_step_fp64(s->fs, s->g, cv, fo, a, s->vp, nz, st));
+        if (s->cfg.precision == PSIM_PRECISION_FP64)
+            PSIM_CUDA(launch_step_fp64(s->fs, s->g, cv, fo, a, s->vp, nz, st));
+        else
+            PSIM_CUDA(launch_step_direct(s->fs, s->g, cv, fo, a, s->vp, nz, st));
     } else if (s->cfg.precision == PSIM_PRECISION_FP64)
         PSIM_CUDA(launch_vgb_system(a, s->vp, s->g, nz, st));
     else
@@ -1634,14 +1638,19 @@ int graph_steps(psim_system* s, int phase, int steps, bool fused, cudaGraphExec_
 // FP64 systems whose normal steps are one kernel for force pass and update: at 16000
 // particles a step takes 26.5 us so and 27.6 as two, at 20001 33.6 and 29.5.
 constexpr int kStep64 = 1 << 14;
+// Mixed systems without a pair list likewise: AO colloids of 300001 65.0 us so and 67.5 as
+// two, the gel of 2^20 192.5 and 187.6.
+constexpr int kStepDirect = 3 << 17;
 
-// Whether the force pass and the update of a normal step of s are one kernel: that of
-// psim_step.cu with a pair list, step_quad_kernel for a small FP64 system without one.
+// Whether the force pass and the update of a normal step of s are one kernel: with a pair
+// list step_list_kernel, without one step_direct_kernel (mixed) or step_quad_kernel (FP64).
 bool fused_steps(const psim_system* s) {
     if (s->cfg.force_launch || s->img.p) return false;
     if (s->list_on) return s->lcompact && s->list_lanes == 1;
-    return s->cfg.precision == PSIM_PRECISION_FP64 && !s->n_reps && !s->fs.tile &&
-           s->n <= kStep64 && one_order(s);
+    if (s->n_reps) return false;
+    if (s->cfg.precision == PSIM_PRECISION_MIXED)
+        return s->n <= kStepDirect && step_direct_fits(s->fs, s->g);
+    return !s->fs.tile && s->n <= kStep64 && one_order(s);
 }
 // The velocity counter's period: step t > 0 writes the velocities when it
 // divides t; step 0 is the first step.
@@ -2862,7 +2871,7 @@ int psim_system_launches_per_step(psim_system* s) {
     // on normal steps where fused_steps allows), the step end with its rebuild; a small
     // system's normal step alone, or a stretch of them, is one kernel
     if (!s) return 7;
-    if (!s->list_on) return fused_steps(s) ? 2 : (one_order(s) ? 3 : 7);
+    if (!s->list_on) return (one_order(s) ? 3 : 7) - (fused_steps(s) ? 1 : 0);
     DeviceGuard dg(s->device);
     return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
 }

@@ -232,16 +232,15 @@ __host__ __device__ __forceinline__ bool direct_walk(const DevGeom& g, int walk 
 }
 
 template <class Body>
-__device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeom& g,
-                                                  const CellView& cv, const ForceOut& out,
-                                                  float pre_rc2, int i, bool active, int lane,
-                                                  uint32_t (*q)[32]) {
+__device__ __forceinline__ void direct_terms(const Body& body, const DevGeom& g,
+                                             const CellView& cv, float pre_rc2, int i, bool active,
+                                             int lane, uint32_t (*q)[32],
+                                             typename Body::Acc& acc, uint32_t& err) {
     using Aux = typename Body::Aux;
     const Aux* g_aux = body.aux(cv);
     float4 hi = make_float4(0.f, 0.f, 0.f, 0.f);
     int cx = 0, cy = 0, cz = 0;
     typename Body::Home home;
-    typename Body::Acc acc;
     body.init(acc);
     if (active) {
         hi = cv.posh[i];
@@ -250,7 +249,6 @@ __device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeo
     }
     typename Body::Shifted hs;
     body.shift(home, hi, 0, 0, 0, g, hs);
-    uint32_t err = 0;
     int cnt = 0;   // entries in the lane's queue
     auto drain = [&]() {
         const int kmax = __reduce_max_sync(0xffffffffu, cnt);
@@ -323,6 +321,16 @@ __device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeo
         }
     }
     drain();
+}
+
+template <class Body>
+__device__ __forceinline__ void force_direct_warp(const Body& body, const DevGeom& g,
+                                                  const CellView& cv, const ForceOut& out,
+                                                  float pre_rc2, int i, bool active, int lane,
+                                                  uint32_t (*q)[32]) {
+    typename Body::Acc acc;
+    uint32_t err = 0;
+    direct_terms(body, g, cv, pre_rc2, i, active, lane, q, acc, err);
     if (active) body.store(out, i, acc);
     if (err) atomicOr(out.err, err);
 }

@@ -217,6 +217,12 @@ struct VgbSystemArgs {
     // the unwrapped position is x + img L
     int* img;
 };
+// A normal step of a mixed system without a pair list, likewise; whether it can be taken.
+bool step_direct_fits(const ForceSetup& fs, const DevGeom& g);
+cudaError_t launch_step_direct(const ForceSetup& fs, const DevGeom& g, const CellView& cv,
+                               const ForceOut& out, const VgbSystemArgs& a, const VgbParams& p,
+                               const NoiseView& nz, cudaStream_t st);
+
 // A normal step of a small FP64 system without a pair list: force pass and update in one
 // kernel (single systems; a.key receives the cells, a.count and a.img are null).
 cudaError_t launch_step_fp64(const ForceSetup& fs, const DevGeom& g, const CellView& cv,

@@ -417,6 +417,31 @@ __device__ __forceinline__ void vgb_normal_one(const VgbSystemArgs& a, const Vgb
     if (err) atomicOr(a.err, err);
 }
 
+// vgb_system_one for a normal step of the mixed form without a pair list, with the force
+// F in hand: the state gathered from the previous order, the next cell list hashed.
+__device__ __forceinline__ void vgb_normal_moved(const VgbSystemArgs& a, const VgbParams& p,
+                                                 const DevGeom& g, const NoiseView& nz, int f,
+                                                 const double F[3], uint32_t err) {
+    const long long step = a.state->step;
+    const int o = a.perm[f], tag = a.tag[f];
+    const double m = a.inv_mass[f];
+    const double x[3] = {a.x[o], a.y[o], a.z[o]};
+    const double x0[3] = {a.x0[o], a.y0[o], a.z0[o]};
+    double mx[3] = {a.mx[o], a.my[o], a.mz[o]};
+    const double F0[3] = {a.gx[o], a.gy[o], a.gz[o]};
+    float xf[6];
+    load_noise_f(nz, p.seed, a.n, tag, tag - g.p0, step, xf, err);
+    double xn[3], x0n[3];
+    vgb_normal_fast(p, g.L, g.half, x, x0, mx, F, F0, xf, m, xn, x0n, err);
+    a.ox[f] = xn[0]; a.oy[f] = xn[1]; a.oz[f] = xn[2];
+    a.ox0[f] = x0n[0]; a.oy0[f] = x0n[1]; a.oz0[f] = x0n[2];
+    a.omx[f] = mx[0]; a.omy[f] = mx[1]; a.omz[f] = mx[2];
+    const int key = hash_pos(xn, g, err);
+    a.key[f] = key;
+    if (a.count) a.rank[f] = atomicAdd(&a.count[key], 1);   // (order_kernel counts itself)
+    if (err) atomicOr(a.err, err);
+}
+
 // One system (the geometry is a kernel parameter) or, with kBatch, each
 // particle's replica of a batch (its geometry and Philox seed from tables).
 template <class Tag, bool kBatch>
