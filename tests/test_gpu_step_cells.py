@@ -1,7 +1,7 @@
 """The step without a pair list as one kernel (small systems) against the force pass and
-the update as two:
-with velocity steps and with injected noise.  (A system whose displacement tracker has
-been started runs the two kernels.)"""
+the update as two: the same bits, at the edges of a warp's eight particles and of the
+sizes it takes, with velocity steps and with injected noise.  (A system whose displacement
+tracker has been started runs the two kernels.)"""
 import numpy as np
 import pytest
 
