@@ -31,16 +31,19 @@ struct ComboPair {  // AO + LJ(n) summed; each part inside its own cutoff
 
 // F(r)/r of a pair at r^2 in FP64: a functor's own fr64(r2, size, size^2) of
 // 1/r or 1/r^2 (rsqrt64 / rcp64) with fused multiply-adds, or fnet64 / r for a
-// functor that has only that (a plugin's, the composite), which may test r or
+// functor without one (a plugin's, the composite), which may test r or
 // r^2 against distances of its own and so gets them as the reference rounds
 // them: r is the square root by Markstein's correction of r2/sqrt(r2).
 // GB300 issues two FP64 operations a clock and SM, so the FP64 pass takes as
 // long as it has FP64 operations: sqrt, 1/r and fnet64 in the reference's order
 // were ~180 a pair, the LJ(6) form here is 12 and AO's 17.
+// A functor has an fr64 of its own where its Fr64 names the functor itself: one
+// derived from a library functor, with a force of its own, inherits both and is
+// asked for that force.
 template <class P, class = void>
 struct HasFr64 : std::false_type {};
 template <class P>
-struct HasFr64<P, decltype((void)&P::fr64)> : std::true_type {};
+struct HasFr64<P, std::void_t<typename P::Fr64>> : std::is_same<typename P::Fr64, P> {};
 template <class P>
 __device__ __forceinline__ double pair_fr64(const P& p, double r2, double size, double s2) {
     if constexpr (HasFr64<P>::value) {

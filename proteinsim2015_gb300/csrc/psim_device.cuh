@@ -384,6 +384,7 @@ struct AOPair {
         return -f;
     }
     // F(r)/r for the FP64 passes (see pair_fr64)
+    using Fr64 = AOPair;
     __device__ __forceinline__ double fr64(double r2, double, double) const {
         const double ri = rsqrt64(r2);
         const double i2 = __dmul_rn(ri, ri), i4 = __dmul_rn(i2, i2), i8 = __dmul_rn(i4, i4),
@@ -436,6 +437,7 @@ struct LJPair {
         return __dmul_rn(a, i2);
     }
     // an even exponent without a Yukawa term needs 1/r^2 alone
+    using Fr64 = LJPair;
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
         if ((n & 1) == 0 && pure) {
             const double i2 = rcp64(r2);
@@ -472,6 +474,7 @@ struct CalPair {
         return -(36.0 * (pow36(rinv) * rinv));
     }
     // F(r)/r = -36 r^-38 for the FP64 passes (see pair_fr64)
+    using Fr64 = CalPair;
     __device__ __forceinline__ double fr64(double r2, double, double) const {
         const double i2 = rcp64(r2), i4 = __dmul_rn(i2, i2), i8 = __dmul_rn(i4, i4),
                      i16 = __dmul_rn(i8, i8);

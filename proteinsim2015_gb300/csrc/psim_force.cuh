@@ -592,6 +592,7 @@ struct LJFixed : LJPair {
         return -kTwd * (attract + repel);
     }
     // LJPair::fr64's operations with the exponent unrolled
+    using Fr64 = LJFixed;
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
         if (N % 2 == 0 && pure) {
             const double i2 = rcp64(r2);
@@ -618,6 +619,7 @@ struct LJFixed : LJPair {
 template <int N>
 struct LJPure : LJPair {
     static_assert(N > 0 && N % 2 == 0, "an even, positive exponent");
+    using Fr64 = LJPure;
     __device__ __forceinline__ double fr64(double r2, double, double s2) const {
         const double i2 = rcp64(r2);
         return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));

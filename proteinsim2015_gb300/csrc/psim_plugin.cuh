@@ -15,7 +15,9 @@
 //       __host__ __device__ double fnet64(r2, r, 1/r, size)   F(r) in FP64
 //       __device__ float fnet32(r2, r, 1/r, size)              F(r) in FP32
 //     where F(r) is the reference's fNet: positive attracts, and the pair
-//     term on i is F(r) times the unit vector from i to j;
+//     term on i is F(r) times the unit vector from i to j.  It may derive from
+//     one of the library's functors (psim_device.cuh) and give its own fnet64
+//     and fnet32: both passes then call those;
 //   * its force class, deriving from psim::PluginForce<Class, Pair>: a
 //     constructor from PSim::config* that fills params_ (kind
 //     PSIM_FORCE_PLUGIN, the cutoff, any values in params_.user) and sets
