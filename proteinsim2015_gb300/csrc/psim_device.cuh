@@ -375,7 +375,6 @@ __host__ __device__ __forceinline__ T pow36(T rinv) {
 struct AOPair {
     double rc2, c1, c2;
     float rc2f, c1f, c2f;
-    double rc, e37;   // the cutoff and rc^-37 (u64)
     static constexpr bool kCheckNan = true;
     __host__ __device__ __forceinline__ double fnet64(double r2, double r, double rinv, double) const {
         double r36 = pow36(rinv);
@@ -401,6 +400,12 @@ struct AOPair {
     // the pair energy whose derivative is fnet64 (u' = fNet), zero at the
     // cutoff: 36/37 (r^-37 - rc^-37) + coEff1 ln(rc/r) + coEff2 (rc^2 - r^2)/2
     __host__ __device__ __forceinline__ double u64(double r2, double, double rinv, double) const {
+        const double rc = sqrt(rc2), rcinv = 1.0 / rc;
+        return u64_at(r2, rinv, rc, pow36(rcinv) * rcinv);
+    }
+    // with the cutoff and rc^-37 in hand
+    __host__ __device__ __forceinline__ double u64_at(double r2, double rinv, double rc,
+                                                      double e37) const {
         return (36.0 / 37.0) * (pow36(rinv) * rinv - e37) + c1 * log(rc * rinv) +
                0.5 * c2 * (rc2 - r2);
     }
@@ -412,8 +417,6 @@ struct LJPair {
     double rc2, kTwd, four_n, yuk, lambda, inv_lambda;
     float rc2f, kTwdf, four_nf, yukf, lambdaf, inv_lambdaf;
     int n;
-    int pure;   // no Yukawa term
-    double c64; // -kTwd four_n
     static constexpr bool kCheckNan = false;
     __host__ __device__ __forceinline__ double fnet64(double r2, double r, double rinv, double size) const {
         double lj = powi_binary(size * rinv, n);
@@ -426,10 +429,15 @@ struct LJPair {
         }
         return -kTwd * (attract + repel);
     }
+    // whether there is no Yukawa term, by the bits of yuk (a comparison of doubles is an
+    // operation of the FP64 unit)
+    __device__ __forceinline__ bool pure() const {
+        return (__double_as_longlong(yuk) & 0x7fffffffffffffffll) == 0;
+    }
     // F(r)/r with the Yukawa term at 1/r = ri and L = lj (see pair_fr64)
     __device__ __forceinline__ double fr64_of(double r2, double ri, double i2, double lj) const {
-        double a = __dmul_rn(__dmul_rn(c64, lj), __fma_rn(2.0, lj, -1.0));
-        if (!pure) {
+        double a = __dmul_rn(__dmul_rn(-__dmul_rn(kTwd, four_n), lj), __fma_rn(2.0, lj, -1.0));
+        if (!pure()) {
             const double r = __dmul_rn(r2, ri);
             const double e = exp(-1.0 * (r * inv_lambda));
             a = __fma_rn(-__dmul_rn(kTwd, yuk), __dmul_rn(e, __dmul_rn(ri, __dadd_rn(lambda, r))), a);
@@ -439,7 +447,7 @@ struct LJPair {
     // an even exponent without a Yukawa term needs 1/r^2 alone
     using Fr64 = LJPair;
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
-        if ((n & 1) == 0 && pure) {
+        if ((n & 1) == 0 && pure()) {
             const double i2 = rcp64(r2);
             return fr64_of(r2, 0.0, i2, powi_binary(__dmul_rn(s2, i2), n / 2));
         }
@@ -503,8 +511,6 @@ inline AOPair make_ao_pair(double kT, double wd, double rc) {
     AOPair p{};
     ao_coeffs(kT, wd, rc, &p.c1, &p.c2);
     p.rc2 = rc * rc;
-    p.rc = rc;
-    p.e37 = pow36(1.0 / rc) * (1.0 / rc);
     p.rc2f = (float)p.rc2;
     p.c1f = (float)p.c1;
     p.c2f = (float)p.c2;
@@ -517,8 +523,6 @@ inline LJPair make_lj_pair(double kT, double wd, int n, double yuk, double lambd
     p.n = n;
     p.four_n = 4.0 * n;
     p.yuk = yuk;
-    p.pure = yuk == 0.0;
-    p.c64 = -p.kTwd * p.four_n;
     p.lambda = lambda;
     p.inv_lambda = 1.0 / lambda;
     p.rc2f = (float)p.rc2;

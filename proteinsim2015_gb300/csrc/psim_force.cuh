@@ -594,7 +594,7 @@ struct LJFixed : LJPair {
     // LJPair::fr64's operations with the exponent unrolled
     using Fr64 = LJFixed;
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
-        if (N % 2 == 0 && pure) {
+        if (N % 2 == 0 && pure()) {
             const double i2 = rcp64(r2);
             return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));
         }

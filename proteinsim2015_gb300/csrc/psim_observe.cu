@@ -12,6 +12,7 @@
 // Sums are deterministic: each block writes its partial, one block adds the
 // partials in block order.
 #include <algorithm>
+#include <cmath>
 
 #include "psim_force.cuh"
 
@@ -264,6 +265,16 @@ __global__ void __launch_bounds__(256) uf_final_kernel(int n, const int* label, 
 }
 
 // ------------------------------------------------------ energy and virial
+// AO with its cutoff's constants, formed once for all pairs.
+struct AOEnergy : AOPair {
+    double rc, e37;
+    explicit AOEnergy(const AOPair& p) : AOPair(p), rc(std::sqrt(p.rc2)) {
+        e37 = pow36(1.0 / rc) * (1.0 / rc);
+    }
+    __device__ __forceinline__ double u64(double r2, double, double rinv, double) const {
+        return u64_at(r2, rinv, rc, e37);
+    }
+};
 // One pair term of the energy walk: u(r) and fNet(r) inside the cutoff.
 template <class Pair>
 struct OneTerm {
@@ -278,7 +289,7 @@ struct OneTerm {
     }
 };
 struct ComboTerms {  // the AO + LJ(n) composite: each part inside its own cutoff
-    AOPair ao;
+    AOEnergy ao;
     LJPair lj;
     __device__ double rc2() const { return ao.rc2 > lj.rc2 ? ao.rc2 : lj.rc2; }
     __device__ void eval(double r2, double r, double rinv, double size, double& u,
@@ -374,10 +385,10 @@ cudaError_t launch_energy(const ForceSetup& fs, const PairScanArgs& a, double* s
                           double* out, cudaStream_t st) {
     if (a.g.n == 0) return cudaMemsetAsync(out, 0, 2 * sizeof(double), st);
     switch (fs.kind) {
-    case 1: return run_energy(OneTerm<AOPair>{fs.ao}, a, scratch, out, st);
+    case 1: return run_energy(OneTerm<AOEnergy>{AOEnergy(fs.ao)}, a, scratch, out, st);
     case 2: return run_energy(OneTerm<LJPair>{fs.lj}, a, scratch, out, st);
     case 3: return run_energy(OneTerm<CalPair>{fs.cal}, a, scratch, out, st);
-    case 4: return run_energy(ComboTerms{fs.ao, fs.lj}, a, scratch, out, st);
+    case 4: return run_energy(ComboTerms{AOEnergy(fs.ao), fs.lj}, a, scratch, out, st);
     }
     return cudaErrorInvalidValue;
 }

@@ -44,3 +44,10 @@ def check(psim, plugin_so, settings, lj_num, yukawa):
 @pytest.mark.parametrize("lj_num", [6, 7])
 def test_derived_functor_keeps_its_own_force(psim, plugin_so, lj_num):
     check(psim, plugin_so, dict(variant=0, ljNum=lj_num, yukawaStrength=3.0), 0, 3.0)
+
+
+@pytest.mark.parametrize("variant", [1, 2])
+@pytest.mark.parametrize("lj_num,yukawa", [(6, 3.0), (7, 3.0), (6, 0.0)])
+def test_functor_filled_by_the_plugin(psim, plugin_so, variant, lj_num, yukawa):
+    check(psim, plugin_so, dict(variant=variant, ljNum=lj_num, yukawaStrength=yukawa), lj_num,
+          yukawa)
