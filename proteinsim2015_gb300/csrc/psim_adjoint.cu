@@ -929,15 +929,23 @@ int add_hist(psim_adjoint* a, const AdjWalk& w) {
     const bool shared = a->cfg.n_bins <= kAdjHistBins;
     const size_t smem = shared ? 8 * (size_t)a->cfg.n_bins : 0;
     double* out = shared ? a->hpart.as<double>() : a->hsum.as<double>();
+    cudaError_t e = cudaSuccess;
     with_lanes(a, [&](auto g) {
         constexpr int G = decltype(g)::value;
-        if (shared)
-            adj_hist_kernel<G, true><<<b, threads, smem, a->st>>>(w, a->walk_rc2, a->hist, scale,
-                                                                  out);
-        else
+        if (!shared) {
             adj_hist_kernel<G, false><<<b, threads, 0, a->st>>>(w, a->walk_rc2, a->hist, scale,
                                                                 out);
+            return;
+        }
+        // with the queues (25600 bytes at four lanes a particle) the most bins take more
+        // than the 48 KB a kernel has without asking
+        e = cudaFuncSetAttribute(adj_hist_kernel<G, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kAdjHistBins);
+        if (e == cudaSuccess)
+            adj_hist_kernel<G, true><<<b, threads, smem, a->st>>>(w, a->walk_rc2, a->hist, scale,
+                                                                  out);
     });
+    ADJ_CUDA(e);
     ADJ_CUDA(cudaGetLastError());
     return PSIM_OK;
 }
