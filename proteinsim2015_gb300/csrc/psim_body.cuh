@@ -124,11 +124,12 @@ struct F64Body {
                               : r2_exact(d0, d1, d2);
         // updateInteractions' test: r = sqrt(pbcDist) < 1.2 (systemHandling.cpp:112-115)
         if (count && sqrt(r2_exact(d0, d1, d2)) < cont) ++a.cnt;
-        // r^2 < rc^2 by the high words (a NaN is above); where they are equal, or
-        // r^2's is one less, the reference's r^2 decides
+        // r^2 < rc^2 by the high words (a NaN is above); where they differ by no more than
+        // one, either way, the reference's r^2 decides: rounded otherwise, it can lie on the
+        // other side of a change of the high word
         const int hr = __double2hiint(r2), hc = __double2hiint(pf.rc2);
         bool in = hr < hc;
-        if ((unsigned)(hc - hr) <= 1u) {
+        if ((unsigned)(hc - hr + 1) <= 2u) {
             asm volatile("" : "+d"(d0));
             in = r2_exact(d0, d1, d2) < pf.rc2;
         }
