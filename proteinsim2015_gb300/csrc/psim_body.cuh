@@ -63,8 +63,9 @@ __device__ __forceinline__ double pair_fr64(const P& p, double r2, double size, 
 // on the bit patterns as integers, which order like the non-negative values, and
 // the exact ones only next to a threshold; the force itself is pair_fr64 on an
 // r^2 summed with fused multiply-adds.  The image that unitVectorAdv takes by
-// |dx| > int(L)/2 (utilities.cpp:114-142) is the same one for a pair in range:
-// its |dx| is below rc or above L - rc, and rc <= cellSize <= L/3 <= int(L)/2.
+// |dx| > int(L)/2 (utilities.cpp:114-142) is the same one for a pair in range
+// where rc <= int(L)/2: its |dx| is below rc or above L - rc.  With
+// rc <= cellSize <= L/3 that leaves a box of edge 1, whose int(L)/2 is 0 (unit_box).
 template <class Pair>
 struct F64Body {
     Pair pf;
@@ -112,7 +113,11 @@ struct F64Body {
                                          Acc& a, uint32_t& err) const {
         const DevGeom& g = geom;
         double d0 = pj.x - h.p.x, d1 = pj.y - h.p.y, d2 = pj.z - h.p.z;
+        int moved = 0;   // the axes that pbcDist's image moved
         if (abs_above(d0, g.half) | abs_above(d1, g.half) | abs_above(d2, g.half)) {
+            if (unit_box())
+                moved = (abs_above(d0, g.half) ? 1 : 0) | (abs_above(d1, g.half) ? 2 : 0) |
+                        (abs_above(d2, g.half) ? 4 : 0);
             // keeps the compiler from doing the additions for every pair
             asm volatile("" : "+d"(d0), "+d"(d1), "+d"(d2));
             if (abs_above(d0, g.half)) d0 += toward(g.L, d0);
@@ -147,6 +152,11 @@ struct F64Body {
             if (Pair::kCheckNan &&
                 (__double_as_longlong(f) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll)
                 err |= EBIT_NAN;
+            if (unit_box()) {
+                if (!(moved & 1)) d0 = unit_image(d0);
+                if (!(moved & 2)) d1 = unit_image(d1);
+                if (!(moved & 4)) d2 = unit_image(d2);
+            }
             a.n0 = __fma_rn(f, d0, a.n0);
             a.n1 = __fma_rn(f, d1, a.n1);
             a.n2 = __fma_rn(f, d2, a.n2);
@@ -155,6 +165,14 @@ struct F64Body {
     __device__ __forceinline__ void eval_quad(int, const double4_32a& pj, const Home& h, Acc& a,
                                               uint32_t& err) const {
         eval(make_float4(0.f, 0.f, 0.f, 0.f), pj, h, a, err);
+    }
+    // A box of edge 1 (half_uv is 0), where unitVectorAdv may take another image.
+    __device__ __forceinline__ bool unit_box() const { return __double2hiint(geom.half_uv) == 0; }
+    // unitVectorAdv's image of a difference that pbcDist leaves as it is (one that
+    // pbcDist moves, it moves alike)
+    __device__ __forceinline__ double unit_image(double d) const {
+        if (fabs(d) > geom.half_uv) d = d < 0.0 ? d + geom.L : d - geom.L;
+        return d;
     }
     // L for d < 0, else -L
     static __device__ __forceinline__ double toward(double L, double d) {

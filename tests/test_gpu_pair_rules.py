@@ -1,5 +1,6 @@
 """The FP64 pass where the reference's own rules decide a pair in ways that a shorter
-form of them would not: an r^2 whose rounding changes its high word at the cutoff."""
+form of them would not: an r^2 whose rounding changes its high word at the cutoff, and
+the unit vector's image in a box of edge 1."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,19 @@ def test_cutoff_below_a_high_word(psim, force_pass, k):
     assert (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2] < rc * rc
     p = psim.make_force("LJ", rc, kT=1.0, well_depth=1.0, lj_num=6, yukawa_strength=0.0)
     check(psim, psim.geometry(2, 12.0, 3.0, 4), p, np.array([0.0, 0.0, 0.0] + d), np.full(2, 0.5))
+
+
+@pytest.mark.parametrize("kind", ["LJ6", "LJ9Y", "CAL"])
+@pytest.mark.parametrize("box", [1.0, 2.0, 3.0])
+def test_unit_vector_in_a_box_of_edge_1(psim, force_pass, kind, box):
+    # |d| > int(L)/2 is |d| > 0 in a box of edge 1: the reference's unit vector then
+    # points to another image than the one r^2 was taken of
+    p = {"LJ6": lambda rc: psim.make_force("LJ", rc, kT=1.0, well_depth=1.0, lj_num=6,
+                                           yukawa_strength=0.0),
+         "LJ9Y": lambda rc: psim.make_force("LJ", rc, kT=1.0, well_depth=0.5, lj_num=9,
+                                            yukawa_strength=1.0, debye_length=0.1),
+         "CAL": lambda rc: psim.make_force("CAL", rc)}[kind](0.3 * box)
+    rng = np.random.default_rng(0)
+    i = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = np.mod(((i + 0.5) * 0.2 + rng.uniform(-0.04, 0.04, i.shape)) * box, box).reshape(-1)
+    check(psim, psim.geometry(125, box, box / 3, 3), p, pos, np.full(125, 0.05 * box))
