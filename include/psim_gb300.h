@@ -306,6 +306,10 @@ int psim_integrator_next_system(psim_integrator* integ, double current_time, dou
 
 /* --------------------------------------------- device-resident system */
 
+/* Calls that read a system's state (downloads, forces, observables) may come
+ * from several threads at once: they take turns.  Uploads, steps and settings
+ * belong to one thread at a time, with no other call on the system beside
+ * them.  Different systems share nothing. */
 typedef struct psim_system psim_system;
 
 typedef struct {

@@ -460,10 +460,11 @@ struct ScopedBuf : DevBuf {
 
 // Device scratch of one host-facing call, in the owner's buffer: a cudaMalloc and
 // cudaFree pair costs ~100 us, more than most of what these calls run.  The
-// buffer is kept for the next call up to kKeep bytes and goes with its owner.
+// buffer is kept for the next call up to kKeep bytes and goes with its owner.  It is
+// the call's alone while it lives (mu): another thread's call on the same owner waits.
 class Scratch {
 public:
-    explicit Scratch(DevBuf& b) : buf_(b) {}
+    Scratch(DevBuf& b, std::recursive_mutex& mu) : lock_(mu), buf_(b) {}
     ~Scratch() {
         if (buf_.bytes > kKeep) buf_.release();
     }
@@ -482,6 +483,7 @@ public:
 
 private:
     static constexpr size_t kKeep = (size_t)256 << 20;
+    std::lock_guard<std::recursive_mutex> lock_;
     DevBuf& buf_;
     std::vector<size_t> off_;
 };
@@ -1278,6 +1280,7 @@ struct psim_system {
     DevBuf img, track_start;
     DevBuf obs;               // scratch of the host-facing calls (Scratch)
     uint32_t* host = nullptr; // pinned: the step state and the error word (settle)
+    std::recursive_mutex mu;  // of the two, and of the cell view that cell_refs makes
 };
 
 namespace {
@@ -1769,6 +1772,7 @@ struct DeviceGuard {
 // Waits for the stream, reads the error word and the device step counter,
 // and re-aligns the host's step count with the steps the device completed.
 int settle(psim_system* s) {
+    std::lock_guard<std::recursive_mutex> lk(s->mu);
     PSIM_CUDA(cudaMemcpyAsync(s->host, s->state.p, sizeof(StepState), cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaMemcpyAsync(s->host + 8, s->err.p, 4, cudaMemcpyDeviceToHost, s->st));
     PSIM_CUDA(cudaStreamSynchronize(s->st));
@@ -2403,7 +2407,7 @@ int psim_system_download(psim_system* s, double* pos, double* pos0, double* vel,
     cudaStream_t st = s->st;
     // storage order is the previous cell order: its tags are tag[1 - ob]
     const int* tg = store_tags(s);
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({b}));
     double* stage = mem.at<double>(0);
     auto get3 = [&](DevBuf& src, const int* perm, double* dst) -> int {
@@ -2436,7 +2440,7 @@ int psim_system_download_cells(psim_system* s, int32_t* hash_index, uint32_t* cs
     const Phase ph = phase_of(s->total);
     const int n = s->n;
     cudaStream_t st = s->st;
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({8 * (size_t)n, 8 * (size_t)s->ncell, 32 * (size_t)n, 32 * (size_t)n}));
     int32_t* hb = mem.at<int32_t>(0);
     uint32_t* cb = mem.at<uint32_t>(1);
@@ -2509,7 +2513,7 @@ int psim_system_forces(psim_system* s, double* force) {
     if (rc) return rc;
     const Phase ph = phase_of(s->total);
     const int n = s->n;
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({24 * (size_t)n, 24 * (size_t)n}));
     double *f3 = mem.at<double>(0), *out = mem.at<double>(1);
     ForceOut fo{f3, f3 + n, f3 + 2 * (size_t)n, s->err.as<uint32_t>(), nullptr};
@@ -2547,7 +2551,7 @@ int reduce(psim_system* s, ObserveArgs& a, double* out) {
     a.perm_prev = prev_perm(s);
     a.tag = store_tags(s);   // the storage order's tags (as download)
     a.L = s->g.L;
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({8 * (size_t)observe_scratch_doubles(), 8}));
     PSIM_CUDA(launch_observe(a, mem.at<double>(0), mem.at<double>(1), s->st));
     PSIM_CUDA(cudaMemcpyAsync(out, mem.at<double>(1), 8, cudaMemcpyDeviceToHost, s->st));
@@ -2590,7 +2594,7 @@ int psim_system_temperature(psim_system* s, double* kT) {
     if (rc) return rc;
     DeviceGuard dg(s->device);
     if ((rc = settle(s))) return rc;
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({8 * (size_t)observe_scratch_doubles(), 8}));
     PSIM_CUDA(launch_sum_squares(3LL * s->n, s->vel.as<double>(), mem.at<double>(0),
                                  mem.at<double>(1), s->st));
@@ -2671,7 +2675,7 @@ int psim_system_interactions(psim_system* s, double r_contact, int32_t* coor, in
     DeviceGuard dg(s->device);
     int rc = settle(s);
     if (rc) return rc;
-    Scratch mem(s->obs);   // counts, total, and forces or sorted positions
+    Scratch mem(s->obs, s->mu);   // counts, total, and forces or sorted positions
     PSIM_CUDA(mem.ensure({4 * (size_t)s->n, 8, 32 * (size_t)s->n}));
     int* cb = mem.at<int>(0);
     // updateInteractions fused into one force pass on the current state: the
@@ -2732,7 +2736,7 @@ int psim_system_clusters(psim_system* s, double r_contact, int32_t min_size, int
     int rc = settle(s);
     if (rc) return rc;
     const size_t n = (size_t)s->n;
-    Scratch mem(s->obs);   // positions, labels, roots, sizes and the error word
+    Scratch mem(s->obs, s->mu);   // positions, labels, roots, sizes and the error word
     PSIM_CUDA(mem.ensure({32 * n, 4 * n, 4 * n, 4 * n, 4}));
     int *lab = mem.at<int>(1), *rt = mem.at<int>(2), *sz = mem.at<int>(3);
     uint32_t* eb = mem.at<uint32_t>(4);
@@ -2771,7 +2775,7 @@ int psim_system_rdf(psim_system* s, double r_min, double r_max, int32_t n_bins, 
     DeviceGuard dg(s->device);
     int rc = settle(s);
     if (rc) return rc;
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({8 * (size_t)n_bins, 32 * (size_t)s->n}));
     unsigned long long* hb = mem.at<unsigned long long>(0);
     PSIM_CUDA(cudaMemsetAsync(hb, 0, 8 * (size_t)n_bins, s->st));
@@ -2820,7 +2824,7 @@ int psim_system_energy(psim_system* s, double* potential, double* virial) {
     int rc = settle(s);
     if (rc) return rc;
     PairScanArgs a{};
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({32 * (size_t)s->n, 8 * energy_scratch_doubles(s->n), 16}));
     if ((rc = sorted_view(s, mem.at<double4_32a>(0), max_cutoff(&s->cfg.force), a))) return rc;
     double* res = mem.at<double>(2);
@@ -2885,7 +2889,7 @@ int psim_system_cell_occupancy(psim_system* s, int32_t* max_occ, double* mean_oc
     DeviceGuard dg(s->device);
     int rc = settle(s);
     if (rc && rc != code_from_bits(s->latched)) return rc;
-    const Phase ph = phase_of(s->total);
+    std::lock_guard<std::recursive_mutex> lk(s->mu);
     PSIM_CUDA(cudaMemsetAsync(s->occ.p, 0, 4, s->st));
     CellRefs c;
     if ((rc = cell_refs(s, c))) return rc;
@@ -2924,7 +2928,7 @@ int psim_system_pair_count(psim_system* s, double cutoff, double* mean_pairs) {
     int rc = settle(s);
     if (rc) return rc;
     const Phase ph = phase_of(s->total);
-    Scratch mem(s->obs);
+    Scratch mem(s->obs, s->mu);
     PSIM_CUDA(mem.ensure({8, 16 * (size_t)s->n}));
     unsigned long long* tot = mem.at<unsigned long long>(0);
     float4* ph4 = mem.at<float4>(1);
