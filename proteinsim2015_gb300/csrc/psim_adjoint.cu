@@ -49,6 +49,7 @@
 #include <vector>
 
 #include "../../include/psim_gb300.h"
+#include "psim_exp.cuh"
 #include "psim_kernels.cuh"
 
 namespace psim {
@@ -63,32 +64,8 @@ struct AdjPair {
     double eps, sig, lj_rc2; // lj_rc2 = 0: no LJ(n) term
     int ljn;
     double eps4n, eps_n_sig; // 4n eps, n eps / sig
-    const double2* e2;       // 2^(k/256), k = 0 .. 255, and its rounding (exp_table)
+    const double2* e2;       // exp_table_values
 };
-
-// exp(x) by the table-driven method (Tang, "Table-driven implementation of the
-// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989):
-// x = (256 e + k) ln2/256 + r, e^x = 2^e 2^(k/256) (1 + r + r^2/2 + r^3/6 + r^4/24)
-// with |r| <= ln2/512, whose r^5/120 is below 2^-54; the table holds each value's
-// rounding too.  Eleven FP64 operations against exp()'s ~18, in passes that take as
-// long as they have FP64 operations; largest error 1.27 and rms 0.436 x 2^-53 of
-// the value (exp() 1.18 and 0.442) over 40000 x in [-14, 0] and [-690, 690].
-__device__ __forceinline__ double exp_table(double x, const double2* e2) {
-    if ((__double2hiint(x) & 0x7fffffff) >= 0x40859000) return exp(x);   // |x| >= 690, NaN
-    // rounding to an integer by adding 1.5 2^52, which leaves it in the low word
-    const double magic = 6755399441055744.0;
-    const double t = __fma_rn(x, 369.3299304675746271, magic);   // 256 / ln2
-    const double k = __dadd_rn(t, -magic);
-    const int n = __double2loint(t);
-    // ln2/256 in two parts, the first short enough for an exact product with k
-    double r = __fma_rn(k, -0x1.62e42fefap-9, x);
-    r = __fma_rn(k, -0x1.cf79abc9e3b3ap-48, r);
-    const double q = __fma_rn(r, __fma_rn(r, 1.0 / 24.0, 1.0 / 6.0), 0.5);
-    const double p = __fma_rn(__dmul_rn(r, r), q, r);
-    const double2 f = __ldg(e2 + (n & 255));
-    const double v = __dadd_rn(f.x, __fma_rn(f.x, p, f.y));
-    return __hiloint2double(__double2hiint(v) + ((n >> 8) << 20), __double2loint(v));
-}
 
 // r2 < rc2 on the bit patterns (a NaN is above), off the FP64 unit
 __device__ __forceinline__ bool below_rc(double r2, double rc2) {
@@ -1177,7 +1154,7 @@ psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device
               !a->lam[0].ensure(b3) && !a->lam[1].ensure(b3) && !a->lam[2].ensure(b3) &&
               !a->u[0].ensure(b4) && !a->u[1].ensure(b4) && !a->x0.ensure(b3) &&
               !a->part.ensure(8 * kAdjTh * threads) && !a->acc.ensure(8 * kAdjTh * (1 + kAdjRowBlocks)) &&
-              !a->e2.ensure(16 * 256) &&
+              !a->e2.ensure(16 * kExpTable) &&
               (cfg->n_bins > kAdjHistBins ||
                !a->hpart.ensure(8 * (size_t)cfg->n_bins * blocks_of(a, kAdjHistWarps))) &&
               !a->hsum.ensure(8 * (size_t)cfg->n_bins) && !a->wgt.ensure(8 * (size_t)cfg->n_bins);
@@ -1197,12 +1174,8 @@ psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device
         a->K = a->K > asked ? asked : std::max(2, a->K / 2);
     }
     if (ok) {
-        double2 e2[256];
-        for (int k = 0; k < 256; ++k) {
-            const long double v = exp2l(k / 256.0L);
-            e2[k].x = (double)v;
-            e2[k].y = (double)(v - (long double)e2[k].x);
-        }
+        double2 e2[kExpTable];
+        exp_table_values(e2);
         ok = cudaMemcpy(a->e2.p, e2, sizeof e2, cudaMemcpyHostToDevice) == cudaSuccess;
     }
     if (!ok) {

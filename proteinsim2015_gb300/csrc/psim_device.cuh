@@ -156,8 +156,10 @@ __device__ __forceinline__ T load_as(const T* p) {
 // 1/a and 1/sqrt(a) to about an ulp in 3 and 5 FP64 operations, from the
 // hardware's ~20-bit seeds (rcp.approx / rsqrt.approx, not on the FP64 unit) and
 // one third-order Householder iteration: with h = 1 - a y (1 - a y^2) the seed's
-// relative error e becomes e^3, below the rounding of the last operation.  a
-// positive and normal; 0 gives a NaN.
+// relative error e becomes e^3, below the rounding of the last operation.  Largest and
+// rms error over 2^20 a of any exponent, x 2^-53 of the value: 1.00 and 0.425, 1.24 and
+// 0.475 (CUDA's 1/a the same, 1/sqrt(a) 1.50 and 0.601).  a positive and normal; 0 gives
+// a NaN.
 __device__ __forceinline__ double rcp64(double a) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
