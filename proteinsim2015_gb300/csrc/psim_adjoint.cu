@@ -557,7 +557,7 @@ adj_hist_kernel(AdjWalk w, double rc2, AdjHist h, double scale, double* part) {
     const double unit = h.dr * scale;
     for_pairs<G>(w, rc2, i, active, lane, xi, sq[wid][lane / G],
                  [&](int, const double*, double r2) {
-                     gauss_bins(h, __dmul_rn(r2, rsqrt64(r2)), kShared ? unit : h.dr, w.q.e2,
+                     gauss_bins(h, sqrt64(r2, rsqrt64(r2)), kShared ? unit : h.dr, w.q.e2,
                                 [&](int b, double, double v) {
                                     if (kShared)
                                         atomicAdd(&bins[b],
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adj_reverse_kernel(AdjWalk w, 
         if (a.wgt) {
             // d/dx_i of the smoothed counts of pairs (i, j) and (j, i)
             double wr = 0.0;
-            gauss_bins(a.h, __dmul_rn(r2, ri), 1.0, w.q.e2,
+            gauss_bins(a.h, sqrt64(r2, ri), 1.0, w.q.e2,
                        [&](int b, double z, double G_) { wr = __fma_rn(a.wgt[b] * G_, z, wr); });
             wr *= 2.0 * a.h.dr * a.h.inv_sig * ri;
 #pragma unroll

@@ -33,7 +33,7 @@ struct ComboPair {  // AO + LJ(n) summed; each part inside its own cutoff
 // 1/r or 1/r^2 (rsqrt64 / rcp64) with fused multiply-adds, or fnet64 / r for a
 // functor without one (a plugin's, the composite), which may test r or
 // r^2 against distances of its own and so gets them as the reference rounds
-// them: r is the square root by Markstein's correction of r2/sqrt(r2).
+// them (sqrt64).
 // GB300 issues two FP64 operations a clock and SM, so the FP64 pass takes as
 // long as it has FP64 operations: sqrt, 1/r and fnet64 in the reference's order
 // were ~180 a pair, the LJ(6) form here is 12 and AO's 17.
@@ -50,9 +50,7 @@ __device__ __forceinline__ double pair_fr64(const P& p, double r2, double size, 
         return p.fr64(r2, size, s2);
     } else {
         const double ri = rsqrt64(r2);
-        double r = __dmul_rn(r2, ri);
-        r = __fma_rn(__dmul_rn(0.5, ri), __fma_rn(-r, r, r2), r);
-        return __dmul_rn(p.fnet64(r2, r, ri, size), ri);
+        return __dmul_rn(p.fnet64(r2, sqrt64(r2, ri), ri, size), ri);
     }
 }
 

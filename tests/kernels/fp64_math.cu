@@ -1,4 +1,4 @@
-// fp64_math.cu -- the FP64 passes' own 1/a, 1/sqrt(a) and exp(x) beside CUDA's, for the
+// fp64_math.cu -- the FP64 passes' own 1/a, 1/sqrt(a), sqrt(a) and exp(x) beside CUDA's, for the
 // tests: run(what, n, in, out), host arrays.
 #include <cuda_runtime.h>
 
@@ -7,7 +7,7 @@
 
 namespace {
 
-enum { RCP, RCP_CUDA, RSQRT, RSQRT_CUDA, EXP, EXP_CUDA };
+enum { RCP, RCP_CUDA, RSQRT, RSQRT_CUDA, EXP, EXP_CUDA, SQRT };
 
 __global__ void eval(int what, int n, const double* in, double* out, const double2* e2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -20,6 +20,7 @@ __global__ void eval(int what, int n, const double* in, double* out, const doubl
     case RSQRT_CUDA: out[i] = 1.0 / sqrt(a); break;
     case EXP: out[i] = psim::exp_table(a, e2); break;
     case EXP_CUDA: out[i] = exp(a); break;
+    case SQRT: out[i] = psim::sqrt64(a, psim::rsqrt64(a)); break;
     }
 }
 

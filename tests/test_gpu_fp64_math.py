@@ -1,4 +1,4 @@
-"""The FP64 passes' own 1/a, 1/sqrt(a) and exp(x) against extended precision and beside
+"""The FP64 passes' own 1/a, 1/sqrt(a), sqrt(a) and exp(x) against extended precision and beside
 CUDA's, over the ranges of their arguments, in units of 2^-53 of the value.
 
 Bounds.  The last operation of each rounds once: at most 1, and 0.4247 in the mean square
@@ -80,3 +80,10 @@ def test_exp_edges(run):
                   np.nan, 1e-300, -1e-300, 5e-324])
     ours, cuda = run(4, x), run(5, x)
     assert np.array_equal(ours, cuda, equal_nan=True)
+
+
+@pytest.mark.parametrize("lo,hi", [(-14, 14), (-1000, 1000)])
+def test_sqrt_is_correctly_rounded(run, lo, hi):
+    rng = np.random.default_rng(12)
+    x = np.ldexp(2.0 ** rng.uniform(0.0, 1.0, N), rng.integers(lo, hi, N).astype(np.int32))
+    assert np.array_equal(run(6, x), np.sqrt(x))
