@@ -250,6 +250,7 @@ ForceSetup make_setup(const psim_force_params* p, double L) {
     fs.rc_max = max_cutoff(p);
     fs.pre_rc2f = prefilter_r2(fs.rc_max, L);
     fs.lj_pure = p->kind == PSIM_FORCE_LJ && p->yukawa_strength == 0.0;
+    fs.unit_box = L == 1.0;
     return fs;
 }
 
@@ -1653,7 +1654,7 @@ bool fused_steps(const psim_system* s) {
     if (s->n_reps) return false;
     if (s->cfg.precision == PSIM_PRECISION_MIXED)
         return s->n <= kStepDirect && step_direct_fits(s->fs, s->g);
-    return !s->fs.tile && s->n <= kStep64 && one_order(s);
+    return !s->fs.tile && !s->fs.unit_box && s->n <= kStep64 && one_order(s);
 }
 // The velocity counter's period: step t > 0 writes the velocities when it
 // divides t; step 0 is the first step.
@@ -1990,6 +1991,7 @@ psim_system* psim_batch_create_list(const psim_replica* reps, int32_t n_reps,
         for (int i = g.p0; i < g.p1; ++i) rep[(size_t)i] = r;
         const ForceSetup fr = make_setup(&reps[r].force, g.L);
         s->fs.lj_pure = s->fs.lj_pure && fr.lj_pure;
+        s->fs.unit_box = s->fs.unit_box || fr.unit_box;
         pre[(size_t)r] = fr.pre_rc2f;
         seeds[(size_t)r] = (uint32_t)reps[r].seed;
         const void* src = kind == PSIM_FORCE_AO ? (const void*)&fr.ao

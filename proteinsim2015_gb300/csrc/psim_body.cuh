@@ -63,13 +63,15 @@ __device__ __forceinline__ double pair_fr64(const P& p, double r2, double size, 
 // r^2 summed with fused multiply-adds.  The image that unitVectorAdv takes by
 // |dx| > int(L)/2 (utilities.cpp:114-142) is the same one for a pair in range
 // where rc <= int(L)/2: its |dx| is below rc or above L - rc.  With
-// rc <= cellSize <= L/3 that leaves a box of edge 1, whose int(L)/2 is 0 (unit_box).
-template <class Pair>
+// rc <= cellSize <= L/3 that leaves a box of edge 1, whose int(L)/2 is 0: kUnitBox (a
+// test per pair in every box costs a step of 4000 LJ particles 4 to 7%).
+template <class Pair, bool kUnitBox = false>
 struct F64Body {
     Pair pf;
     using Aux = double4_32a;  // the FP64 neighbour positions {x, y, z, R}
     static constexpr bool kBatchable = !std::is_same<Pair, ComboPair>::value;
     static constexpr bool kQuadWalk = true;   // force_quad_kernel
+    static constexpr bool kUnit = kUnitBox;
     struct Home {
         double4_32a p;
         double size, s2;      // contact diameter with a neighbour of the same radius, squared
@@ -113,7 +115,7 @@ struct F64Body {
         double d0 = pj.x - h.p.x, d1 = pj.y - h.p.y, d2 = pj.z - h.p.z;
         int moved = 0;   // the axes that pbcDist's image moved
         if (abs_above(d0, g.half) | abs_above(d1, g.half) | abs_above(d2, g.half)) {
-            if (unit_box())
+            if (kUnitBox && unit_box())
                 moved = (abs_above(d0, g.half) ? 1 : 0) | (abs_above(d1, g.half) ? 2 : 0) |
                         (abs_above(d2, g.half) ? 4 : 0);
             // keeps the compiler from doing the additions for every pair
@@ -150,7 +152,7 @@ struct F64Body {
             if (Pair::kCheckNan &&
                 (__double_as_longlong(f) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll)
                 err |= EBIT_NAN;
-            if (unit_box()) {
+            if (kUnitBox && unit_box()) {
                 if (!(moved & 1)) d0 = unit_image(d0);
                 if (!(moved & 2)) d1 = unit_image(d1);
                 if (!(moved & 4)) d2 = unit_image(d2);
@@ -164,7 +166,8 @@ struct F64Body {
                                               uint32_t& err) const {
         eval(make_float4(0.f, 0.f, 0.f, 0.f), pj, h, a, err);
     }
-    // A box of edge 1 (half_uv is 0), where unitVectorAdv may take another image.
+    // A box of edge 1 (half_uv is 0), where unitVectorAdv may take another image (a batch's
+    // replicas differ).
     __device__ __forceinline__ bool unit_box() const { return __double2hiint(geom.half_uv) == 0; }
     // unitVectorAdv's image of a difference that pbcDist leaves as it is (one that
     // pbcDist moves, it moves alike)

@@ -443,9 +443,13 @@ struct LJPair {
     __device__ __forceinline__ bool pure() const {
         return (__double_as_longlong(yuk) & 0x7fffffffffffffffll) == 0;
     }
+    // r F(r) without the Yukawa term at L = lj
+    __device__ __forceinline__ double fr64_lj(double lj) const {
+        return __dmul_rn(__dmul_rn(-__dmul_rn(kTwd, four_n), lj), __fma_rn(2.0, lj, -1.0));
+    }
     // F(r)/r with the Yukawa term at 1/r = ri and L = lj (see pair_fr64)
     __device__ __forceinline__ double fr64_of(double r2, double ri, double i2, double lj) const {
-        double a = __dmul_rn(__dmul_rn(-__dmul_rn(kTwd, four_n), lj), __fma_rn(2.0, lj, -1.0));
+        double a = fr64_lj(lj);
         if (!pure()) {
             // r carries ri's error, which the three factors of 1/r take back in part: rms
             // error of the term at r of 0.8 to 3, x 2^-53, so and with the rounded sqrt and
@@ -461,7 +465,7 @@ struct LJPair {
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
         if ((n & 1) == 0 && pure()) {
             const double i2 = rcp64(r2);
-            return fr64_of(r2, 0.0, i2, powi_binary(__dmul_rn(s2, i2), n / 2));
+            return __dmul_rn(fr64_lj(powi_binary(__dmul_rn(s2, i2), n / 2)), i2);
         }
         const double ri = rsqrt64(r2);
         return fr64_of(r2, ri, __dmul_rn(ri, ri), powi_binary(__dmul_rn(size, ri), n));

@@ -23,43 +23,43 @@ namespace psim {
 
 template <class Pair>
 static cudaError_t run_fp64(const Pair& p, const DevGeom& g, const CellView& cv,
-                            const ForceOut& out, float pre, cudaStream_t st, int tile,
+                            const ForceOut& out, const ForceSetup& fs, cudaStream_t st,
                             const BatchView* bv) {
-    F64Body<Pair> body{p, g};
-    body.count = out.coor && out.cont > 0.0;   // updateInteractions fused into the pass
-    body.cont = out.cont;
-    if (tile && !bv) return launch_force_cells(body, g, cv, out, pre, st);
-    return launch_force_pass(body, g, cv, out, pre, st, bv);
+    auto run = [&](auto body) {
+        body.count = out.coor && out.cont > 0.0;   // updateInteractions fused into the pass
+        body.cont = out.cont;
+        if constexpr (!decltype(body)::kUnit)
+            if (fs.tile && !bv) return launch_force_cells(body, g, cv, out, fs.pre_rc2f, st);
+        return launch_force_pass(body, g, cv, out, fs.pre_rc2f, st, bv);
+    };
+    return fs.unit_box ? run(F64Body<Pair, true>{p, g}) : run(F64Body<Pair>{p, g});
 }
 
 template <int N>
-static cudaError_t run_lj_fp64(const LJPair& lj, const DevGeom& g, const CellView& cv,
-                               const ForceOut& out, float pre, cudaStream_t st, int tile,
-                               const BatchView* bv) {
+static cudaError_t run_lj_fp64(const DevGeom& g, const CellView& cv, const ForceOut& out,
+                               const ForceSetup& fs, cudaStream_t st, const BatchView* bv) {
     LJFixed<N> p;
-    static_cast<LJPair&>(p) = lj;
-    return run_fp64(p, g, cv, out, pre, st, tile, bv);
+    static_cast<LJPair&>(p) = fs.lj;
+    return run_fp64(p, g, cv, out, fs, st, bv);
 }
 
 cudaError_t launch_forces_fp64(const ForceSetup& fs, const DevGeom& g, const CellView& cv,
                                const ForceOut& out, cudaStream_t st, const BatchView* bv) {
-    const int t = fs.tile;
-    const float pre = fs.pre_rc2f;
     switch (fs.kind) {
-    case 1: return run_fp64(fs.ao, g, cv, out, pre, st, t, bv);
+    case 1: return run_fp64(fs.ao, g, cv, out, fs, st, bv);
     case 2:
         switch (fs.lj.n) {
-        case 0: return run_lj_fp64<0>(fs.lj, g, cv, out, pre, st, t, bv);
-        case 6: return run_lj_fp64<6>(fs.lj, g, cv, out, pre, st, t, bv);
-        case 12: return run_lj_fp64<12>(fs.lj, g, cv, out, pre, st, t, bv);
-        case 18: return run_lj_fp64<18>(fs.lj, g, cv, out, pre, st, t, bv);
-        default: return run_fp64(fs.lj, g, cv, out, pre, st, t, bv);
+        case 0: return run_lj_fp64<0>(g, cv, out, fs, st, bv);
+        case 6: return run_lj_fp64<6>(g, cv, out, fs, st, bv);
+        case 12: return run_lj_fp64<12>(g, cv, out, fs, st, bv);
+        case 18: return run_lj_fp64<18>(g, cv, out, fs, st, bv);
+        default: return run_fp64(fs.lj, g, cv, out, fs, st, bv);
         }
-    case 3: return run_fp64(fs.cal, g, cv, out, pre, st, t, bv);
+    case 3: return run_fp64(fs.cal, g, cv, out, fs, st, bv);
     case 4: {
         if (bv) return cudaErrorInvalidValue;  // batches hold single-plugin replicas
         ComboPair cp{fs.ao, fs.lj, fs.ao.rc2 > fs.lj.rc2 ? fs.ao.rc2 : fs.lj.rc2};
-        return run_fp64(cp, g, cv, out, pre, st, t, bv);
+        return run_fp64(cp, g, cv, out, fs, st, bv);
     }
     }
     return cudaErrorInvalidValue;

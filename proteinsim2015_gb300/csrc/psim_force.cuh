@@ -596,7 +596,7 @@ struct LJFixed : LJPair {
     __device__ __forceinline__ double fr64(double r2, double size, double s2) const {
         if (N % 2 == 0 && pure()) {
             const double i2 = rcp64(r2);
-            return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));
+            return __dmul_rn(fr64_lj(powi_fixed<N / 2>(__dmul_rn(s2, i2))), i2);
         }
         const double ri = rsqrt64(r2);
         return fr64_of(r2, ri, __dmul_rn(ri, ri), powi_fixed<N>(__dmul_rn(size, ri)));
@@ -622,7 +622,7 @@ struct LJPure : LJPair {
     using Fr64 = LJPure;
     __device__ __forceinline__ double fr64(double r2, double, double s2) const {
         const double i2 = rcp64(r2);
-        return fr64_of(r2, 0.0, i2, powi_fixed<N / 2>(__dmul_rn(s2, i2)));
+        return __dmul_rn(fr64_lj(powi_fixed<N / 2>(__dmul_rn(s2, i2))), i2);
     }
     __device__ __forceinline__ float fnet32(float, float, float rinv, float size) const {
         const float lj = powi_fixed<N>(size * rinv);

@@ -37,6 +37,7 @@ struct ForceSetup {
     int tile;          // 0: a warp per 32 consecutive particles; 1: a block per home cell
     int walk;          // with tile 0, the mixed form's walk: 0 direct (default), 1 staged, 2 direct
     int lj_pure;       // LennardJones with yukawaStrength 0 in every replica
+    int unit_box;      // a box (of a replica) of edge 1 (F64Body)
 };
 
 // Elements a posh array holds past its n particles wherever a pair list is

@@ -70,9 +70,12 @@ inline int plugin_status(cudaError_t e) { return e == cudaSuccess ? PSIM_OK : PS
 template <class Pair>
 int plugin_launch_fp64(const Pair& p, const psim_force_args* a, cudaStream_t st) {
     const DevGeom g = plugin_geom(a);
-    const F64Body<Pair> body{p, g};
     const CellView cv = plugin_cells(a);
     const ForceOut out = plugin_out(a);
+    if (g.L == 1.0)
+        return plugin_status(
+            launch_force_pass(F64Body<Pair, true>{p, g}, g, cv, out, a->prefilter_r2, st));
+    const F64Body<Pair> body{p, g};
     if (a->tile) return plugin_status(launch_force_cells(body, g, cv, out, a->prefilter_r2, st));
     return plugin_status(launch_force_pass(body, g, cv, out, a->prefilter_r2, st));
 }

@@ -50,3 +50,32 @@ def test_unit_vector_in_a_box_of_edge_1(psim, force_pass, kind, box):
     i = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)
     pos = np.mod(((i + 0.5) * 0.2 + rng.uniform(-0.04, 0.04, i.shape)) * box, box).reshape(-1)
     check(psim, psim.geometry(125, box, box / 3, 3), p, pos, np.full(125, 0.05 * box))
+
+
+def test_boxes_of_edge_1_in_a_batch_and_a_system(psim):
+    # one replica of edge 1 beside one of edge 2, and each alone: the same forces, bit for
+    # bit, and the oracle's
+    i = np.stack(np.meshgrid(*[np.arange(5)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    x = (i + 0.5) * 0.2 + np.random.default_rng(1).uniform(-0.04, 0.04, i.shape)
+    single, reps, pos, rad = [], [], [], []
+    for box in (1.0, 2.0):
+        p = psim.make_force("LJ", 0.3 * box, kT=1.0, well_depth=1.0, lj_num=6, yukawa_strength=0.0)
+        g, r = psim.geometry(125, box, box / 3, 3), np.full(125, 0.05 * box)
+        q = np.mod(x * box, box).reshape(-1)
+        s = psim.System(g, p, dt=0.001, precision=psim.PRECISION_FP64)
+        s.upload(q, r)
+        s.step(3)
+        f, now = s.forces(), s.download()["pos"]
+        s.close()
+        *_, ref, err, sc = oracle_force(p.as_dict(), g, now, r)
+        assert err == 0 and rel_per_particle(f, ref, sc) <= FORCE_TOL_FP64
+        single.append(f)
+        reps.append((g, p))
+        pos.append(q)
+        rad.append(r)
+    b = psim.Batch([(g, p, 90210) for g, p in reps], dt=0.001,
+                   precision=psim.PRECISION_FP64)
+    b.upload(np.concatenate(pos), np.concatenate(rad))
+    b.step(3)
+    assert np.array_equal(b.forces(), np.concatenate(single))
+    b.close()
