@@ -397,13 +397,13 @@ def run_batched(psim, dev, steps=2000, n_reps=512, tune=True, skin=0.3):
         lanes = None
         if sk > 0 and tune:   # threads per particle of the list pass, on the live batch
             lanes = batch.tune_lanes(b, steps=min(steps, 100))
-        b0 = b.list_builds()
+        b0, l0 = b.list_builds(), b.launches()
         ms = b.time_steps(steps)
-        builds = b.list_builds() - b0
+        builds, launches = b.list_builds() - b0, b.launches() - l0
         prof = b.profile(5)
         out = {"value": b.n * steps / (ms * 1e-3), "ms_per_step": ms / steps,
                "phases_ms": {k: round(v, 5) for k, v in prof.items()},
-               "launches": steps * b.launches_per_step() + builds * b.launches_per_rebuild()}
+               "launches": launches}
         if sk > 0:
             out["list_builds"] = builds
         if lanes:
@@ -629,9 +629,9 @@ def run_gpu(args):
     with ClockSampler(dev) as clk:
         if not args.profile_only:
             s.time_steps(CLOCK_WINDOW_STEPS)
-        builds0 = s.list_builds()
+        launches0 = s.launches()
         ms = s.time_steps(args.steps)
-        builds_timed = s.list_builds() - builds0
+        launches_timed = s.launches() - launches0
     if dist:
         import torch
         t = torch.tensor([ms], dtype=torch.float64)
@@ -748,7 +748,7 @@ def run_gpu(args):
                                   "peak_source": "measured: SM loads and stores on pinned "
                                                  "host memory, both directions at once"},
                 "path": "force_evaluate -> next_system -> cells_build on pinned host arrays, read and written in place by the GPU over NVLink-C2C (copies where the device has no pageable host access)"},
-        "gpu_launches": args.steps * s.launches_per_step() + builds_timed * s.launches_per_rebuild(),
+        "gpu_launches": launches_timed,
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": fp32_peak,
                      "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                      "traffic": profiled_traffic(FORCE_PROFILE),

@@ -568,13 +568,16 @@ void* psim_system_stream(psim_system* sys);
  * [3] total.  Runs n_steps steps. */
 int psim_system_profile(psim_system* sys, int32_t n_steps, double* out_ms);
 
-/* Number of kernel launches one step issues (for launch accounting). */
+/* Kernel launches of one normal step in a long run.  The first step and the
+ * velocity steps take up to one more; 1 for a small system with a pair list,
+ * up to 1024 of whose normal steps share one launch. */
 int psim_system_launches_per_step(psim_system* sys);
-/* Kernel launches of a step's pair-list rebuild (0 without a pair list): with
- * a pair list a step launches psim_system_launches_per_step kernels, and the
- * steps that rebuild the list this many more (0 where a small system's steps and
- * rebuilds are one kernel). */
+/* Kernel launches that a pair-list rebuild adds to its step: 0, it is part of
+ * the step's last kernel. */
 int psim_system_launches_per_rebuild(psim_system* sys);
+/* Kernels launched by the system's steps so far (psim_system_step, step_async,
+ * time_steps): the count of what was launched, for launch accounting. */
+int64_t psim_system_launches(psim_system* sys);
 
 /* Occupancy of the current cell list: max and mean particles per cell. */
 int psim_system_cell_occupancy(psim_system* sys, int32_t* max_occ, double* mean_occ);

@@ -165,6 +165,7 @@ def lib():
             "psim_system_profile": ([P, C.c_int32, P], C.c_int),
             "psim_system_launches_per_step": ([P], C.c_int),
             "psim_system_launches_per_rebuild": ([P], C.c_int),
+            "psim_system_launches": ([P], C.c_int64),
             "psim_system_cell_occupancy": ([P, C.POINTER(C.c_int32), C.POINTER(C.c_double)], C.c_int),
             "psim_system_time_steps": ([P, C.c_int32, C.POINTER(C.c_double)], C.c_int),
             "psim_system_pair_count": ([P, C.c_double, C.POINTER(C.c_double)], C.c_int),
@@ -663,6 +664,10 @@ class System:
 
     def launches_per_rebuild(self):
         return lib().psim_system_launches_per_rebuild(self._h)
+
+    def launches(self):
+        """Kernels launched by the system's steps so far."""
+        return lib().psim_system_launches(self._h)
 
     def cell_occupancy(self):
         m, a = C.c_int32(), C.c_double()

@@ -1236,6 +1236,7 @@ struct psim_system {
         snap;
     long long noise_first = 0, noise_steps = 0;
     long long total = 0;      // steps since upload, as the host has enqueued them
+    long long launches = 0;   // kernels that its steps have launched (step_kernels)
     bool uploaded = false;
     bool snap_pending = false;
     // one graph per buffer phase (one step), and one of kGraphSteps steps
@@ -1655,6 +1656,12 @@ bool fused_steps(const psim_system* s) {
     if (s->cfg.precision == PSIM_PRECISION_MIXED)
         return s->n <= kStepDirect && step_direct_fits(s->fs, s->g);
     return !s->fs.tile && !s->fs.unit_box && s->n <= kStep64 && one_order(s);
+}
+// Kernels of a step: force, vGB (one kernel where fused), then scan x3, scatter and
+// canonicalise, or the one kernel of a small system's cell order, or with a pair list the
+// step end with its rebuild.
+int step_kernels(const psim_system* s, bool fused) {
+    return (s->list_on || one_order(s) ? 3 : 7) - (fused ? 1 : 0);
 }
 // The velocity counter's period: step t > 0 writes the velocities when it
 // divides t; step 0 is the first step.
@@ -2397,6 +2404,7 @@ int psim_system_step_async(psim_system* s, int32_t n_steps) {
             return rc;
         }
         s->total += steps;
+        s->launches += !g && fused ? 1 : steps * step_kernels(s, fused);
         return (int)PSIM_OK;
     });
     return rc || n_steps == 0 ? rc : capture_others(s);
@@ -2890,15 +2898,12 @@ int psim_system_profile(psim_system* s, int32_t n_steps, double* out_ms) {
 }
 
 int psim_system_launches_per_step(psim_system* s) {
-    // force, vGB, scan x3, scatter, canonicalise (+1 memset node), or force, vGB and the
-    // one kernel of a small system's cell order; with a pair list: force, vGB (one kernel
-    // on normal steps where fused_steps allows), the step end with its rebuild; a small
-    // system's normal step alone, or a stretch of them, is one kernel
     if (!s) return 7;
-    if (!s->list_on) return (one_order(s) ? 3 : 7) - (fused_steps(s) ? 1 : 0);
     DeviceGuard dg(s->device);
-    return small_system(s) ? 1 : (fused_steps(s) ? 2 : 3);
+    return small_system(s) ? 1 : step_kernels(s, fused_steps(s));
 }
+
+int64_t psim_system_launches(psim_system* s) { return s ? s->launches : 0; }
 
 int psim_system_launches_per_rebuild(psim_system*) {
     return 0;   // part of the step's last kernel
