@@ -1,6 +1,7 @@
 """Which kernels a system's steps take, by the launches it reports and counts, on both
-sides of each size's line.  (A system whose displacement tracker has been started runs the
-two kernels.)"""
+sides of each size's line; and the pair-list step as one kernel on systems too large for
+the cluster kernel, on batches, and beside steps with unequal radii.  (A system whose
+displacement tracker has been started runs the two kernels, and so do profiled steps.)"""
 import numpy as np
 import pytest
 
@@ -53,4 +54,65 @@ def test_kernels_with_lanes_and_unequal_radii(psim):
     assert s.launches_per_step() == 1
     upload(s, n, box, np.where(np.arange(n) % 2, 0.5, 0.45))
     assert s.launches_per_step() == 3
+    s.close()
+
+
+def outcome(s):
+    return dict(s.download(), forces=s.forces(), at=np.array(s.get_step() + (s.list_builds(),)))
+
+
+def same(a, b):
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("n,box,scale", [(9000, 34.0, 22), (20001, 45.0, 30)])
+@pytest.mark.parametrize("vel_freq", [3, 25, 1000])
+def test_list_step_as_one_kernel(psim, n, box, scale, vel_freq):
+    out = []
+    for two in (False, True):
+        s = system(psim, n, box, scale, vel_freq=vel_freq)
+        if two:
+            s.track_start()
+        assert s.launches_per_step() == (3 if two else 2)
+        for k in (1, 2, 17, 40, 5, 60, 1):
+            s.step(k)
+        out.append(outcome(s))
+        s.close()
+    same(*out)
+    assert out[0]["at"][2] > 0
+
+
+def test_batch_list_step_as_one_kernel(psim):
+    sizes = [(9000, 34.0, 22), (300, 14.0, 9), (8193, 34.0, 22)]
+    f = psim.make_force("AO", 1.2, kT=1.0, well_depth=0.3)
+    parts = [gas(n, box, n) for n, box, _ in sizes]
+    out = []
+    for two in (False, True):
+        b = psim.Batch([(psim.geometry(n, box, box / s, s), f, 5 + k)
+                        for k, (n, box, s) in enumerate(sizes)], dt=0.001, kT=1.0, vel_freq=25,
+                       skin=0.3)
+        b.upload(np.concatenate([p for p, _ in parts]), np.concatenate([r for _, r in parts]),
+                 vel=np.random.default_rng(7).standard_normal(3 * b.n) * 2.0)
+        assert b.launches_per_step() == 2
+        (b.profile if two else b.step)(126)
+        out.append(outcome(b))
+        b.close()
+    same(*out)
+    assert out[0]["at"][2] > 0
+
+
+@pytest.mark.parametrize("n,box,scale", [(1000, 18.0, 11), (9000, 34.0, 22)])
+def test_radii_change_with_an_upload(psim, n, box, scale):
+    # equal radii (one kernel), unequal ones (two) and equal ones again on one system: the
+    # bits of a system of its own each
+    mixed = np.where(np.arange(n) % 2, 0.5, 0.45)
+    s = system(psim, n, box, scale, up=False)
+    for rad in (None, mixed, np.full(n, 0.48), None):
+        upload(s, n, box, rad)
+        s.step(60)
+        one = system(psim, n, box, scale, rad=rad)
+        one.step(60)
+        same(outcome(s), outcome(one))
+        one.close()
     s.close()
