@@ -855,7 +855,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
                                       w.lslot_of.as<int>(), w.lbuild.as<float4>(),
                                       w.lhalo.as<int>(), w.lpos.as<float4>(), z.disp2, g,
                                       w.lcompact ? 1.0f / w.lunit : 0.f, w.lradius, flags, st));
-        const PairList pl{nullptr, w.lpos.as<float4>(), w.lcount.as<int>(),
+        const PairList pl{w.lpos.as<float4>(), w.lcount.as<int>(),
                           w.list.as<uint32_t>(), g.n, w.lcompact, w.lradius, w.lunit};
         PSIM_CUDA(fr.run(PSIM_PASS_LIST, g, nullptr, &pl, out, st));
         PSIM_CUDA(launch_export_force(g.n, w.lslot_of.as<int>(), f, f + n, f + 2 * n,
@@ -938,7 +938,7 @@ int force_evaluate(psim_force_launch_fn plugin, const psim_force_params* params,
             }
         }
         if (listed) {
-            const PairList pl{nullptr, w.lpos.as<float4>(), w.lcount.as<int>(),
+            const PairList pl{w.lpos.as<float4>(), w.lcount.as<int>(),
                               w.list.as<uint32_t>(), g.n, w.lcompact, w.lradius, w.lunit};
             PSIM_CUDA(fr.run(PSIM_PASS_LIST, g, nullptr, &pl, out, st));
             inv = w.lslot_of.as<int>();
@@ -1246,8 +1246,7 @@ struct psim_system {
     cudaGraphExec_t graph_multi = nullptr;
     int small = -1;           // whether stretches of normal steps run in one kernel (-1: not asked)
     uint32_t latched = 0;
-    // Verlet pair list of the mixed form (list_on): list slot of each storage
-    // slot (ping-pong with the order), positions at the build, entries,
+    // Verlet pair list of the mixed form (list_on): positions at the build, entries,
     // counts, and the two step-parity rebuild flags
     bool list_on = false;
     int list_lanes = 1;   // threads per particle of the list force pass (1, 2 or 4)
@@ -1256,12 +1255,12 @@ struct psim_system {
     float lpre = 0.f, ldisp2 = 0.f, hr = 0.f;
     // the records (lpos) ping-pong with the step's parity: a step reads one buffer and
     // writes the next step's
-    DevBuf lslot[2], lbuild, lpos[2], list, lcount, lflag, lhalo, lhcount;
+    DevBuf lbuild, lpos[2], list, lcount, lflag, lhalo, lhcount;
     // With a pair list the cell list is rebuilt only with the list (the
     // storage order then stays the list order between builds): the state is
     // carried into the new order through pscratch (15 n doubles), and the
     // per-slot arrays live in buffer 0 (buffer 1 receives a new order or the
-    // cell view of the current positions that refresh_cells computes).
+    // cell view of the current positions that cell_refs computes).
     DevBuf pscratch;
     DevBuf rebuild;                        // the rebuild kernel's barrier counter and sums
     // compact 16-byte records when every particle has one radius (set by the upload)
@@ -1361,10 +1360,10 @@ cudaError_t enqueue_list_build(psim_system* s, int cb) {
                              s->st);
 }
 
-// The pair list of the state at phase ph (the storage order is the list order: no
-// slot table); in a batch, with each particle's replica and its pair functor.
+// The pair list of the state at phase ph; in a batch, with each particle's replica and
+// its pair functor.
 PairList pair_list(psim_system* s, const Phase& ph) {
-    PairList pl{nullptr, s->lpos[ph.sb].as<float4>(), s->lcount.as<int>(), s->list.as<uint32_t>(),
+    PairList pl{s->lpos[ph.sb].as<float4>(), s->lcount.as<int>(), s->list.as<uint32_t>(),
                 s->n, s->lcompact, s->lradius, s->lunit};
     if (s->n_reps) {
         pl.rep = s->b_rep.as<int>();
@@ -1506,7 +1505,6 @@ int enqueue_step_lazy(psim_system* s, long long t, cudaEvent_t* evs, bool fused 
     a.count = nullptr;  // no hash: the cell list is rebuilt with the list
     a.err = s->err.as<uint32_t>();
     a.state = s->state.as<StepState>();
-    a.lslot = nullptr;  // list slot = storage slot
     a.lbuild = s->lbuild.as<float4>();
     a.lpos = s->lpos[nsb].as<float4>();
     a.linv_unit = s->lcompact ? 1.0f / s->lunit : 0.f;
@@ -2151,7 +2149,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
     if (ok && cfg->precision == PSIM_PRECISION_MIXED)
         ok = !s->posl.ensure(16 * n);
     if (ok && list_on) {
-        ok = !s->lslot[0].ensure(4 * n) && !s->lslot[1].ensure(4 * n) && !s->lbuild.ensure(16 * n) &&
+        ok = !s->lbuild.ensure(16 * n) &&
              !s->lpos[0].ensure(32 * (n + 1 + (size_t)s->hcap)) &&
              !s->lpos[1].ensure(32 * (n + 1 + (size_t)s->hcap)) &&
              !s->list.ensure(4 * n * (size_t)(s->lcap + kListFold)) && !s->lcount.ensure(4 * n) &&
@@ -2184,7 +2182,7 @@ psim_system* system_new(const psim_system_config* cfg, const DevGeom& g, bool ba
             const ForceRunner fr{&s->fs, cfg->force_launch, &s->cfg.force};
             CellView cv{s->posd.as<double4_32a>(), s->posh.as<float4>(), s->posl.as<float4>(),
                         s->cellid.as<int>(), s->start.as<int>(), s->count[0].as<int>()};
-            PairList pl{nullptr, s->lpos[0].as<float4>(), s->lcount.as<int>(),
+            PairList pl{s->lpos[0].as<float4>(), s->lcount.as<int>(),
                         s->list.as<uint32_t>(), s->n, 0, 0.f, 0.f};
             const int pass = cfg->precision == PSIM_PRECISION_FP64
                                  ? PSIM_PASS_FP64
@@ -2214,7 +2212,7 @@ void psim_system_destroy(psim_system* s) {
     drop_graphs(s);
     DevBuf* arrs[] = {&s->cellid, &s->key, &s->rank, &s->tmp, &s->start, &s->scratch, &s->posd,
                       &s->posh, &s->posl, &s->vel, &s->err, &s->state, &s->occ, &s->noise,
-                      &s->snap, &s->lslot[0], &s->lslot[1], &s->lbuild, &s->lpos[0], &s->lpos[1], &s->list,
+                      &s->snap, &s->lbuild, &s->lpos[0], &s->lpos[1], &s->list,
                       &s->lcount, &s->lflag, &s->lhalo, &s->lhcount, &s->pscratch, &s->rebuild, &s->b_tasks,
                       &s->b_geoms, &s->b_pairs, &s->b_pre, &s->b_rep, &s->b_seeds,
                       &s->img, &s->track_start, &s->b_lpre, &s->b_hr, &s->obs};

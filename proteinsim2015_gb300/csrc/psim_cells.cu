@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) canonicalize_kernel(CanonArgs a, int vel_
     if (a.err && *a.err) return;
     if (p < a.n) canon_slot(a, p);
     if (a.state && a.advance && p == 0)
-        step_advance(a.state, vel_freq, a.rebuild && *a.rebuild);
+        step_advance(a.state, vel_freq, false);
 }
 
 cudaError_t launch_canonicalize(const CanonArgs& a, cudaStream_t st) {

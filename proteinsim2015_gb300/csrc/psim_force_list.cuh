@@ -10,11 +10,10 @@
 // has.  The force of each step is then the same set of pair terms, read from
 // ~(rc+skin)^3/(27 cs^3) as many candidates as the cell walk tests.
 //
-//   build  the warp kernel of psim_force.cuh with a body that appends, rather
-//          than evaluates, the candidates within rc + skin (plus the rounding
-//          margin of its FP32 test).  It runs on the step's own cell list, so
-//          list order is the cell order of the build step, and it needs
-//          cellSize >= rc + skin.  A pair across the box edge refers to a
+//   build  (psim_list_build.cuh) a thread per particle appends the candidates of
+//          its 27 cells within rc + skin (plus the rounding margin of the FP32
+//          test).  It runs on the cell order made with it, so list order is the
+//          cell order of the build step, and it needs cellSize >= rc + skin.  A pair across the box edge refers to a
 //          halo record: a copy of the neighbour shifted by the box, made for
 //          every particle within rc + skin of a face and rewritten with it
 //          each step, so the force pass does no periodic arithmetic.
@@ -220,11 +219,10 @@ force_list_kernel(Body body0, DevGeom g, PairList pl, ForceOut out) {
     // a batch: the pair functor of the particle's replica (its neighbours are
     // all of the same replica)
     const Body body = kReplicas ? body0.for_replica(pl.pairs, pl.rep[f], g) : body0;
-    const int s = pl.lslot ? pl.lslot[f] : f;   // no slot table: storage order is list order
     typename Body::Acc acc;
     uint32_t err = 0;
     float rmin = 3.0e38f;
-    list_terms<Body, kCompact, kCount, kLanes>(body, pl, s, lane, acc, rmin, err);
+    list_terms<Body, kCompact, kCount, kLanes>(body, pl, f, lane, acc, rmin, err);
     const float us2 = (2.0f * pl.radius) * (2.0f * pl.radius);
     if constexpr (kLanes > 1) {
         // lane 0 adds the other lanes' sums in lane order

@@ -96,7 +96,7 @@ cudaError_t launch_forces_mixed(const ForceSetup& fs, const DevGeom& g, const Ce
 constexpr int kListFold = 8;   // pair terms per Kahan fold
 constexpr int kHaloBaseMax = (1 << 25) - 1;   // halo records per system
 struct PairList {
-    const int* lslot;      // list slot of each current storage slot (null: the same slot)
+    // the storage order is the list order
     // list order, unwrapped, one record per slot (+ the ghost slot n and the
     // halo records): full, pos[2 s] = {x, y, z, R} high parts and pos[2 s + 1]
     // the low parts; or compact (one float4, compact_record: fixed-point
@@ -197,9 +197,7 @@ struct VgbSystemArgs {
     // also written in list order as the image nearest the list-build position
     // (an exact float pair), and *lflag_set is raised when it lies more than
     // sqrt(ldisp2) from that position; *lflag_clear (the other step parity's
-    // flag) is cleared.  lslot: the list slot of each storage slot (null: the
-    // same slot, when the storage order is the list order).
-    const int* lslot;
+    // flag) is cleared.  The storage order is the list order.
     const float4* lbuild;       // list order: positions at the build, .w radius
     float4* lpos;               // PairList::pos
     float linv_unit;            // 1 / PairList::unit (compact), or 0 (full records)
@@ -320,17 +318,11 @@ struct CanonArgs {
     int advance;            // 1: this rebuild ends a step (advance state)
     int vel_freq;           // brownianIntegrator::velFreq
     uint32_t* err;          // non-zero: a previous kernel failed, skip the work
-    // pair-list bookkeeping (null: none).  lslot is carried with the particles;
-    // when *rebuild != 0 the list is rebuilt on the new order, so lslot becomes
-    // the identity and posh/posl/lbuild are written -- otherwise posh/posl
-    // hold the list-order positions and are left alone.
-    const int* rebuild;
-    const int* lslot_in;
-    int* lslot_out;
+    // of a pair list built on the new order (null: none): positions at the build, records
     float4* lbuild;
-    float4* lpos;           // PairList::pos, written with posh/posl
+    float4* lpos;           // PairList::pos
     float linv_unit;        // 1 / PairList::unit (compact), or 0 (full records)
-    // halo records of the particles within hr of a face (rebuild only):
+    // halo records of the particles within hr of a face:
     // lhalo per slot, records n + 1 + [0, hcap) handed out by *lhcount
     int* lhalo;
     int* lhcount;

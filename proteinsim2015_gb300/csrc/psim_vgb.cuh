@@ -335,14 +335,11 @@ __device__ __forceinline__ void vgb_system_one(const VgbSystemArgs& a, const Vgb
     double mx[3] = {a.mx[o], a.my[o], a.mz[o]};
     const double F[3] = {a.fx[f], a.fy[f], a.fz[f]};
     const double F0[3] = {a.gx[o], a.gy[o], a.gz[o]};
-    int ls = 0, lhal = 0;
+    int lhal = 0;
     float4 lb = make_float4(0.f, 0.f, 0.f, 0.f);
     if (a.lbuild) {
-        // list slot: carried with the particle, or its storage slot when the
-        // storage order is the list order
-        ls = a.lslot ? __ldg(a.lslot + f) : f;
-        lb = __ldg(a.lbuild + ls);
-        lhal = __ldg(a.lhalo + ls);
+        lb = __ldg(a.lbuild + f);
+        lhal = __ldg(a.lhalo + f);
     }
     double v[3] = {0.0, 0.0, 0.0};
     if (first || vel_step) {
@@ -375,7 +372,7 @@ __device__ __forceinline__ void vgb_system_one(const VgbSystemArgs& a, const Vgb
         a.vel[3 * (size_t)tag + 1] = v[1];
         a.vel[3 * (size_t)tag + 2] = v[2];
     }
-    if (a.lbuild) list_position(a, ls, lb, lhal, xn, g);
+    if (a.lbuild) list_position(a, f, lb, lhal, xn, g);
     if (f == 0 && a.lflag_clear) {
         *a.lflag_clear = 0;
         *a.lhcount = 0;   // halo records are handed out afresh at the next build
