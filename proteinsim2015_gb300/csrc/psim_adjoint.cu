@@ -27,7 +27,7 @@
 // memory is (T/K + K) positions.  K is the caller's interval or, where that is longer,
 // what 256 MB hold (kAdjTraj): a trajectory that fits is never computed twice.
 // All sums are taken in an order that the positions decide: two runs agree bit for
-// bit.  What bounds it is the FP64 unit: 33 FP64 operations a pair forward and ~65
+// bit (but for the counts of more than 3072 bins, which are added as they come).  What bounds it is the FP64 unit: 33 FP64 operations a pair forward and ~65
 // back with the lanes of an instruction 75% full at 32768 particles.  Gradient of 60
 // steps, with a cell list and a thread per particle for every pass before, and now:
 // 4096 particles 186 -> 5.6 ms, 32768 286 -> 22.8 ms (7.7 and 29.7 with each segment
@@ -327,8 +327,9 @@ struct AdjWalk {
     const int* bad;         // first step with a particle beyond skin/2 of the build
 };
 
-// fn(j, d, r2) for every neighbour j of slot i with r2 < rc2
-template <int G, class Fn>
+// fn(j, d, r2) for every neighbour j of slot i with r2 < rc2; kAll: fn(ok, r2) by all
+// lanes together, ok where a lane has such a neighbour
+template <int G, bool kAll = false, class Fn>
 __device__ __forceinline__ void for_pairs(const AdjWalk& w, double rc2, int i, bool active,
                                           int lane, const double4_32a& xi, uint32_t* q, Fn&& fn) {
     constexpr int U = 2;
@@ -351,6 +352,8 @@ __device__ __forceinline__ void for_pairs(const AdjWalk& w, double rc2, int i, b
         const int last = __reduce_max_sync(0xffffffffu, cnt);
         int k = (m - done) & (G - 1);
         for (int it = 0; it < last; it += G, k += G) {
+            double r2 = 0.0;
+            bool ok = false;
             if (k < cnt) {
                 const int j = (int)q[k];
                 const double4_32a xj = w.x[j];
@@ -365,10 +368,12 @@ __device__ __forceinline__ void for_pairs(const AdjWalk& w, double rc2, int i, b
                     for (int a = 0; a < 3; ++a)
                         if (fabs(d[a]) > w.half) d[a] = d[a] < 0.0 ? d[a] + w.L : d[a] - w.L;
                 }
-                const double r2 =
-                    __fma_rn(d[2], d[2], __fma_rn(d[1], d[1], __dmul_rn(d[0], d[0])));
-                if (below_rc(r2, rc2)) fn(j, d, r2);
+                r2 = __fma_rn(d[2], d[2], __fma_rn(d[1], d[1], __dmul_rn(d[0], d[0])));
+                ok = below_rc(r2, rc2);
+                if constexpr (!kAll)
+                    if (ok) fn(j, d, r2);
             }
+            if constexpr (kAll) fn(ok, r2);
         }
         done += cnt;
         cnt = 0;
@@ -512,64 +517,121 @@ struct AdjHist {
 };
 
 // The kernel values G_b = norm exp(-z_b^2 / 2) of distance r at the bins
-// b_lo..b_hi, z_b = (r - r_b) / sigma, by the recurrence of consecutive bins
+// lo..hi, z_b = (r - r_b) / sigma, by the recurrence of consecutive bins
 // (z_{b+1} = z_b - dz): G_{b+1} = G_b q_b, q_{b+1} = q_b e^{-dz^2},
-// q_b = e^{dz z_b - dz^2 / 2} -- two exponentials per distance.  fn(b, z, G).
-// G starts at g times the kernel.
-template <class Fn>
-__device__ __forceinline__ void gauss_bins(const AdjHist& h, double r, double g, const double2* e2,
-                                           Fn&& fn) {
-    const int b0 = __double2int_rd((r - h.r_min) * h.inv_dr);
-    const int lo = max(0, b0 - h.reach), hi = min(h.n_bins - 1, b0 + h.reach);
-    if (lo > hi) return;
-    double z = (r - (h.r_min + (lo + 0.5) * h.dr)) * h.inv_sig;
-    double G = g * h.norm * exp_table(-0.5 * z * z, e2);
-    double q = exp_table(h.dz * z - 0.5 * h.dz * h.dz, e2);
-    for (int b = lo; b <= hi; ++b) {
-        fn(b, z, G);
+// q_b = e^{dz z_b - dz^2 / 2} -- two exponentials per distance.
+struct GaussBins {
+    int lo, hi;     // no bin: lo > hi
+    double z, G, q;
+    // G starts at g times the kernel
+    __device__ __forceinline__ GaussBins(const AdjHist& h, double r, double g, const double2* e2) {
+        const int b0 = __double2int_rd((r - h.r_min) * h.inv_dr);
+        lo = max(0, b0 - h.reach);
+        hi = min(h.n_bins - 1, b0 + h.reach);
+        z = (r - (h.r_min + (lo + 0.5) * h.dr)) * h.inv_sig;
+        G = g * h.norm * exp_table(-0.5 * z * z, e2);
+        q = exp_table(h.dz * z - 0.5 * h.dz * h.dz, e2);
+    }
+    __device__ __forceinline__ void next(const AdjHist& h) {
         G *= q;
         q *= h.qq;
         z -= h.dz;
     }
+};
+
+// The smoothed counts of x_t.  Each warp has bins of its own in shared memory, to which its
+// lanes add in a fixed order: a lane waits a few steps where needed, so that no two lanes
+// are at the same bin in any step.  So the sums are FP64's, to the far tails of the kernel,
+// and the same from run to run.  A block takes every gridDim-th group of its particles and
+// adds its warps' bins, in order, to its own row of part.  Bound by the FP64 unit and the
+// latency of a step's load, addition and store.  20 steps, each sampled, with 64-bit
+// integer sums (whose unit the tails fall below) and so: 4096 particles 1716 -> 1775 us,
+// 32768 8057 -> 8273; with one copy of a warp's bins 1848 and 8680; 400 bins 7687 -> 7441,
+// 2900 8332 -> 9016.
+constexpr int kAdjHistBins = 3072;          // the most bins in shared memory
+constexpr int kAdjHistBlocks = 152 * 16;    // the most rows
+// Warps of a block, fewer where their bins are many; and copies of a warp's bins, more
+// where they are few, for its lanes would wait for one another.
+int hist_warps(int bins) { return bins <= 384 ? 8 : 2; }
+int hist_copies(int bins) {
+    int c = 8;
+    while (c > 1 && c * bins > 512) c /= 2;
+    return c;
+}
+int hist_blocks(int n, int lanes, int bins) {
+    const int per = hist_warps(bins) * (32 / lanes);
+    return std::min(kAdjHistBlocks, (n + per - 1) / per);
+}
+constexpr int kAdjHistSmem = 60 << 10;      // the most that hist_smem says
+size_t hist_smem(int lanes, int bins) {
+    return hist_warps(bins) *
+           (8 * (size_t)bins * hist_copies(bins) + 4 * (size_t)(32 / lanes) * kAdjStride);
+}
+template <int G>
+__global__ void __launch_bounds__(256)
+adj_hist_kernel(AdjWalk w, double rc2, AdjHist h, int copies, double* part) {
+    extern __shared__ double bins[];
+    if (*w.bad <= w.t) return;
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int held = copies * h.n_bins, first = lane * copies / 32 * h.n_bins;
+    double* mine = bins + wid * held;
+    uint32_t* q = reinterpret_cast<uint32_t*>(bins + warps * held) +
+                  (wid * (32 / G) + lane / G) * kAdjStride;
+    for (int b = lane; b < held; b += 32) mine[b] = 0.0;
+    mine += first;
+    __syncwarp();
+    const int per = warps * (32 / G);
+    for (int g0 = blockIdx.x * per; g0 < w.n; g0 += gridDim.x * per) {
+        const int i = g0 + wid * (32 / G) + lane / G;
+        const bool active = i < w.n;
+        double4_32a xi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
+        if (active) xi = w.x[i];
+        for_pairs<G, true>(w, rc2, i, active, lane, xi, q, [&](bool ok, double r2) {
+            GaussBins a(h, ok ? sqrt64(r2, rsqrt64(r2)) : h.r_min, h.dr, w.q.e2);
+            const int len = ok ? max(0, a.hi - a.lo + 1) : 0;
+            // lane by lane, a wait before the first bin that keeps it from every other lane's:
+            // at step t the lane is at bin lo + t - wait
+            int wait = 0;
+            for (bool again = true; __any_sync(0xffffffffu, again); wait += again ? 1 : 0) {
+                const uint32_t same = __match_any_sync(
+                    0xffffffffu, len > 0 ? first + a.lo - wait : held + lane);
+                again = len > 0 && (same & ((1u << lane) - 1u)) != 0;
+            }
+            const int steps = __reduce_max_sync(0xffffffffu, len > 0 ? len + wait : 0);
+            for (int t = 0; t < steps; ++t) {
+                const int k = t - wait;
+                if (k >= 0 && k < len) {
+                    mine[a.lo + k] += a.G;
+                    a.next(h);
+                }
+                __syncwarp();
+            }
+        });
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < h.n_bins; b += blockDim.x) {
+        double t = 0.0;
+        for (int k = 0; k < warps * copies; ++k) t += bins[k * h.n_bins + b];
+        part[(size_t)blockIdx.x * h.n_bins + b] += t;
+    }
 }
 
-// The smoothed counts of x_t.  Each block sums its particles' in shared memory as
-// 64-bit integers in units of 2^-k (scale = 2^k: the largest sum a block can
-// have fills them), exact to that unit and in any order, and adds the sums to its own
-// row of part; without shared memory for the bins, to global doubles.
-constexpr int kAdjHistWarps = 8;
-constexpr int kAdjHistBins = 3072;
-template <int G, bool kShared>
-__global__ void __launch_bounds__(kAdjHistWarps * 32)
-adj_hist_kernel(AdjWalk w, double rc2, AdjHist h, double scale, double* part) {
-    __shared__ uint32_t sq[kAdjHistWarps][32 / G][kAdjStride];
-    extern __shared__ unsigned long long bins[];
+// The same with more bins than shared memory holds: added to global doubles, in any order.
+template <int G>
+__global__ void __launch_bounds__(kAdjWarps * 32)
+adj_hist_global_kernel(AdjWalk w, double rc2, AdjHist h, double* sum) {
+    __shared__ uint32_t sq[kAdjWarps][32 / G][kAdjStride];
     if (*w.bad <= w.t) return;
-    if (kShared) {
-        for (int b = threadIdx.x; b < h.n_bins; b += blockDim.x) bins[b] = 0ull;
-        __syncthreads();
-    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int i = (blockIdx.x * kAdjHistWarps + wid) * (32 / G) + lane / G;
+    const int i = (blockIdx.x * kAdjWarps + wid) * (32 / G) + lane / G;
     const bool active = i < w.n;
     double4_32a xi = make_double4_32a(0.0, 0.0, 0.0, 0.0);
     if (active) xi = w.x[i];
-    const double unit = h.dr * scale;
     for_pairs<G>(w, rc2, i, active, lane, xi, sq[wid][lane / G],
                  [&](int, const double*, double r2) {
-                     gauss_bins(h, sqrt64(r2, rsqrt64(r2)), kShared ? unit : h.dr, w.q.e2,
-                                [&](int b, double, double v) {
-                                    if (kShared)
-                                        atomicAdd(&bins[b],
-                                                  (unsigned long long)__double2ll_rn(v));
-                                    else
-                                        atomicAdd(&part[b], v);
-                                });
+                     GaussBins a(h, sqrt64(r2, rsqrt64(r2)), h.dr, w.q.e2);
+                     for (int b = a.lo; b <= a.hi; ++b, a.next(h)) atomicAdd(&sum[b], a.G);
                  });
-    if (!kShared) return;
-    __syncthreads();
-    for (int b = threadIdx.x; b < h.n_bins; b += blockDim.x)
-        part[(size_t)blockIdx.x * h.n_bins + b] += (double)bins[b] / scale;
 }
 
 // out[b] = the sum of column b of part[rows][cols], rows in order
@@ -646,8 +708,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32) adj_reverse_kernel(AdjWalk w, 
         if (a.wgt) {
             // d/dx_i of the smoothed counts of pairs (i, j) and (j, i)
             double wr = 0.0;
-            gauss_bins(a.h, sqrt64(r2, ri), 1.0, w.q.e2,
-                       [&](int b, double z, double G_) { wr = __fma_rn(a.wgt[b] * G_, z, wr); });
+            GaussBins g(a.h, sqrt64(r2, ri), 1.0, w.q.e2);
+            for (int b = g.lo; b <= g.hi; ++b, g.next(a.h)) wr = __fma_rn(a.wgt[b] * g.G, g.z, wr);
             wr *= 2.0 * a.h.dr * a.h.inv_sig * ri;
 #pragma unroll
             for (int k = 0; k < 3; ++k) gl[k] = __fma_rn(wr, d[k], gl[k]);
@@ -897,30 +959,21 @@ AdjWalk walk_at(psim_adjoint* a, const AdjPair& q, int slot, int t) {
 }
 
 int add_hist(psim_adjoint* a, const AdjWalk& w) {
-    const int b = blocks_of(a, kAdjHistWarps), threads = kAdjHistWarps * 32;
-    // the unit of a block's integer sums: the largest sum its particles' lists
-    // allow stays below 2^62
-    const double top = a->hist.dr * a->hist.norm * (kAdjHistWarps * 32.0 / a->lanes) *
-                       std::max(a->most, 1);
-    const double scale = std::ldexp(1.0, 61 - std::ilogb(top));
-    const bool shared = a->cfg.n_bins <= kAdjHistBins;
-    const size_t smem = shared ? 8 * (size_t)a->cfg.n_bins : 0;
-    double* out = shared ? a->hpart.as<double>() : a->hsum.as<double>();
+    const int nb = a->cfg.n_bins;
     cudaError_t e = cudaSuccess;
     with_lanes(a, [&](auto g) {
         constexpr int G = decltype(g)::value;
-        if (!shared) {
-            adj_hist_kernel<G, false><<<b, threads, 0, a->st>>>(w, a->walk_rc2, a->hist, scale,
-                                                                out);
+        if (nb > kAdjHistBins) {
+            adj_hist_global_kernel<G><<<blocks_of(a, kAdjWarps), kAdjWarps * 32, 0, a->st>>>(
+                w, a->walk_rc2, a->hist, a->hsum.as<double>());
             return;
         }
-        // with the queues (25600 bytes at four lanes a particle) the most bins take more
-        // than the 48 KB a kernel has without asking
-        e = cudaFuncSetAttribute(adj_hist_kernel<G, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kAdjHistBins);
+        const size_t smem = hist_smem(G, nb);
+        e = cudaFuncSetAttribute(adj_hist_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kAdjHistSmem);
         if (e == cudaSuccess)
-            adj_hist_kernel<G, true><<<b, threads, smem, a->st>>>(w, a->walk_rc2, a->hist, scale,
-                                                                  out);
+            adj_hist_kernel<G><<<hist_blocks(a->n, G, nb), hist_warps(nb) * 32, smem, a->st>>>(
+                w, a->walk_rc2, a->hist, hist_copies(nb), a->hpart.as<double>());
     });
     ADJ_CUDA(e);
     ADJ_CUDA(cudaGetLastError());
@@ -1046,7 +1099,7 @@ int forward_all(psim_adjoint* a, const AdjPair& q, const double* pos0, const dou
     ADJ_CUDA(cudaMemsetAsync(force_at(a, -1), 0, 24 * (size_t)n, a->st));
     ADJ_CUDA(cudaMemsetAsync(a->hsum.p, 0, 8 * (size_t)nb, a->st));
     const bool shared = nb <= kAdjHistBins;
-    const int rows = blocks_of(a, kAdjHistWarps);
+    const int rows = hist_blocks(n, a->lanes, nb);
     if (shared) ADJ_CUDA(cudaMemsetAsync(a->hpart.p, 0, 8 * (size_t)nb * rows, a->st));
     for (int t0 = 0; t0 < a->T; t0 += a->K) {
         const int t1 = std::min(t0 + a->K, a->T);
@@ -1156,7 +1209,7 @@ psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device
               !a->part.ensure(8 * kAdjTh * threads) && !a->acc.ensure(8 * kAdjTh * (1 + kAdjRowBlocks)) &&
               !a->e2.ensure(16 * kExpTable) &&
               (cfg->n_bins > kAdjHistBins ||
-               !a->hpart.ensure(8 * (size_t)cfg->n_bins * blocks_of(a, kAdjHistWarps))) &&
+               !a->hpart.ensure(8 * (size_t)cfg->n_bins * hist_blocks(n, a->lanes, cfg->n_bins))) &&
               !a->hsum.ensure(8 * (size_t)cfg->n_bins) && !a->wgt.ensure(8 * (size_t)cfg->n_bins);
     // the segments' positions and the checkpoints: shorter segments where the memory
     // does not hold K steps
