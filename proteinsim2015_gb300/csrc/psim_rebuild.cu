@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(kRebuildThreads, 4) step_rebuild_kernel(Rebuil
 int rebuild_sums() { return 8192; }
 
 cudaError_t launch_step_rebuild(const RebuildArgs& a, const DevGeom& g, cudaStream_t st) {
-    if (a.n == 0) return cudaSuccess;
     int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -177,8 +176,9 @@ cudaError_t launch_step_rebuild(const RebuildArgs& a, const DevGeom& g, cudaStre
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, step_rebuild_kernel,
                                                           kRebuildThreads, 0);
     if (e != cudaSuccess) return e;
-    const int blocks = std::min({sms * per, rebuild_sums(),
-                                 (a.n + kRebuildThreads - 1) / kRebuildThreads});
+    // one block at least: an empty system's steps count too
+    const int blocks = std::max(1, std::min({sms * per, rebuild_sums(),
+                                             (a.n + kRebuildThreads - 1) / kRebuildThreads}));
     RebuildArgs args = a;
     DevGeom geom = g;
     void* params[] = {&args, &geom};
