@@ -2389,7 +2389,9 @@ int psim_system_step_async(psim_system* s, int32_t n_steps) {
     if (s->latched) return fail(code_from_bits(s->latched), "%s", bits_text(s->latched));
     if (n_steps < 0) return fail(PSIM_ERR_INPUT, "negative step count");
     DeviceGuard dg(s->device);
-    if (s->list_on) {   // not in a caller's capture (the stream is handed out)
+    // not in a caller's capture (the stream is handed out): a launched graph cannot be
+    // captured, and single kernels would be, but for the steps between them
+    if (s->list_on || n_steps > 0) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         PSIM_CUDA(cudaStreamIsCapturing(s->st, &capture));
         if (capture != cudaStreamCaptureStatusNone) PSIM_CUDA(cudaErrorStreamCaptureUnsupported);
