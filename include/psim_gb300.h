@@ -390,6 +390,11 @@ typedef struct {
     int32_t lj_n;
 } psim_adjoint_params;
 
+/* Device memory: about 1 KB a particle (the forces of 18 steps among it) and 4
+ * bytes an entry of its neighbour list; 48 bytes a particle and step of the
+ * segment kept, which is checkpoint_every steps or what 256 MB hold, whichever
+ * is more (shorter where the memory does not hold it); 88 a particle and
+ * segment. */
 psim_adjoint* psim_adjoint_create(const psim_adjoint_config* cfg, int32_t device);
 /* The Philox Gaussians the systems and the adjoint draw (PSIM_NOISE_PHILOX):
  * n_steps steps from first_step for particles 0..n-1 with `seed`, in the
@@ -445,7 +450,12 @@ psim_system* psim_batch_create_list(const psim_replica* reps, int32_t n_reps,
                                     int32_t noise_mode, int32_t device, double skin);
 
 /* Creates the system and its device buffers (the role of system::system,
- * system.cpp:69-103, without the random initialisation: states are uploaded). */
+ * system.cpp:69-103, without the random initialisation: states are uploaded).
+ * They are kept until psim_system_destroy: about 350 bytes a particle; with a
+ * pair list 4 a list entry (room for 1.5 times the mean neighbours within
+ * cutOff + skin, and 40) and about 230 more, among them two buffers of 32 for
+ * the records of particles and images; and, from the first call that reads the
+ * state, that call's scratch, up to 256 MB. */
 psim_system* psim_system_create(const psim_system_config* cfg);
 void psim_system_destroy(psim_system* sys);
 

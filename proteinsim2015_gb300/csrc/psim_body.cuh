@@ -2,8 +2,9 @@
 // (psim_force.cuh, psim_force_cell.cuh, psim_force_list.cuh) are
 // instantiated with, one per precision form, each over a plugin's pair
 // functor:
-//   F64Body<Pair>    the plain FP64 form in the reference's operation order
-//                    (a translation unit built with --fmad=false)
+//   F64Body<Pair>    the plain FP64 form: the reference's own decisions (images,
+//                    cutoff, overlap), pair terms in an order of its own (a
+//                    translation unit built with --fmad=false)
 //   MixedBody<Pair>  FP32 pair terms, Kahan-compensated FP32 sums over
 //                    float-pair positions
 // Header-only, so that a force plugin compiles the same passes with its own

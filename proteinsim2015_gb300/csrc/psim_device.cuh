@@ -344,7 +344,7 @@ __device__ __forceinline__ void cell_xyz(int c, const DevGeom& g, int& x, int& y
 
 // ------------------------------------------------------------ pair functors
 // fnet64: the plugin's FP64 per-pair magnitude in the reference's operation
-// order, except that integer powers use binary powering and divisions by r2
+// order (a functor's fr64, which the FP64 passes call, has its own), except that integer powers use binary powering and divisions by r2
 // or r multiply by 1/r (a few ulp, far inside the 1e-12 parity tolerance).
 // It is host-callable too: a plugin's CPU getAcceleration (the reference's
 // per-particle entry) evaluates the same functor.

@@ -2,7 +2,8 @@
 // rounds twice as in the reference's x86-64 build (no FMA contraction).
 //
 //   F64Body             plain form of the plugin force pass (the pair body of
-//                       force_pass_kernel, psim_force.cuh)
+//                       force_quad_kernel, psim_force.cuh)
+//   step_quad_kernel    that pass and the update of a small system in one
 //   vgb_system_kernel   brownianIntegrator::nextSystem fused with the gather
 //                       into the new cell order and the cell hash + count of
 //                       the next rebuild (brownianIntegrator.cpp:181-356,
@@ -19,7 +20,6 @@
 namespace psim {
 
 // ------------------------------------------------------------------ forces
-
 
 template <class Pair>
 static cudaError_t run_fp64(const Pair& p, const DevGeom& g, const CellView& cv,

@@ -9,7 +9,8 @@
 //     d = (x_j,hi - h) + (x_j,lo - l)
 // where the first difference is exact for nearby values (Sterbenz), so d
 // carries one FP32 rounding of a number of size <= rc, not of the box.
-// The pair loop itself is force_pass_kernel (psim_force.cuh).
+// The pair loops are force_direct_kernel (psim_force.cuh) and force_list_kernel
+// (psim_force_list.cuh).
 #include <cmath>
 
 #include "psim_body.cuh"
